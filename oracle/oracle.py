@@ -33,7 +33,7 @@ def build(ref: bool | None = None) -> None:
     tree is present)."""
     subprocess.run(["make", "-s", "-C", str(HERE), "all"], check=True)
     if ref is None:
-        ref = REFERENCE_TREE.is_dir()
+        ref = (REFERENCE_TREE / "potential.cpp").is_file()  # an empty directory is no tree
     if ref:
         subprocess.run(["make", "-s", "-C", str(HERE), "ref", f"REF={REFERENCE_TREE}"], check=True)
         subprocess.run(["make", "-s", "-C", str(HERE), "geo", f"REF={REFERENCE_TREE}"], check=True)
