@@ -26,9 +26,21 @@
 // reconstruction with FMA.  Its error is ~0.5 ulp and, being plain IEEE
 // arithmetic, it gives the same bits on the host and on the device, which
 // lets the CPU oracle reproduce the GPU plain form exactly.
+//
+// On the device cr_exp, cr_log and cr_pow first try quick forms (quick_exp,
+// quick_log): table-driven argument reduction (Tang 1989, 1990) carried in
+// hi + lo doubles, 25-40 FP64 operations with errors below 2^-70, against
+// 600-700 for the double-double series above.  Ziv's rounding test (Ziv
+// 1991) then decides: when hi + (lo - bound) and hi + (lo + bound) round to
+// the same double, every value within the bound rounds to it, the
+// double-double result among them, so the quick result has its bits; else (about once in 2^15 calls) the series runs.  GB300
+// has two FP64 lanes per SM and clock, so these operation counts are the
+// time of the occupancy update and of the per-site functions.  The host
+// build keeps the series alone: the oracle stays an independent check.
 #pragma once
 
 #include <cmath>
+#include <cstring>
 
 namespace a2c {
 namespace dd {
@@ -182,14 +194,75 @@ A2C_HD double round_dd(D2 a) { return a.hi + a.lo; }
     {1.9571441241754002, 8.960767791036668e-17}, \
     {1.978456026387951, 4.0388753109278167e-17}
 #if defined(__CUDACC__)
-__device__ const double kExp2TabDev[64][2] = {A2C_EXP2_TABLE};
+__device__ const __align__(16) double kExp2TabDev[64][2] = {A2C_EXP2_TABLE};
 #endif
 static const double kExp2TabHost[64][2] = {A2C_EXP2_TABLE};
 #undef A2C_EXP2_TABLE
 
+A2C_HD int hi_word(double x) {
+#if defined(__CUDA_ARCH__)
+  return __double2hiint(x);
+#else
+  unsigned long long b;
+  std::memcpy(&b, &x, 8);
+  return (int)(b >> 32);
+#endif
+}
+A2C_HD int lo_word(double x) {
+#if defined(__CUDA_ARCH__)
+  return __double2loint(x);
+#else
+  unsigned long long b;
+  std::memcpy(&b, &x, 8);
+  return (int)(unsigned)b;
+#endif
+}
+A2C_HD double from_words(int hi, int lo) {
+#if defined(__CUDA_ARCH__)
+  return __hiloint2double(hi, lo);
+#else
+  const unsigned long long b = ((unsigned long long)(unsigned)hi << 32) | (unsigned)lo;
+  double x;
+  std::memcpy(&x, &b, 8);
+  return x;
+#endif
+}
+
+// Adding 1.5 2^52 rounds |v| < 2^31 to an integer (ties to even), held in
+// the sum's low word.
+constexpr double kRoundShift = 6755399441055744.0;
+
+// The same values for |x| < 708 with integer operations where the FP64
+// pipe is not needed: rounding by an addition, the integer from the sum's
+// low word, the power of two added to the exponent (the result is normal).
+// 13 FP64 operations.
+A2C_HD double fexp_mid(double x) {
+  const double t = x * 92.33248261689366 + kRoundShift;  // x * 64/ln2
+  const double n = t - kRoundShift;
+  const int ni = lo_word(t);
+  double r = fma(-n, 0.010830424696249145, x);
+  r = fma(-n, 3.623510646634843e-19, r);
+  double p = fma(r, 0.001388888888888889, 0.008333333333333333);
+  p = fma(r, p, 0.041666666666666664);
+  p = fma(r, p, 0.16666666666666666);
+  p = fma(r, p, 0.5);
+  p = fma(r * r, p, r);
+#if defined(__CUDA_ARCH__)
+  const double2 e = *reinterpret_cast<const double2 *>(kExp2TabDev[ni & 63]);
+  const double th = e.x, tl = e.y;
+#else
+  const double th = kExp2TabHost[ni & 63][0], tl = kExp2TabHost[ni & 63][1];
+#endif
+  const double v = th + fma(th, p, tl);
+  return from_words(hi_word(v) + (int)((unsigned)(ni >> 6) << 20), lo_word(v));
+}
+
 // Results below 2^-1021 are flushed to zero (no argument of the potential
 // comes near), above 709.78 overflow to +inf; NaN propagates.
 A2C_HD double fexp(double x) {
+#if defined(__CUDA_ARCH__)
+  if ((hi_word(x) & 0x7fffffff) < 0x40862000) return fexp_mid(x);  // |x| < 708
+#endif
   if (!(x > -708.0)) return (x != x) ? x : 0.0;
   if (x > 709.78) return HUGE_VAL;
   const double n = rint(x * 92.33248261689366);  // x * 64/ln2
@@ -211,21 +284,288 @@ A2C_HD double fexp(double x) {
   return ldexp(th + fma(th, p, tl), k);
 }
 
-// Correctly rounded except in rare near-midpoint cases.
-A2C_HD double cr_exp(double x) {
-  if (!(x > -700.0 && x < 700.0)) return exp(x);
-  return round_dd(exp_dd({x, 0.0}));
+// e^(a.hi + a.lo) = 2^k (v.hi + v.lo) with relative error below 2^-70, for
+// |a.hi| < 700 and a.lo below an ulp of a.hi.  a = (64 k + j) ln2/64 + r: n times
+// the 36-bit head of ln2/64 is exact, the tail product carried in two
+// doubles; e^r - 1 = r + r^2/2 + (degree 7 from r^3/6 on, below 2^-25, in
+// double); times 2^(j/64) as hi + lo.
+A2C_HD D2 quick_exp(D2 a, int &k) {
+  const double t = a.hi * 92.33248261689366 + kRoundShift;  // 64/ln2
+  const double n = t - kRoundShift;
+  const int ni = lo_word(t), j = ni & 63;
+  k = (ni - j) / 64;
+  const double r1 = fma(-n, 0.010830424696223417, a.hi);  // exact
+  const double p = n * 2.572804622327669e-14, pe = fma(n, 2.572804622327669e-14, -p);
+  D2 r = two_sum(r1, -p);
+  r = two_sum(r.hi, r.lo - pe + a.lo);
+  const double v = r.hi * r.hi, ve = fma(r.hi, r.hi, -v);
+  double c = fma(r.hi, 1.984126984126984e-04, 1.388888888888889e-03);
+  c = fma(r.hi, c, 8.333333333333333e-03);
+  c = fma(r.hi, c, 4.1666666666666664e-02);
+  c = fma(r.hi, c, 1.6666666666666666e-01);
+  c = (r.hi * v) * c;
+  const D2 s = quick_two_sum(r.hi, 0.5 * v);
+  const double e2 = s.lo + (c + (0.5 * ve + fma(r.hi, r.lo, r.lo)));
+#if defined(__CUDA_ARCH__)
+  const double th = kExp2TabDev[j][0], tl = kExp2TabDev[j][1];
+#else
+  const double th = kExp2TabHost[j][0], tl = kExp2TabHost[j][1];
+#endif
+  const D2 q = two_prod(th, s.hi);
+  const D2 h = quick_two_sum(th, q.hi);
+  return quick_two_sum(h.hi, h.lo + (q.lo + fma(th, e2, fma(tl, s.hi, tl))));
 }
-A2C_HD double cr_log(double u) {
-  if (!(u > 0.0) || !(u < 1.0e300) || u < 1.0e-300) return log(u);
-  return round_dd(log_dd(u));
+
+// -log of the 9-bit c below for the 128 intervals of m in [0.707, 1.414):
+// c ~ 1/m, hi a multiple of 2^-42, lo the rest.
+#define A2C_LOG_TABLE \
+    {1.41015625, -0.34370051385326406, -5.438888329899065e-14}, \
+    {1.40234375, -0.3381449440087181, 1.686950122813039e-15}, \
+    {1.39453125, -0.3325583373000427, -3.390686133672229e-14}, \
+    {1.38671875, -0.32694034499581903, -3.428840012666946e-14}, \
+    {1.37890625, -0.3212906124538222, 8.788542769971545e-14}, \
+    {1.37109375, -0.3156087789864159, 1.1259274624680829e-13}, \
+    {1.36328125, -0.30989447772276435, -1.0033796982039214e-13}, \
+    {1.359375, -0.30702503529482783, -8.403156304792425e-14}, \
+    {1.3515625, -0.3012613305781997, 3.7923164802093147e-14}, \
+    {1.34375, -0.2954642128938758, 3.993416384387844e-14}, \
+    {1.3359375, -0.28963329258294834, -9.43339818951269e-14}, \
+    {1.328125, -0.28376817313073843, 9.3834172236637e-14}, \
+    {1.32421875, -0.2808226629008459, -4.188609137863701e-14}, \
+    {1.31640625, -0.27490548587275043, -4.8816703646769986e-14}, \
+    {1.30859375, -0.26895308734560786, 1.0389630784002988e-13}, \
+    {1.30078125, -0.2629650455007777, -1.0364636459896663e-13}, \
+    {1.296875, -0.25995752443691345, -1.2621729398885316e-14}, \
+    {1.2890625, -0.25391520998095984, -3.600176732637335e-15}, \
+    {1.28125, -0.2478361639045943, 1.3029797173308663e-14}, \
+    {1.27734375, -0.24478272641772492, 3.399981108361833e-14}, \
+    {1.26953125, -0.23864773785021498, 3.997050909530134e-14}, \
+    {1.265625, -0.23556607131286, 9.30945949519689e-14}, \
+    {1.2578125, -0.22937410106487732, 3.149265065191484e-14}, \
+    {1.25, -0.22314355131425145, 4.169796584527195e-14}, \
+    {1.24609375, -0.2200136583053336, 5.149667234141408e-14}, \
+    {1.23828125, -0.21372432939779173, 7.359580186440514e-14}, \
+    {1.234375, -0.21056476910735, 3.6507188831790577e-16}, \
+    {1.2265625, -0.2042155414287663, 7.540916511956189e-14}, \
+    {1.22265625, -0.20102574606062262, 3.188184937543774e-14}, \
+    {1.21484375, -0.1946154676995775, -9.41653814571825e-14}, \
+    {1.2109375, -0.19139485299956505, -6.440856150696892e-14}, \
+    {1.203125, -0.18492233849406148, 4.9485167661250996e-14}, \
+    {1.19921875, -0.18167030310769405, 5.937506333384701e-14}, \
+    {1.1953125, -0.17840765747291698, 9.86835038673495e-14}, \
+    {1.1875, -0.17185025692674571, 8.649239607212071e-14}, \
+    {1.18359375, -0.16855536102980295, -3.714397754170472e-15}, \
+    {1.17578125, -0.16193282026938505, 7.179390019295677e-14}, \
+    {1.171875, -0.15860503017665906, 2.0472357800461955e-14}, \
+    {1.16796875, -0.15526612891108016, -4.3792508292406054e-14}, \
+    {1.16015625, -0.1485546943231384, 1.24915489807516e-15}, \
+    {1.15625, -0.14518200984457508, 7.718001336828099e-14}, \
+    {1.15234375, -0.14179791186029433, 3.698459506697097e-14}, \
+    {1.14453125, -0.13499516453748583, -1.8996158041578768e-14}, \
+    {1.140625, -0.13157635778861732, -1.0195735223708473e-13}, \
+    {1.13671875, -0.12814582269197672, 4.668031403945796e-14}, \
+    {1.12890625, -0.12124924363297396, 1.0427241278273008e-13}, \
+    {1.125, -0.11778303565643, 4.654729747598445e-14}, \
+    {1.12109375, -0.11430477128010352, 4.488953352238699e-14}, \
+    {1.1171875, -0.11081436634026431, -2.5799991283069902e-14}, \
+    {1.109375, -0.10379679368156758, -7.598636597194141e-14}, \
+    {1.10546875, -0.10026945316371894, 4.378637617078398e-14}, \
+    {1.1015625, -0.09672962645845473, -9.638067658552277e-14}, \
+    {1.09765625, -0.0931772248541165, -6.678708517162898e-14}, \
+    {1.08984375, -0.0860343373417436, -5.955922987625643e-14}, \
+    {1.0859375, -0.08244366921098845, -8.614512936087814e-14}, \
+    {1.08203125, -0.07884006170775137, -2.465018906176612e-14}, \
+    {1.078125, -0.07522342123752424, -6.329065958724544e-14}, \
+    {1.07421875, -0.07159365318693744, -7.137308225343178e-14}, \
+    {1.0703125, -0.06795066190852594, 1.8195060030168815e-14}, \
+    {1.0625, -0.06062462181648698, 5.213620639136504e-14}, \
+    {1.05859375, -0.056941376400118315, -2.0109399435564958e-14}, \
+    {1.0546875, -0.053244514518837605, 2.532168943117445e-14}, \
+    {1.05078125, -0.04953393512232651, 4.9880309107981426e-14}, \
+    {1.046875, -0.0458095360313564, 6.219834199475792e-14}, \
+    {1.04296875, -0.04207121392073532, 4.826314000551128e-14}, \
+    {1.0390625, -0.03831886430202758, -1.0902154302203302e-13}, \
+    {1.03515625, -0.034552381506728125, 6.839139742328777e-14}, \
+    {1.03125, -0.03077165866670839, -4.529814257790929e-14}, \
+    {1.02734375, -0.026976587698300136, 9.806050516843177e-14}, \
+    {1.0234375, -0.023167059281604452, 7.007359704310036e-14}, \
+    {1.01953125, -0.019342962843211353, 8.041853850522586e-14}, \
+    {1.015625, -0.015504186535963527, -1.7274567499706107e-15}, \
+    {1.01171875, -0.011650617220084314, 1.0903974971735932e-13}, \
+    {1.00390625, -0.0038986404156275967, -2.972634690092895e-14}, \
+    {1.0, 0.0, 0.0}, \
+    {1.0, 0.0, 0.0}, \
+    {0.98828125, 0.011787955751970003, 7.223757580209288e-14}, \
+    {0.98046875, 0.019724505347767263, 1.1326399700142234e-14}, \
+    {0.97265625, 0.027724548014930406, -7.554530328896727e-14}, \
+    {0.966796875, 0.03376686247088401, -6.652375062271929e-14}, \
+    {0.958984375, 0.041880497245074366, -8.71601984429868e-14}, \
+    {0.951171875, 0.05006050195697753, -5.953822004049194e-14}, \
+    {0.9453125, 0.05623971832278585, 9.023009281142904e-14}, \
+    {0.9375, 0.0645385211375924, -2.1225608044809997e-14}, \
+    {0.931640625, 0.07080813415109333, 7.324072905400027e-14}, \
+    {0.923828125, 0.07922923654746228, 1.1253882534313481e-13}, \
+    {0.91796875, 0.0855919303353403, 6.322009333691484e-14}, \
+    {0.91015625, 0.0941389909139616, -9.969653023079706e-14}, \
+    {0.904296875, 0.10059757095336863, -9.49206327250953e-14}, \
+    {0.8984375, 0.10709813555627079, 9.631011033519217e-14}, \
+    {0.892578125, 0.1136412341452342, 6.889214192008475e-14}, \
+    {0.884765625, 0.12243249955645297, 2.0797337102277177e-14}, \
+    {0.87890625, 0.1290770422751848, -4.2451216089619995e-14}, \
+    {0.873046875, 0.1357660304258843, 5.4642560554597724e-14}, \
+    {0.8671875, 0.14250006260726877, 1.4256439478199035e-14}, \
+    {0.861328125, 0.14927974959255152, 1.1026677017414112e-13}, \
+    {0.85546875, 0.15610571466299916, 6.249274931606537e-14}, \
+    {0.849609375, 0.16297859395081105, 1.2645632984431417e-14}, \
+    {0.845703125, 0.16758689703692653, 9.140819889491412e-14}, \
+    {0.83984375, 0.17453941635199044, -9.076231556699796e-14}, \
+    {0.833984375, 0.18154061181098768, -1.0445339530284443e-13}, \
+    {0.828125, 0.18859116980752333, 2.6693431578015818e-14}, \
+    {0.822265625, 0.19569179135714876, -2.239166785505485e-14}, \
+    {0.818359375, 0.20045370511729743, 7.262215167738776e-14}, \
+    {0.8125, 0.20763936477828793, -4.3425422595242564e-14}, \
+    {0.806640625, 0.21487703207844788, 2.714636557077735e-14}, \
+    {0.802734375, 0.2197314105433179, -4.472851385991314e-14}, \
+    {0.796875, 0.22705745063535687, -1.078736749871691e-14}, \
+    {0.79296875, 0.2319714654377094, 6.573097737831975e-14}, \
+    {0.787109375, 0.23938806309274696, 7.784172549574863e-14}, \
+    {0.783203125, 0.24436319773303694, -9.834201296269778e-14}, \
+    {0.77734375, 0.25187261975497677, 9.331234677945918e-14}, \
+    {0.7734375, 0.25691041378513546, -1.0822171646799124e-13}, \
+    {0.76953125, 0.26197371574153294, 4.102651071698446e-14}, \
+    {0.763671875, 0.26961706505403527, 1.0674835088128526e-13}, \
+    {0.759765625, 0.27474528142101917, 4.2320076202145394e-14}, \
+    {0.755859375, 0.2798999320098119, -8.591298393628546e-14}, \
+    {0.75, 0.28768207245184385, -6.292357389008195e-14}, \
+    {0.74609375, 0.29290401643288533, 4.727452940514406e-14}, \
+    {0.7421875, 0.29815337231912054, -4.4204083338755686e-14}, \
+    {0.73828125, 0.3034304294199046, 1.548345993498083e-14}, \
+    {0.734375, 0.30873548164959175, 2.1522127491642888e-14}, \
+    {0.728515625, 0.3167462053957024, -1.0174753377507561e-14}, \
+    {0.724609375, 0.3221225624320141, 5.855316792709415e-14}, \
+    {0.720703125, 0.3275279809990934, -1.1281735060685524e-13}, \
+    {0.716796875, 0.33296277698491394, 2.3569101751290204e-14}, \
+    {0.712890625, 0.33842727145702156, -5.280156204729064e-15}, \
+    {0.708984375, 0.3439217907746297, 2.730651892134709e-14}
+#if defined(__CUDACC__)
+__device__ const double kLogTabDev[128][3] = {A2C_LOG_TABLE};
+#endif
+static const double kLogTabHost[128][3] = {A2C_LOG_TABLE};
+#undef A2C_LOG_TABLE
+
+// log(u) for 1e-300 <= u < 1e300; this value and log_dd's are within `err`
+// of each other (2^-71; near 1, where the reduction leaves u unchanged,
+// 2^-66 of the value and 2^-90).
+// u = 2^e m, z = c m - 1 with |z| < 2^-6.9 exact in two doubles, log u =
+// e ln2 - log c + log1p(z); terms from z^3/3 on (below 2^-22) in double.
+A2C_HD D2 quick_log(double u, double &err) {
+  const int hu = hi_word(u), t = hu - 0x3fe6a09e;
+  const int e = t >> 20, i = (t >> 13) & 127;
+  const double m = from_words(hu - (e << 20), lo_word(u));
+#if defined(__CUDA_ARCH__)
+  const double c = kLogTabDev[i][0], lh = kLogTabDev[i][1], ll = kLogTabDev[i][2];
+  const double de = __hiloint2double(0x43300000, 0x80000000 ^ e) - 4503601774854144.0;  // e, by its bits
+#else
+  const double c = kLogTabHost[i][0], lh = kLogTabHost[i][1], ll = kLogTabHost[i][2];
+  const double de = (double)e;
+#endif
+  const D2 p = two_prod(m, c);
+  const double z = p.hi - 1.0, zl = p.lo;
+  const double v = z * z, ve = fma(z, z, -v);
+  double q = fma(z, 9.090909090909091e-02, -0.1);
+  q = fma(z, q, 1.1111111111111111e-01);
+  q = fma(z, q, -0.125);
+  q = fma(z, q, 1.4285714285714285e-01);
+  q = fma(z, q, -1.6666666666666666e-01);
+  q = fma(z, q, 0.2);
+  q = fma(z, q, -0.25);
+  q = fma(z, q, 3.333333333333333e-01);
+  q = (z * v) * q;
+  const D2 s = quick_two_sum(z, -0.5 * v);
+  const double s2 = s.lo + (q + fma(-0.5, ve, zl * (1.0 - z + v)));
+  const double a = fma(de, 0.6931471805598903, lh);  // exact: both multiples of 2^-42
+  const D2 b = two_sum(a, s.hi);
+  const double l = b.lo + (s2 + fma(de, 5.497923018708371e-14, ll));
+  const D2 r = quick_two_sum(b.hi, l);
+  // 2^-66 of it and 2^-90 (the series' absolute error), or 2^-71
+  err = a == 0.0 ? fma(fabs(r.hi), 1.3552527156068805e-20, 8.077935669463161e-28) : 4.235164736271502e-22;
+  return r;
 }
-A2C_HD double cr_pow(double u, double y) {
-  if (!(u > 0.0) || !(u < 1.0e300) || u < 1.0e-300 || !(fabs(y) < 1.0e6)) return pow(u, y);
+
+// Ziv's test: true when every value within err of v rounds to `out`.
+A2C_HD bool rounds_to(D2 v, double err, double &out) {
+  out = v.hi + (v.lo + err);
+  return out == v.hi + (v.lo - err);
+}
+// out times 2^k for a result whose scaled value is a normal double
+A2C_HD double scale_normal(double out, int k) { return from_words(hi_word(out) + (k << 20), lo_word(out)); }
+
+// The quick forms: false when the rounding test leaves the result open.
+A2C_HD bool quick_cr_exp(double x, double &out) {
+  int k;
+  const D2 v = quick_exp({x, 0.0}, k);
+  const bool ok = rounds_to(v, v.hi * 8.470329472543003e-22, out);  // 2^-70
+  out = scale_normal(out, k);
+  return ok;
+}
+A2C_HD bool quick_cr_log(double u, double &out) {
+  double err;
+  const D2 v = quick_log(u, err);
+  return rounds_to(v, err, out);
+}
+// y log(u) is off by |y| times the log's error and 2^-104 of itself, which
+// is the relative error it adds to the power.
+A2C_HD bool quick_cr_pow(double u, double y, double &out) {
+  double err;
+  const D2 l = mul_d(quick_log(u, err), y);
+  if (!(l.hi > -700.0 && l.hi < 700.0)) return false;
+  int k;
+  const D2 v = quick_exp(l, k);
+  const bool ok = rounds_to(v, v.hi * (8.470329472543003e-22 + 1.0625 * fabs(y) * err), out);
+  out = scale_normal(out, k);
+  return ok;
+}
+
+// The series alone, out of line on the device: the quick forms' rare rest.
+#if defined(__CUDACC__)
+#define A2C_REST static __host__ __device__ __noinline__
+#else
+#define A2C_REST inline
+#endif
+A2C_REST double series_exp(double x) { return round_dd(exp_dd({x, 0.0})); }
+A2C_REST double series_log(double u) { return round_dd(log_dd(u)); }
+A2C_REST double series_pow(double u, double y) {
   const D2 l = mul_d(log_dd(u), y);
   if (!(l.hi > -700.0 && l.hi < 700.0)) return pow(u, y);
   return round_dd(exp_dd(l));
 }
+
+// Correctly rounded except in rare near-midpoint cases.
+A2C_HD double cr_exp(double x) {
+  if (!(x > -700.0 && x < 700.0)) return exp(x);
+#if defined(__CUDA_ARCH__)
+  double q;
+  if (quick_cr_exp(x, q)) return q;
+#endif
+  return series_exp(x);
+}
+A2C_HD double cr_log(double u) {
+  if (!(u > 0.0) || !(u < 1.0e300) || u < 1.0e-300) return log(u);
+#if defined(__CUDA_ARCH__)
+  double q;
+  if (quick_cr_log(u, q)) return q;
+#endif
+  return series_log(u);
+}
+A2C_HD double cr_pow(double u, double y) {
+  if (!(u > 0.0) || !(u < 1.0e300) || u < 1.0e-300 || !(fabs(y) < 1.0e6)) return pow(u, y);
+#if defined(__CUDA_ARCH__)
+  double q;
+  if (quick_cr_pow(u, y, q)) return q;
+#endif
+  return series_pow(u, y);
+}
+#undef A2C_REST
 
 #undef A2C_HD
 
