@@ -9,11 +9,17 @@
 
 #include "ddmath.cuh"
 
+#if defined(__CUDACC__)
+#define A2C_EAM __host__ __device__ __forceinline__
+#else
+#define A2C_EAM inline
+#endif
+
 namespace a2c {
 namespace eam64 {
 
 // potential.cpp:16-38
-__device__ __forceinline__ double F_Pd(double rho) {
+A2C_EAM double F_Pd(double rho) {
   rho = rho / 50.0;
   double y = 295878.9003038662 * (rho - 0.20581955357385892);
   y = y * (rho - 0.081228755904399);
@@ -31,7 +37,7 @@ __device__ __forceinline__ double F_Pd(double rho) {
 // potential.cpp:45-57.  F_H is differentiated by a central difference, so
 // its three pow calls use the correctly rounded dd::cr_pow (a one-ulp pow
 // difference would otherwise become a ~1e-11 relative gradient error).
-__device__ __forceinline__ double F_H(double rho) {
+A2C_EAM double F_H(double rho) {
   const double c = 0.000197047, d = 1.18860, a = 9.99780, b = 60.0155, eps1 = 0.0540638;
   const double u = rho + eps1;
   double y = -c * (1.0 / (2.0 + d) * dd::cr_pow(u, 2.0 + d) - (a + b) / (1.0 + d) * dd::cr_pow(u, 1.0 + d) +
@@ -41,7 +47,7 @@ __device__ __forceinline__ double F_H(double rho) {
 }
 
 // potential.cpp:64-98
-__device__ __forceinline__ double f_Pd(double r) {
+A2C_EAM double f_Pd(double r) {
   r = r / 5.0;
   double ra = r;
   ra = ra * (r * (r - 2.7267629107325706) + 1.8716766113599643);
@@ -60,14 +66,14 @@ __device__ __forceinline__ double f_Pd(double r) {
 }
 
 // potential.cpp:105-119
-__device__ __forceinline__ double f_H(double r) {
+A2C_EAM double f_H(double r) {
   if (r <= 0.0) return 0.0;
   if (r > 5.35) return 0.009986990526578 * dd::fexp(-0.013075667086408 / 0.009986990526578 * (r - 5.35));
   return 11.0025 * dd::fexp(-1.30927 * r);
 }
 
 // potential.cpp:126-155
-__device__ __forceinline__ double phi_Pd(double r) {
+A2C_EAM double phi_Pd(double r) {
   r = r / 5.0;
   double y = -79415.24035137112 * (r - 1.0699996145674568);
   y = y * (r - 1.06015072612581);
@@ -85,7 +91,7 @@ __device__ __forceinline__ double phi_Pd(double r) {
 }
 
 // potential.cpp:162-177
-__device__ __forceinline__ double phi_PdH(double r) {
+A2C_EAM double phi_PdH(double r) {
   if (r <= 0.0) return 0.0;
   if (r > 5.35) return -3.353001113951400e-04 * dd::fexp(7.147062196813336e-04 / -3.353001113951400e-04 * (r - 5.35));
   const double D = 0.2494540, alpha = 4.82613, beta = 2.13158, r0 = 1.50964;
@@ -93,7 +99,7 @@ __device__ __forceinline__ double phi_PdH(double r) {
 }
 
 // potential.cpp:185-200
-__device__ __forceinline__ double phi_H(double r) {
+A2C_EAM double phi_H(double r) {
   if (r <= 0.0) return 0.0;
   if (r > 5.35) return -0.003702722457147 * dd::fexp(0.005465945471933 / -0.003702722457147 * (r - 5.35));
   const double D = 0.0661496, alpha = 3.67263, beta = 1.47797, r0 = 2.51980;
@@ -102,13 +108,15 @@ __device__ __forceinline__ double phi_H(double r) {
 
 // Central finite differences with step eps (potential.cpp:40, 59, 100, 121,
 // 157, 179, 202).
-__device__ __forceinline__ double F_Pd_d(double x, double e) { return (F_Pd(x + e) - F_Pd(x - e)) / (2.0 * e); }
-__device__ __forceinline__ double F_H_d(double x, double e) { return (F_H(x + e) - F_H(x - e)) / (2.0 * e); }
-__device__ __forceinline__ double f_Pd_d(double x, double e) { return (f_Pd(x + e) - f_Pd(x - e)) / (2.0 * e); }
-__device__ __forceinline__ double f_H_d(double x, double e) { return (f_H(x + e) - f_H(x - e)) / (2.0 * e); }
-__device__ __forceinline__ double phi_Pd_d(double x, double e) { return (phi_Pd(x + e) - phi_Pd(x - e)) / (2.0 * e); }
-__device__ __forceinline__ double phi_PdH_d(double x, double e) { return (phi_PdH(x + e) - phi_PdH(x - e)) / (2.0 * e); }
-__device__ __forceinline__ double phi_H_d(double x, double e) { return (phi_H(x + e) - phi_H(x - e)) / (2.0 * e); }
+A2C_EAM double F_Pd_d(double x, double e) { return (F_Pd(x + e) - F_Pd(x - e)) / (2.0 * e); }
+A2C_EAM double F_H_d(double x, double e) { return (F_H(x + e) - F_H(x - e)) / (2.0 * e); }
+A2C_EAM double f_Pd_d(double x, double e) { return (f_Pd(x + e) - f_Pd(x - e)) / (2.0 * e); }
+A2C_EAM double f_H_d(double x, double e) { return (f_H(x + e) - f_H(x - e)) / (2.0 * e); }
+A2C_EAM double phi_Pd_d(double x, double e) { return (phi_Pd(x + e) - phi_Pd(x - e)) / (2.0 * e); }
+A2C_EAM double phi_PdH_d(double x, double e) { return (phi_PdH(x + e) - phi_PdH(x - e)) / (2.0 * e); }
+A2C_EAM double phi_H_d(double x, double e) { return (phi_H(x + e) - phi_H(x - e)) / (2.0 * e); }
 
 }  // namespace eam64
 }  // namespace a2c
+
+#undef A2C_EAM

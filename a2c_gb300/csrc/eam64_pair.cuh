@@ -1,0 +1,181 @@
+// The pair functions of eam64.cuh as the FP64 pair kernels evaluate them:
+// the same bits (tests/test_fp64_pair_forms.py compares them on the host)
+// in fewer FP64 operations.  GB300's FP64 pipe takes two lanes per SM and
+// clock, so a warp's FP64 instruction occupies its scheduler's share of the
+// pipe for 64 clocks and the count of such instructions is the time of
+// these kernels.  What is spared:
+//   * phi_Pd(x) holds f_Pd(x1) with x1 = (x / 5) * 5, and f_Pd depends on
+//     its argument through r = x / 5 alone.  x1 is x or its neighbor; x1 / 5
+//     rounds to the same r whenever x's significand is 1.25 or more (then
+//     ulp(r) = ulp(x) / 4 and x1 / 5 lies within 0.4 ulp(r) of r), and often
+//     otherwise, so the f_Pd values of f_Pd' serve phi_Pd' too: three
+//     evaluations in place of five outside [2, 2.5) and [4, 5) A;
+//   * x / 5 by two operations and the other quotients by four, correctly
+//     rounded (div5, Divisor);
+//   * comparisons with the switch radii on the bits, by integer operations.
+// The fast forms hold for kPairMin <= x < kPairMax (in_pair_range); callers
+// take eam64.cuh's functions elsewhere.
+#pragma once
+
+#include "eam64.cuh"
+
+#if defined(__CUDACC__)
+#define A2C_EAM __host__ __device__ __forceinline__
+#else
+#define A2C_EAM inline
+#endif
+
+namespace a2c {
+namespace eam64 {
+
+constexpr double kPairMin = 0.0625, kPairMax = 128.0;
+
+// a > b for positive finite doubles
+A2C_EAM bool above(double a, double b) {
+  const int ha = dd::hi_word(a), hb = dd::hi_word(b);
+  return ha > hb || (ha == hb && (unsigned)dd::lo_word(a) > (unsigned)dd::lo_word(b));
+}
+// kPairMin <= x < kPairMax, both powers of two
+A2C_EAM bool in_pair_range(double x) {
+  return (unsigned)(dd::hi_word(x) - 0x3fb00000) < (unsigned)(0x40600000 - 0x3fb00000);
+}
+
+// x / 5, correctly rounded for normal results: 1/5 as hi + lo, one fused
+// operation on the exact product's head.  A quotient by 5 is at least 1/20
+// ulp from every midpoint of two doubles (x - 5 m is a multiple of 1/16 ulp
+// of x, and not zero, for a midpoint m), the sum below is within 2^-50 ulp
+// of it before its one rounding.
+A2C_EAM double div5(double x) { return fma(x, 0.2, x * -1.1102230246251565e-17); }
+
+// Quotients by one divisor b, correctly rounded: z = 1/b rounded to
+// nearest, with its error zl a quotient q within one ulp, then Markstein's
+// correction q + (a - q b) z (Markstein 1990, theorem on final rounding).
+// The remainder must not underflow: exact_for(a) is the range of
+// numerators (zero included) for divisors between 2^-100 and 2^100.
+struct Divisor {
+  double b, z, zl;
+};
+A2C_EAM Divisor divisor(double b) {
+  Divisor d;
+  d.b = b;
+#if defined(__CUDA_ARCH__)
+  d.z = __drcp_rn(b);
+#else
+  d.z = 1.0 / b;
+#endif
+  d.zl = fma(-b, d.z, 1.0) * d.z;
+  return d;
+}
+A2C_EAM double quotient(double a, const Divisor &d) {
+  const double q = fma(a, d.z, a * d.zl);
+  return fma(fma(-d.b, q, a), d.z, q);
+}
+A2C_EAM bool exact_for(double a) {
+  const unsigned h = (unsigned)dd::hi_word(a) & 0x7fffffffu;
+  return h - 0x10000000u < 0x60000000u || (h | (unsigned)dd::lo_word(a)) == 0;  // 2^-767 <= |a| < 2^769, or 0
+}
+// a / d.b for any a
+A2C_EAM double divide(double a, const Divisor &d) { return exact_for(a) ? quotient(a, d) : a / d.b; }
+
+// f_Pd as a function of r = x / 5 (potential.cpp:64-98)
+A2C_EAM double f_Pd_at(double r) {
+  const double x1 = r * 5.0;
+  if (above(x1, 5.0)) return 0.001510569378297 * dd::fexp(-0.077976566126292 / 0.001510569378297 * (x1 - 5.0));
+  double ra = r;
+  ra = ra * (r * (r - 2.7267629107325706) + 1.8716766113599643);
+  ra = ra * (r * (r - 2.50290548851635) + 1.668549182690922);
+  ra = ra * (r * (r - 2.0924467509943674) + 1.3150372774478005);
+  ra = ra * (r * (r - 1.564328475106985) + 0.8987511149780485);
+  ra = ra * (r * (r - 1.009780903403673) + 0.5124363774128722);
+  ra = ra * (r * (r - 0.5304054524800665) + 0.2169886022464641);
+  ra = ra * (r * (r - 0.1356566408715063) + 0.035852347523891395);
+  return -0.02972698211669922 +
+         r * (0.6676807403564453 + r * (-255.8965835571289 + r * (14673.409149169922 + -2.597301181336601e7 * ra)));
+}
+// x1 / 5 for x1 = r * 5, r = x / 5: r itself where x's significand is 1.25
+// or more (see above)
+A2C_EAM double second_fifth(double x, double r) {
+  return (dd::hi_word(x) & 0xfffff) >= 0x40000 ? r : div5(r * 5.0);
+}
+// phi_Pd with r = x / 5 and f = f_Pd(x1) (potential.cpp:126-155)
+A2C_EAM double phi_Pd_at(double r, double f) {
+  const double x1 = r * 5.0;
+  if (above(x1, 5.05)) return -0.016958780164980 * dd::fexp(0.089019679316328 / -0.016958780164980 * (x1 - 5.05));
+  double y = -79415.24035137112 * (r - 1.0699996145674568);
+  y = y * (r - 1.06015072612581);
+  y = y * (r - 0.42433991011376526);
+  y = y * (r + 0.06169160085238687);
+  y = y * (r * (r - 2.0586473420376348) + 1.0683922574015199);
+  y = y * (r * (r - 1.6696359816422877) + 0.7337878627470482);
+  y = y * (r * (r - 1.1690370066230809) + 0.3909805777737639);
+  y = y * (r * (r - 0.2635598721249787) + 0.033551116514910245);
+  return y + (2 * 0.251546) * f;
+}
+A2C_EAM double f_Pd_pos(double x) { return f_Pd_at(div5(x)); }
+A2C_EAM double f_H_pos(double x) {
+  if (above(x, 5.35)) return 0.009986990526578 * dd::fexp(-0.013075667086408 / 0.009986990526578 * (x - 5.35));
+  return 11.0025 * dd::fexp(-1.30927 * x);
+}
+A2C_EAM double phi_PdH_pos(double x) {
+  if (above(x, 5.35))
+    return -3.353001113951400e-04 * dd::fexp(7.147062196813336e-04 / -3.353001113951400e-04 * (x - 5.35));
+  const double D = 0.2494540, alpha = 4.82613, beta = 2.13158, r0 = 1.50964, t = x - r0;
+  return D * (beta * dd::fexp(-alpha * t) - alpha * dd::fexp(-beta * t));
+}
+A2C_EAM double phi_H_pos(double x) {
+  if (above(x, 5.35)) return -0.003702722457147 * dd::fexp(0.005465945471933 / -0.003702722457147 * (x - 5.35));
+  const double D = 0.0661496, alpha = 3.67263, beta = 1.47797, r0 = 2.51980, t = x - r0;
+  return D * (beta * dd::fexp(-alpha * t) - alpha * dd::fexp(-beta * t));
+}
+
+// What one quadrature point of a pair at distance s takes from the pair
+// functions: da, db the density derivatives that F'(rho_i) and F'(rho_j)
+// multiply (f' of the neighbor's and of the site's own species), the pair
+// function and its derivative; derivatives by central differences of step e
+// (h: the divisor 2 e).
+struct PairPoint {
+  double da, db, phi, dphi;
+};
+A2C_EAM PairPoint pair_point(bool iPd, bool jPd, double s, double e, const Divisor &h) {
+  const double xp = s + e, xm = s - e;
+  PairPoint p;
+  if (!in_pair_range(xp) || !in_pair_range(xm)) {
+    const double fP = (iPd || jPd) ? f_Pd_d(s, e) : 0.0, fH = (iPd && jPd) ? 0.0 : f_H_d(s, e);
+    p.da = jPd ? fP : fH;
+    p.db = iPd ? fP : fH;
+    p.phi = (iPd && jPd) ? phi_Pd(s) : (iPd || jPd) ? phi_PdH(s) : phi_H(s);
+    p.dphi = (iPd && jPd) ? phi_Pd_d(s, e) : (iPd || jPd) ? phi_PdH_d(s, e) : phi_H_d(s, e);
+    return p;
+  }
+  if (iPd && jPd) {
+    const double r = div5(s), rp = div5(xp), rm = div5(xm);
+    double fp = f_Pd_at(rp), fm = f_Pd_at(rm);
+    p.da = p.db = divide(fp - fm, h);
+    p.phi = phi_Pd_at(r, f_Pd_at(second_fifth(s, r)));
+    const double rp2 = second_fifth(xp, rp), rm2 = second_fifth(xm, rm);
+    if (rp2 != rp) fp = f_Pd_at(rp2);
+    if (rm2 != rm) fm = f_Pd_at(rm2);
+    p.dphi = divide(phi_Pd_at(rp, fp) - phi_Pd_at(rm, fm), h);
+  } else if (iPd || jPd) {
+    const double fP = divide(f_Pd_pos(xp) - f_Pd_pos(xm), h), fH = divide(f_H_pos(xp) - f_H_pos(xm), h);
+    p.da = jPd ? fP : fH;
+    p.db = iPd ? fP : fH;
+    p.phi = phi_PdH_pos(s);
+    p.dphi = divide(phi_PdH_pos(xp) - phi_PdH_pos(xm), h);
+  } else {
+    p.da = p.db = divide(f_H_pos(xp) - f_H_pos(xm), h);
+    p.phi = phi_H_pos(s);
+    p.dphi = divide(phi_H_pos(xp) - phi_H_pos(xm), h);
+  }
+  return p;
+}
+// the density a neighbor at distance s adds at one point
+A2C_EAM double density_point(bool jPd, double s) {
+  if (!in_pair_range(s)) return jPd ? f_Pd(s) : f_H(s);
+  return jPd ? f_Pd_pos(s) : f_H_pos(s);
+}
+
+}  // namespace eam64
+}  // namespace a2c
+
+#undef A2C_EAM

@@ -1,9 +1,23 @@
 // FP64 plain-form kernels: pass 1 (site electron density), pass 2 (energy
 // and gradient gather) and the occupancy gradient.  Compiled with
-// -fmad=false.  One thread owns one site and walks its neighbor list in
-// order, so every per-site sum is formed in the reference's order
-// (electrondensity.cpp:20-49, minimizer.cpp:162-351, 658-789); the only
-// difference from the CPU arithmetic is the device exp/pow/log.
+// -fmad=false.  Every per-site sum is formed term by term in the
+// reference's order (electrondensity.cpp:20-49, minimizer.cpp:162-351,
+// 658-789); the only difference from the CPU arithmetic is the device
+// exp/pow/log.
+//
+// Pass 1 and pass 2 evaluate a warp's quadrature points side by side and
+// then add their terms in order: S sites share a warp, a round takes the
+// next neighbors of each (32 pairs in pass 1, 8 in pass 2), the lanes
+// evaluate the round's points -- 12 per pair, whatever site they belong to
+// -- into shared memory, and the lanes that own a site's sums (one in pass
+// 1; x, y, z and sigma + V in pass 2) add them.  Why: the FP64 pipe (two
+// lanes per SM and clock) bounds these kernels, a warp's instruction holds
+// it for 32 lanes whether they work or not, and one thread per site left
+// a 512-site system 16 warps, each with 960 points in a row.  S trades the
+// two ends (rho_sites_per_warp, grad_sites_per_warp).  With the pair
+// functions' fewer operations (eam64_pair.cuh) an evaluation takes, one
+// thread per site -> now: 15.3 -> 0.69 ms at 512 sites, 23.0 -> 8.7 ms at
+// 10,296, 210.6 -> 149.7 ms at 262,144.
 //
 // Geometry: for quadrature point k = 2m (+sqrt(3)) or 2m+1 (-sqrt(3)) only
 // coordinate m of R^6 is non-zero, so r_k differs from the pair's base
@@ -13,8 +27,9 @@
 // forms used below are bit-identical to it.
 #include <algorithm>
 #include <mutex>
+#include <vector>
 
-#include "eam64.cuh"
+#include "eam64_pair.cuh"
 
 #include "internal.cuh"
 
@@ -79,191 +94,325 @@ __device__ __forceinline__ double point(const PairGeo &g, int k, double r[3], in
   return sqrt(s2);
 }
 
-// Fsigma += dot(v, xi0): xi0 has one non-zero component, +-sqrt(3) at
-// index comp (k < 6), or is all zero (k >= 6), and x + (+-0) == x.
-__device__ __forceinline__ void accum(double Fq[3], double &Fs, double c, const double r[3], int k, int comp,
-                                      double xi0) {
-  const double v0 = c * r[0], v1 = c * r[1], v2 = c * r[2];
-  Fq[0] = Fq[0] + v0;
-  Fq[1] = Fq[1] + v1;
-  Fq[2] = Fq[2] + v2;
-  if (k < 6) {
-    const double vc = (comp == 0) ? v0 : (comp == 1) ? v1 : v2;
-    Fs = Fs + vc * xi0;
-  }
+constexpr unsigned kAll = 0xffffffffu;
+constexpr double kSqrt2 = 1.4142135623730951, kSqrt3 = 1.7320508075688772;
+
+// A neighbor's coordinates (image applied) and displacement sqrt(6) sigma
+// in the reference's operation order.
+__device__ __forceinline__ double displacement(double sigma) { return (kSqrt2 * sigma) * kSqrt3; }
+
+// |r_k| of quadrature point k (quadrature.cpp:111-132 ordering): component m
+// of the pair vector replaced by rm.
+__device__ __forceinline__ double radius(int m, double rm, double d20, double d21, double d22) {
+  const double q = rm * rm;
+  return sqrt((m == 0 ? q : d20) + (m == 1 ? q : d21) + (m == 2 ? q : d22));
 }
 
-// Pass 1 for site s (electrondensity.cpp:20-49).
-__device__ __forceinline__ void density_site(const SiteArgs &a, int64_t s, bool iPd, const double *box) {
-  const double qi[3] = {a.X[4 * s], a.X[4 * s + 1], a.X[4 * s + 2]};
-  const double ui = (1.4142135623730951 * a.X[4 * s + 3]) * 1.7320508075688772;
-  const int64_t b = a.off[s], m = b + a.npd[s], e = a.off[s + 1];
+// The site a warp's slot works on and its instance (LIST: batched launch).
+struct Site64 {
+  int64_t s;
+  bool live, iPd;
+  const double *box;
+  double T;
+};
+template <bool LIST>
+__device__ __forceinline__ Site64 site64(const SiteArgs &a, int64_t k, int64_t n) {
+  Site64 r;
+  r.live = k < n;
+  if (LIST) {
+    r.s = r.live ? a.bv.list[k] : 0;
+    const InstGeo &g = a.bv.geo[r.live ? a.bv.inst[r.s] : 0];
+    r.iPd = r.s - g.start < g.nPd;
+    r.box = g.S;
+    r.T = g.T;
+  } else {
+    r.s = r.live ? k : 0;
+    r.iPd = r.s < a.nPd;
+    r.box = a.box;
+    r.T = a.T;
+  }
+  return r;
+}
+
+// A listed pair's inputs, loaded one round ahead of their use.
+struct Neighbor64 {
+  uint32_t en;
+  double q[3], sigma, x, Fp;
+};
+template <bool FP>
+__device__ __forceinline__ Neighbor64 load_neighbor(const SiteArgs &a, int64_t t, bool valid) {
+  Neighbor64 v{};
+  if (!valid) return v;
+  v.en = __ldg(&a.nbr[t]);
+  const int64_t j = v.en & kIdMask;
+  const double *X = a.X + 4 * j;  // 8-byte loads: the caller's X is aligned to no more
+  v.q[0] = __ldg(X);
+  v.q[1] = __ldg(X + 1);
+  v.q[2] = __ldg(X + 2);
+  v.sigma = __ldg(X + 3);
+  v.x = __ldg(&a.occ[j]);
+  if (FP) v.Fp = __ldg(&a.Fp[j]);
+  return v;
+}
+__device__ __forceinline__ void apply_image(Neighbor64 &v, const double *box) {
+  const uint32_t c = v.en >> kIdBits;
+  if (c == kNoShift) return;
+  const int m0 = (int)(c % 3u) - 1, m1 = (int)((c / 3u) % 3u) - 1, m2 = (int)(c / 9u) - 1;
+  if (m0) v.q[0] = v.q[0] + m0 * box[0];
+  if (m1) v.q[1] = v.q[1] + m1 * box[1];
+  if (m2) v.q[2] = v.q[2] + m2 * box[2];
+}
+
+constexpr int kWarps = 4;  // warps per block of both passes
+
+// ---------------------------------------------------------------- pass 1
+constexpr int kRhoPairs = 32, kRhoRow = 13;  // 12 terms per pair, padded against bank conflicts
+struct RhoShared {
+  double qp[32][6];  // per site q + u, q - u of each coordinate
+  double qj[3][kRhoPairs], D[3][kRhoPairs], D2[3][kRhoPairs], uj[kRhoPairs], xj[kRhoPairs];
+  double term[kRhoPairs * kRhoRow];
+};
+
+template <int S, bool LIST>
+__global__ void __launch_bounds__(32 * kWarps) k_density64(SiteArgs a) {
+  constexpr int NB = kRhoPairs / S;  // pairs of one site per round
+  extern __shared__ double2 smem64[];
+  RhoShared &sh = reinterpret_cast<RhoShared *>(smem64)[threadIdx.x / 32];
+  const int lane = threadIdx.x % 32, slot = lane / NB, sub = lane % NB;
+  const int64_t n = LIST ? (int64_t)*a.bv.count : (int64_t)a.nPd + a.nH;
   const double W = a.W;
-  double rho = 0.0;
-  for (int64_t t = b; t < m; ++t) {
-    const uint32_t en = a.nbr[t];
-    const int64_t j = en & kIdMask;
-    double qj[3];
-    image_pos(a, box, en, qj);
-    const double uj = (1.4142135623730951 * a.X[4 * j + 3]) * 1.7320508075688772;
-    PairGeo g;
-    make_geo(qi, ui, qj, uj, g);
+  const int64_t stride = (int64_t)gridDim.x * kWarps * S;
+  for (int64_t first = ((int64_t)blockIdx.x * kWarps + threadIdx.x / 32) * S; first < n; first += stride) {
+    const Site64 st = site64<LIST>(a, first + slot, n);
+    double qi[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) qi[c] = a.X[4 * st.s + c];
+    const double ui = displacement(a.X[4 * st.s + 3]);
+    __syncwarp();
+    if (sub == 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        sh.qp[slot][2 * c] = qi[c] + ui;
+        sh.qp[slot][2 * c + 1] = qi[c] + (-ui);
+      }
+    }
+    const int64_t b = a.off[st.s], npd = a.npd[st.s], e = a.off[st.s + 1];
+    double rho = 0.0;  // in lane s for site slot s (s < S)
+    for (int part = 0; part < 2; ++part) {  // the Pd neighbors, then the H neighbors
+      const bool jPd = part == 0;
+      const int64_t t0 = jPd ? b : b + npd;
+      const int cnt = st.live ? (int)(jPd ? npd : e - b - npd) : 0;
+      const int rounds = __reduce_max_sync(kAll, (cnt + NB - 1) / NB);
+      Neighbor64 v = load_neighbor<false>(a, t0 + sub, sub < cnt);
+      for (int r = 0; r < rounds; ++r) {
+        const bool valid = r * NB + sub < cnt;
+        if (valid) {
+          apply_image(v, st.box);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const double D = qi[c] - v.q[c];
+            sh.qj[c][lane] = v.q[c];
+            sh.D[c][lane] = D;
+            sh.D2[c][lane] = D * D;
+          }
+          sh.uj[lane] = displacement(v.sigma);
+          sh.xj[lane] = v.x;
+        }
+        const unsigned vm = __ballot_sync(kAll, valid);
+        const int nx = (r + 1) * NB + sub;
+        v = load_neighbor<false>(a, t0 + nx, nx < cnt);
+        __syncwarp();
 #pragma unroll 1
-    for (int k = 0; k < 12; ++k) {
-      double r[3], xi0;
-      int comp;
-      const double sk = point(g, k, r, comp, xi0);
-      rho = rho + eam64::f_Pd(sk) * W;
+        for (int p = lane; p < kRhoPairs * 12; p += 32) {
+          const int q = p / 12, k = p - 12 * q;
+          if (!(vm >> q & 1u)) continue;
+          const int m = (k < 6 ? k : k - 6) >> 1, sgn = k & 1;
+          const double u = sh.uj[q];
+          const double rm = k < 6 ? sh.qp[q / NB][2 * m + sgn] - sh.qj[m][q] : sh.D[m][q] - (sgn ? -u : u);
+          const double f = eam64::density_point(jPd, radius(m, rm, sh.D2[0][q], sh.D2[1][q], sh.D2[2][q]));
+          sh.term[q * kRhoRow + k] = (jPd ? f : sh.xj[q] * f) * W;
+        }
+        __syncwarp();
+        if (lane < S) {
+#pragma unroll 1
+          for (int i = 0; i < NB; ++i) {
+            const int q = lane * NB + i;
+            if (!(vm >> q & 1u)) break;
+            const double *t = sh.term + q * kRhoRow;
+#pragma unroll
+            for (int k = 0; k < 12; ++k) rho = rho + t[k];
+          }
+        }
+        __syncwarp();
+      }
+    }
+    const Site64 own = site64<LIST>(a, first + lane, n);
+    if (lane < S && own.live) {
+      a.rho[own.s] = rho;
+      a.Fp[own.s] = own.iPd ? eam64::F_Pd_d(rho, a.eps) : eam64::F_H_d(rho, a.eps);
+      if (!isfinite(rho)) atomicOr(a.status, kStatusNonfinite);
     }
   }
-  for (int64_t t = m; t < e; ++t) {
-    const uint32_t en = a.nbr[t];
-    const int64_t j = en & kIdMask;
-    double qj[3];
-    image_pos(a, box, en, qj);
-    const double uj = (1.4142135623730951 * a.X[4 * j + 3]) * 1.7320508075688772;
-    const double xj = a.occ[j];
-    PairGeo g;
-    make_geo(qi, ui, qj, uj, g);
-#pragma unroll 1
-    for (int k = 0; k < 12; ++k) {
-      double r[3], xi0;
-      int comp;
-      const double sk = point(g, k, r, comp, xi0);
-      rho = rho + (xj * eam64::f_H(sk)) * W;
-    }
-  }
-  a.rho[s] = rho;
-  a.Fp[s] = iPd ? eam64::F_Pd_d(rho, a.eps) : eam64::F_H_d(rho, a.eps);
-  if (!isfinite(rho)) atomicOr(a.status, kStatusNonfinite);
 }
 
-__global__ void __launch_bounds__(kBlock) k_density64(SiteArgs a) {
-  const int64_t N = (int64_t)a.nPd + a.nH;
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= N) return;
-  density_site(a, s, s < a.nPd, a.box);
-}
-
-// Pass 2.  Per pair-point the three gradient terms of minimizer.cpp:180-190
-// (and their Pd-H / H-Pd / H-H forms) are, with x_j = 1 for a Pd neighbor:
+// ---------------------------------------------------------------- pass 2
+// Per pair-point the three gradient terms of minimizer.cpp:180-190 (and
+// their Pd-H / H-Pd / H-H forms) are, with x_j = 1 for a Pd neighbor:
 //   c1 = (((x_j*W)*F'_A(rho_i))*f'_B(s))/s
 //   c2 = (((x_j*W)*F'_B(rho_j))*f'_A(s))/s
 //   c3 = ((x_j*W)*phi'_AB(s))/s
 // and the energy term ((0.5*x_i)*x_j)*W*phi_AB(s); the factors equal to 1
 // for Pd sites multiply exactly, so one form serves all four pair types.
-__device__ __forceinline__ void gradient_site(const SiteArgs &a, int64_t s, bool iPd, const double *box, double T) {
-  const double qi[3] = {a.X[4 * s], a.X[4 * s + 1], a.X[4 * s + 2]};
-  const double sigmai = a.X[4 * s + 3];
-  const double ui = (1.4142135623730951 * sigmai) * 1.7320508075688772;
-  const double xi = a.occ[s];
-  const double rhoi = a.rho[s];
-  const double Fpi = a.Fp[s];
+// A point's products with its vector's components are staged as 12 rows
+// (c1, c2, c3 times x, y, z and, for the points that move site i, the moved
+// component times its xi0 = +-sqrt(3)); the sigma rows of the six points
+// without a sigma part hold the pair's 12 energy terms, in order, so that
+// the lane with sigma also sums V.
+constexpr int kGradPairs = 8, kGradPts = 12 * kGradPairs;
+constexpr int kGradRow = kGradPts + 3;  // the padding keeps the adding lanes off each other's banks
+struct GradShared {
+  double qp[kGradPairs][6];
+  double qj[3][kGradPairs], D[3][kGradPairs], D2[3][kGradPairs], uj[kGradPairs];
+  double A1[kGradPairs], A2[kGradPairs], A3[kGradPairs], AV[kGradPairs];
+  double pt[12 * kGradRow];
+};
+
+template <int S, bool LIST>
+__global__ void __launch_bounds__(32 * kWarps) k_gradient64(SiteArgs a) {
+  constexpr int NB = kGradPairs / S;
+  extern __shared__ double2 smem64[];
+  GradShared &sh = reinterpret_cast<GradShared *>(smem64)[threadIdx.x / 32];
+  const int lane = threadIdx.x % 32;
+  const int slot = (lane % kGradPairs) / NB, sub = lane % NB;  // pair role: lanes 0-7
+  const int own = (lane / 4) % S, comp = lane & 3;              // adding role: lanes 0 to 4 S - 1
+  const bool adds = lane < 4 * S;
+  const int64_t n = LIST ? (int64_t)*a.bv.count : (int64_t)a.nPd + a.nH;
   const double W = a.W, eps = a.eps;
-  const int64_t b = a.off[s], m = b + a.npd[s], e = a.off[s + 1];
-  double V = 0.0;
-  V = V + (iPd ? eam64::F_Pd(rhoi) : xi * eam64::F_H(rhoi));
-  double Fq[3] = {0.0, 0.0, 0.0}, Fs = 0.0;
-  const double half_xi = 0.5 * xi;
-
-  // Pd neighbors (PdPd for a Pd site, HPd for an H site)
-  for (int64_t t = b; t < m; ++t) {
-    const uint32_t en = a.nbr[t];
-    const int64_t j = en & kIdMask;
-    double qj[3];
-    image_pos(a, box, en, qj);
-    const double uj = (1.4142135623730951 * a.X[4 * j + 3]) * 1.7320508075688772;
-    const double Fpj = a.Fp[j];
-    PairGeo g;
-    make_geo(qi, ui, qj, uj, g);
-#pragma unroll 1
-    for (int k = 0; k < 12; ++k) {
-      double r[3], xi0;
-      int comp;
-      const double sk = point(g, k, r, comp, xi0);
-      if (iPd) {
-        const double fd = eam64::f_Pd_d(sk, eps);
-        accum(Fq, Fs, ((W * Fpi) * fd) / sk, r, k, comp, xi0);
-        accum(Fq, Fs, ((W * Fpj) * fd) / sk, r, k, comp, xi0);
-        V = V + (0.5 * W) * eam64::phi_Pd(sk);
-        accum(Fq, Fs, (W * eam64::phi_Pd_d(sk, eps)) / sk, r, k, comp, xi0);
-      } else {
-        accum(Fq, Fs, ((W * Fpi) * eam64::f_Pd_d(sk, eps)) / sk, r, k, comp, xi0);
-        accum(Fq, Fs, ((W * Fpj) * eam64::f_H_d(sk, eps)) / sk, r, k, comp, xi0);
-        V = V + (half_xi * W) * eam64::phi_PdH(sk);
-        accum(Fq, Fs, (W * eam64::phi_PdH_d(sk, eps)) / sk, r, k, comp, xi0);
+  const eam64::Divisor h = eam64::divisor(2.0 * eps);
+  const int64_t stride = (int64_t)gridDim.x * kWarps * S;
+  for (int64_t first = ((int64_t)blockIdx.x * kWarps + threadIdx.x / 32) * S; first < n; first += stride) {
+    const Site64 st = site64<LIST>(a, first + slot, n);
+    double qi[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) qi[c] = a.X[4 * st.s + c];
+    const double ui = displacement(a.X[4 * st.s + 3]);
+    const double half_xi = 0.5 * a.occ[st.s], Fpi = a.Fp[st.s];
+    __syncwarp();
+    if (lane < kGradPairs && sub == 0) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        sh.qp[slot][2 * c] = qi[c] + ui;
+        sh.qp[slot][2 * c + 1] = qi[c] + (-ui);
       }
     }
-  }
-  // H neighbors (PdH for a Pd site, HH for an H site)
-  for (int64_t t = m; t < e; ++t) {
-    const uint32_t en = a.nbr[t];
-    const int64_t j = en & kIdMask;
-    double qj[3];
-    image_pos(a, box, en, qj);
-    const double uj = (1.4142135623730951 * a.X[4 * j + 3]) * 1.7320508075688772;
-    const double Fpj = a.Fp[j];
-    const double xj = a.occ[j];
-    const double xW = xj * W;
-    PairGeo g;
-    make_geo(qi, ui, qj, uj, g);
+    const unsigned pdmask = __ballot_sync(kAll, st.iPd);  // bit q: pair q's site is Pd
+    const int64_t b = a.off[st.s], npd = a.npd[st.s], e = a.off[st.s + 1];
+    const Site64 me = site64<LIST>(a, first + own, n);
+    double acc = 0.0, V = 0.0;  // the component's sum; V in the sigma lane
+    if (adds && comp == 3 && me.live) {
+      const double r = a.rho[me.s];
+      V = V + (me.iPd ? eam64::F_Pd(r) : a.occ[me.s] * eam64::F_H(r));
+    }
+    for (int part = 0; part < 2; ++part) {
+      const bool jPd = part == 0;
+      const int64_t t0 = jPd ? b : b + npd;
+      const int cnt = (lane < kGradPairs && st.live) ? (int)(jPd ? npd : e - b - npd) : 0;
+      const int rounds = __reduce_max_sync(kAll, (cnt + NB - 1) / NB);
+      Neighbor64 v = load_neighbor<true>(a, t0 + sub, sub < cnt);
+      for (int r = 0; r < rounds; ++r) {
+        const bool valid = r * NB + sub < cnt;
+        if (valid) {
+          apply_image(v, st.box);
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const double D = qi[c] - v.q[c];
+            sh.qj[c][lane] = v.q[c];
+            sh.D[c][lane] = D;
+            sh.D2[c][lane] = D * D;
+          }
+          sh.uj[lane] = displacement(v.sigma);
+          const double xW = v.x * W;
+          sh.A1[lane] = xW * Fpi;
+          sh.A2[lane] = xW * v.Fp;
+          sh.A3[lane] = xW;
+          sh.AV[lane] = (half_xi * v.x) * W;
+        }
+        const unsigned vm = __ballot_sync(kAll, valid);
+        const int nx = (r + 1) * NB + sub;
+        v = load_neighbor<true>(a, t0 + nx, nx < cnt);
+        __syncwarp();
 #pragma unroll 1
-    for (int k = 0; k < 12; ++k) {
-      double r[3], xi0;
-      int comp;
-      const double sk = point(g, k, r, comp, xi0);
-      if (iPd) {
-        accum(Fq, Fs, ((xW * Fpi) * eam64::f_H_d(sk, eps)) / sk, r, k, comp, xi0);
-        accum(Fq, Fs, ((xW * Fpj) * eam64::f_Pd_d(sk, eps)) / sk, r, k, comp, xi0);
-        V = V + ((0.5 * xj) * W) * eam64::phi_PdH(sk);
-        accum(Fq, Fs, (xW * eam64::phi_PdH_d(sk, eps)) / sk, r, k, comp, xi0);
-      } else {
-        const double fd = eam64::f_H_d(sk, eps);
-        accum(Fq, Fs, ((xW * Fpi) * fd) / sk, r, k, comp, xi0);
-        accum(Fq, Fs, ((xW * Fpj) * fd) / sk, r, k, comp, xi0);
-        V = V + ((half_xi * xj) * W) * eam64::phi_H(sk);
-        accum(Fq, Fs, (xW * eam64::phi_H_d(sk, eps)) / sk, r, k, comp, xi0);
+        for (int p = lane; p < kGradPts; p += 32) {
+          const int q = p / 12, k = p - 12 * q;
+          if (!(vm >> q & 1u)) continue;
+          const int m = (k < 6 ? k : k - 6) >> 1, sgn = k & 1;
+          const double u = sh.uj[q];
+          const double rm = k < 6 ? sh.qp[q / NB][2 * m + sgn] - sh.qj[m][q] : sh.D[m][q] - (sgn ? -u : u);
+          const double s = radius(m, rm, sh.D2[0][q], sh.D2[1][q], sh.D2[2][q]);
+          const eam64::PairPoint f = eam64::pair_point(pdmask >> q & 1u, jPd, s, eps, h);
+          double c[3] = {sh.A1[q] * f.da, sh.A2[q] * f.db, sh.A3[q] * f.dphi};
+          if (eam64::in_pair_range(s)) {
+            const eam64::Divisor ds = eam64::divisor(s);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) c[i] = eam64::divide(c[i], ds);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) c[i] = c[i] / s;
+          }
+          const double rx = m == 0 ? rm : sh.D[0][q], ry = m == 1 ? rm : sh.D[1][q], rz = m == 2 ? rm : sh.D[2][q];
+          const double xi0 = sgn ? -kSqrt3 : kSqrt3;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            double *o = sh.pt + 4 * i * kGradRow + p;
+            const double x = c[i] * rx, y = c[i] * ry, z = c[i] * rz;
+            o[0] = x;
+            o[kGradRow] = y;
+            o[2 * kGradRow] = z;
+            if (k < 6) o[3 * kGradRow] = (m == 0 ? x : m == 1 ? y : z) * xi0;
+          }
+          sh.pt[(4 * (k % 3) + 3) * kGradRow + 12 * q + 6 + k / 3] = sh.AV[q] * f.phi;
+        }
+        __syncwarp();
+        if (adds) {
+#pragma unroll 1
+          for (int i = 0; i < NB; ++i) {
+            const int q = own * NB + i;
+            if (!(vm >> q & 1u)) break;
+            const double *t = sh.pt + comp * kGradRow + 12 * q;
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+#pragma unroll
+              for (int c = 0; c < 3; ++c) acc = acc + t[4 * c * kGradRow + k];
+            double w = comp == 3 ? V : acc;  // the sigma lane turns to V
+#pragma unroll
+            for (int k = 6; k < 12; ++k)
+#pragma unroll
+              for (int c = 0; c < 3; ++c)
+                if (k < 10 || comp < 3) w = w + t[4 * c * kGradRow + k];
+            if (comp == 3) V = w;
+            else acc = w;
+          }
+        }
+        __syncwarp();
       }
     }
-  }
-  // minimizer.cpp:220-223 and 282-285
-  const double cq = (1.0 / T) * xi;
-  const double cs = ((1.0 / T) * 1.4142135623730951) * xi;
-  const double ce = ((3.0 * kB) / sigmai) * xi;
-  a.G[4 * s] = Fq[0] * cq;
-  a.G[4 * s + 1] = Fq[1] * cq;
-  a.G[4 * s + 2] = Fq[2] * cq;
-  a.G[4 * s + 3] = Fs * cs - ce;
-  a.Vs[s] = V;
-  a.Ss[s] = dd::cr_log(sigmai) * xi;
-  if (!isfinite(V) || !isfinite(Fs) || !isfinite(Fq[0] + Fq[1] + Fq[2])) atomicOr(a.status, kStatusNonfinite);
-}
-
-__global__ void __launch_bounds__(kBlock) k_gradient64(SiteArgs a) {
-  const int64_t N = (int64_t)a.nPd + a.nH;
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= N) return;
-  gradient_site(a, s, s < a.nPd, a.box, a.T);
-}
-
-// Batched: the listed sites, each with its instance's box, T and species.
-// Persistent grids (a fixed launch serves any list length, so the launch
-// can live in a CUDA graph while the list shrinks).
-__global__ void __launch_bounds__(kBlock) k_density64_list(SiteArgs a) {
-  const int n = *a.bv.count;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const int64_t s = a.bv.list[k];
-    const InstGeo &g = a.bv.geo[a.bv.inst[s]];
-    density_site(a, s, s - g.start < g.nPd, g.S);
-  }
-}
-
-__global__ void __launch_bounds__(kBlock) k_gradient64_list(SiteArgs a) {
-  const int n = *a.bv.count;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const int64_t s = a.bv.list[k];
-    const InstGeo &g = a.bv.geo[a.bv.inst[s]];
-    gradient_site(a, s, s - g.start < g.nPd, g.S, g.T);
+    // minimizer.cpp:220-223 and 282-285
+    const double f1 = __shfl_down_sync(kAll, acc, 1, 4), f2 = __shfl_down_sync(kAll, acc, 2, 4);
+    if (adds && me.live) {
+      const double xi = a.occ[me.s];
+      if (comp < 3) {
+        const double cq = (1.0 / me.T) * xi;
+        a.G[4 * me.s + comp] = acc * cq;
+        if (comp == 0 && !isfinite(acc + f1 + f2)) atomicOr(a.status, kStatusNonfinite);
+      } else {
+        const double sigmai = a.X[4 * me.s + 3];
+        const double cs = ((1.0 / me.T) * kSqrt2) * xi, ce = ((3.0 * kB) / sigmai) * xi;
+        a.G[4 * me.s + 3] = acc * cs - ce;
+        a.Vs[me.s] = V;
+        a.Ss[me.s] = dd::cr_log(sigmai) * xi;
+        if (!isfinite(V) || !isfinite(acc)) atomicOr(a.status, kStatusNonfinite);
+      }
+    }
   }
 }
 
@@ -280,7 +429,7 @@ __global__ void __launch_bounds__(kBlock) k_chem64(SiteArgs a, const double coeP
   const int64_t s = (int64_t)a.nPd + h;
   const double qi[3] = {a.X[4 * s], a.X[4 * s + 1], a.X[4 * s + 2]};
   const double ui = (1.4142135623730951 * a.X[4 * s + 3]) * 1.7320508075688772;
-  const double W = a.W, T = a.T, eps = a.eps;
+  const double W = a.W, T = a.T;
   const double *box = a.box;
   const int64_t b = a.off[s], m = b + a.npd[s], e = a.off[s + 1];
   const double nHPd = (double)(m - b);
@@ -307,8 +456,9 @@ __global__ void __launch_bounds__(kBlock) k_chem64(SiteArgs a, const double coeP
       double r[3], xi0;
       int comp;
       const double sk = point(g, k, r, comp, xi0);
-      sum = sum + WF * eam64::f_H(sk);
-      sum = sum + W * eam64::phi_PdH(sk);
+      const bool fast = eam64::in_pair_range(sk);
+      sum = sum + WF * (fast ? eam64::f_H_pos(sk) : eam64::f_H(sk));
+      sum = sum + W * (fast ? eam64::phi_PdH_pos(sk) : eam64::phi_PdH(sk));
     }
     const int64_t bj = a.off[j], mj = bj + a.npd[j], ej = a.off[j + 1];
     sum = sum + ((T * coePd0) * coePd2) * (double)(mj - bj);
@@ -330,8 +480,9 @@ __global__ void __launch_bounds__(kBlock) k_chem64(SiteArgs a, const double coeP
       double r[3], xi0;
       int comp;
       const double sk = point(g, k, r, comp, xi0);
-      sum = sum + xWF * eam64::f_H(sk);
-      sum = sum + xW * eam64::phi_H(sk);
+      const bool fast = eam64::in_pair_range(sk);
+      sum = sum + xWF * (fast ? eam64::f_H_pos(sk) : eam64::f_H(sk));
+      sum = sum + xW * (fast ? eam64::phi_H_pos(sk) : eam64::phi_H(sk));
     }
     const int64_t bj = a.off[j], mj = bj + a.npd[j], ej = a.off[j + 1];
     sum = sum + (((xj * T) * coeH0) * coeH2) * (double)(mj - bj);
@@ -387,68 +538,87 @@ SiteArgs site_args(a2c_gpp_ctx *c, const double *dX) {
   return a;
 }
 
-}  // namespace
+// Sites per warp.  Few sites: a warp per site or two, all lanes on its
+// points, though one to eight lanes then do its additions; many: the
+// additions of 8 (32 in pass 1) sites fill the lanes.  Measured on a GB300
+// (152 SMs), pass 1 with 2 / 8 / 32 sites per warp: 512 sites 0.18 / 0.52 /
+// 1.84 ms, 10,296 1.35 / 1.38 / 1.84, 64,000 7.9 / 6.4 / 6.5, 262,144 31.9 /
+// 24.5 / 22.5 ms; pass 2 with 1 / 4 / 8: 512 sites 0.48 / 1.47 / 2.8 ms,
+// 2,744 2.06 / 2.50 / 3.21, 10,296 6.9 / 6.3 / 7.3, 32,768 21.9 / 17.3 /
+// 17.1, 262,144 174 / 133 / 127 ms.  Results do not depend on it.
+int rho_sites_per_warp(int64_t n, int sms) { return n < 64 * (int64_t)sms ? 2 : n < 512 * (int64_t)sms ? 8 : 32; }
+int grad_sites_per_warp(int64_t n, int sms) { return n < 32 * (int64_t)sms ? 1 : n < 128 * (int64_t)sms ? 4 : 8; }
 
-// Block size of the thread-per-site FP64 kernels.  A site's thread runs a
-// long serial FP64 chain, and the warps of one SM share its narrow FP64
-// pipe: a small system finishes sooner when its warps are spread over as
-// many SMs as possible (one-warp blocks); a large one fills the device
-// either way.  Results do not depend on the block size.
-unsigned block64(int64_t n) { return n < (int64_t)current_device_sms() * kBlock * 4 ? 32u : (unsigned)kBlock; }
+// Blocks resident on the device at once for a kernel with its shared
+// memory, asked once per kernel and device under a lock.
+int resident_blocks(const void *fn, int smem, int dev) {
+  struct Entry {
+    const void *fn;
+    int dev, blocks;
+  };
+  static std::mutex m;
+  static std::vector<Entry> cache;
+  std::lock_guard<std::mutex> lock(m);
+  for (const Entry &e : cache)
+    if (e.fn == fn && e.dev == dev) return e.blocks;
+  int nb = 0;
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * kWarps, smem);
+  (void)cudaGetLastError();
+  if (nb < 1) return 1;  // not cached: asked again next time
+  cache.push_back({fn, dev, nb * device_sms(dev)});
+  return cache.back().blocks;
+}
+
+template <class Shared>
+a2c_status launch_warps(void (*fn)(SiteArgs), int sites, const SiteArgs &a, int64_t n, bool list, a2c_gpp_ctx *c) {
+  constexpr int smem = (int)sizeof(Shared) * kWarps;
+  const int cap = resident_blocks((const void *)fn, smem, c->device);
+  int64_t blocks = (n + (int64_t)sites * kWarps - 1) / ((int64_t)sites * kWarps);
+  if (list) blocks = std::min<int64_t>(blocks, cap);  // the list's length is only known on the device
+  fn<<<(unsigned)blocks, 32 * kWarps, smem, c->stream>>>(a);
+  A2C_CUDA(cudaGetLastError());
+  return A2C_OK;
+}
+
+template <bool LIST>
+a2c_status density64(a2c_gpp_ctx *c, const SiteArgs &a, int64_t n) {
+  switch (rho_sites_per_warp(n, device_sms(c->device))) {
+    case 2: return launch_warps<RhoShared>(k_density64<2, LIST>, 2, a, n, LIST, c);
+    case 8: return launch_warps<RhoShared>(k_density64<8, LIST>, 8, a, n, LIST, c);
+    default: return launch_warps<RhoShared>(k_density64<32, LIST>, 32, a, n, LIST, c);
+  }
+}
+template <bool LIST>
+a2c_status gradient64(a2c_gpp_ctx *c, const SiteArgs &a, int64_t n) {
+  switch (grad_sites_per_warp(n, device_sms(c->device))) {
+    case 1: return launch_warps<GradShared>(k_gradient64<1, LIST>, 1, a, n, LIST, c);
+    case 4: return launch_warps<GradShared>(k_gradient64<4, LIST>, 4, a, n, LIST, c);
+    default: return launch_warps<GradShared>(k_gradient64<8, LIST>, 8, a, n, LIST, c);
+  }
+}
+
+}  // namespace
 
 a2c_status launch_density64(a2c_gpp_ctx *c, const double *dX) {
   if (c->N == 0) return A2C_OK;
-  SiteArgs a = site_args(c, dX);
-  const unsigned bs = block64(c->N);
-  k_density64<<<grid_for(c->N, (int)bs), bs, 0, c->stream>>>(a);
-  A2C_CUDA(cudaGetLastError());
-  return A2C_OK;
+  return density64<false>(c, site_args(c, dX), c->N);
 }
 
 a2c_status launch_gradient64(a2c_gpp_ctx *c, const double *dX, double *dG) {
   if (c->N == 0) return A2C_OK;
   SiteArgs a = site_args(c, dX);
   a.G = dG;
-  const unsigned bs = block64(c->N);
-  k_gradient64<<<grid_for(c->N, (int)bs), bs, 0, c->stream>>>(a);
-  A2C_CUDA(cudaGetLastError());
-  return A2C_OK;
+  return gradient64<false>(c, a, c->N);
 }
 
-// One-warp blocks (see block64): the list length is only known on the
-// device, and a short list must still spread over all SMs.
 a2c_status launch_eval64_list(a2c_gpp_ctx *c, const double *dX, double *dG, const BatchView &bv) {
-  constexpr int kLB = 32;
-  // persistent grid sizes per device, computed once under a lock
-  static std::mutex m;
-  static int caps[kMaxDevices][2] = {};
-  int cap[2];
-  {
-    const int dev = (c->device >= 0 && c->device < kMaxDevices) ? c->device : 0;
-    std::lock_guard<std::mutex> lock(m);
-    if (!caps[dev][0]) {
-      const int sms = device_sms(c->device);
-      int b0 = 0, b1 = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_density64_list, kLB, 0);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_gradient64_list, kLB, 0);
-      (void)cudaGetLastError();
-      if (b0 > 0 && b1 > 0) {
-        caps[dev][0] = sms * b0;
-        caps[dev][1] = sms * b1;
-      }
-    }
-    cap[0] = std::max(1, caps[dev][0]);
-    cap[1] = std::max(1, caps[dev][1]);
-  }
   if (c->N == 0) return A2C_OK;
   SiteArgs a = site_args(c, dX);
   a.G = dG;
   a.bv = bv;
-  const int64_t need = (c->N + kLB - 1) / kLB;
-  k_density64_list<<<(unsigned)std::min<int64_t>(need, cap[0]), kLB, 0, c->stream>>>(a);
-  k_gradient64_list<<<(unsigned)std::min<int64_t>(need, cap[1]), kLB, 0, c->stream>>>(a);
-  A2C_CUDA(cudaGetLastError());
-  return A2C_OK;
+  A2C_TRY(density64<true>(c, a, c->N));
+  return gradient64<true>(c, a, c->N);
 }
 
 a2c_status launch_eam64(a2c_gpp_ctx *c, int which, const double *d_in, int64_t n, double *d_out) {
