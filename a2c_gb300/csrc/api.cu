@@ -319,7 +319,7 @@ a2c_status a2c_gpp_create(const a2c_gpp_params *p, a2c_gpp_ctx **out) {
   if (!s) s = dalloc(&c->d_hh1_off, (int64_t)p->nH + 1);
   for (int d = 0; d < 3; ++d) c->list_reach[d] = HUGE_VAL;  // no lists yet
   if (!s && (!p->periodic[0] || !p->periodic[1] || !p->periodic[2])) s = dalloc(&c->d_xlist, 4 * N);
-  if (!s && cudaMallocHost((void **)&c->h_small, 64) != cudaSuccess) s = A2C_ERR_NOMEM;
+  if (!s && cudaMallocHost((void **)&c->h_small, sizeof(double) * kHostSmall) != cudaSuccess) s = A2C_ERR_NOMEM;
   if (!s) {
     if (N > 0) {
       k_fill<<<grid_for(N, 256), 256, 0, c->stream>>>(c->d_occ, N, 0.0);
@@ -346,6 +346,7 @@ a2c_status a2c_gpp_destroy(a2c_gpp_ctx *c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   mixed_free(c);
   lbfgs_free(c);
+  lists_free(c);
   for (void *p : {(void *)c->d_X, (void *)c->d_G, (void *)c->d_occ, (void *)c->d_rho, (void *)c->d_Fp,
                   (void *)c->d_Vs, (void *)c->d_Ss, (void *)c->d_red, (void *)c->d_status, (void *)c->d_off,
                   (void *)c->d_nbr, (void *)c->d_npd, (void *)c->d_shell, (void *)c->d_hh1_off, (void *)c->d_hh1,
@@ -502,12 +503,12 @@ a2c_status a2c_gpp_build_neighbors(a2c_gpp_ctx *c, const double *X, int *max_nei
   DeviceGuard g(c->device);
   // finite, and periodic coordinates within [-L/2, 3L/2] (images are limited
   // to one box length either way): checked on the device
-  int moved = 0;
-  A2C_TRY(stage_positions(c, X, (uintptr_t)X % 8 == 0 ? (const double *)mapped(X) : nullptr, &moved));
+  PosScan scan;
+  A2C_TRY(stage_positions(c, X, (uintptr_t)X % 8 == 0 ? (const double *)mapped(X) : nullptr, &scan));
   c->has_state = true;
   c->has_neighbors = false;
   c->has_density = false;
-  A2C_TRY(build_neighbors_device(c, X));
+  A2C_TRY(build_neighbors_device(c, &scan));
   c->has_neighbors = true;
   A2C_TRY(mixed_lists_changed(c));
   if (max_neighbors) *max_neighbors = c->max_neighbors;
@@ -594,12 +595,12 @@ a2c_status a2c_gpp_update_neighbors(a2c_gpp_ctx *c, const double *X, int *max_ne
   DeviceGuard g(c->device);
   // checked on the device: pinned X is read there directly, other memory
   // is copied first
-  int moved = 0;
-  A2C_TRY(stage_positions(c, X, (uintptr_t)X % 8 == 0 ? (const double *)mapped(X) : nullptr, &moved));
+  PosScan scan;
+  A2C_TRY(stage_positions(c, X, (uintptr_t)X % 8 == 0 ? (const double *)mapped(X) : nullptr, &scan));
   c->has_state = true;
   c->has_neighbors = false;
   c->has_density = false;
-  A2C_TRY(update_neighbors_device(c, X, rebuilt, moved));
+  A2C_TRY(update_neighbors_device(c, &scan, rebuilt));
   c->has_neighbors = true;
   A2C_TRY(mixed_lists_changed(c));
   if (max_neighbors) *max_neighbors = c->max_neighbors;
@@ -1087,7 +1088,6 @@ a2c_status a2c_gpp_dmd_run(a2c_gpp_ctx *c, double *X, double *xH, double *gamma,
              cudaMemcpyAsync(dsurf, flags.data(), sizeof(int) * nH, cudaMemcpyHostToDevice, st)))
     s = A2C_ERR_CUDA;
   c->has_state = true;
-  std::vector<double> hX;
   // After an eager first step (one-time set-up, the engine), the remaining
   // steps can run as one CUDA graph (engine_dmd_graph).
   const bool graph = !dp->host_steps && nsteps >= 2 && !dp->neighbor_update &&
@@ -1098,15 +1098,7 @@ a2c_status a2c_gpp_dmd_run(a2c_gpp_ctx *c, double *X, double *xH, double *gamma,
     double f = 0.0, gn = 0.0;
     int it = 0, fev = 0, why = 0;
     if (k > 0 && dp->neighbor_update) {  // findNeighbors + findLocalNeighbors at the current positions
-      if (c->skin > 0.0) {
-        s = update_neighbors_device(c, nullptr, nullptr, -1);
-      } else {
-        hX.resize((size_t)(4 * c->N));
-        if (cudaMemcpyAsync(hX.data(), c->d_X, sizeof(double) * 4 * c->N, cudaMemcpyDeviceToHost, st) ||
-            cudaStreamSynchronize(st))
-          s = A2C_ERR_CUDA;
-        if (!s) s = build_neighbors_device(c, hX.data());
-      }
+      s = c->skin > 0.0 ? update_neighbors_device(c, nullptr, nullptr) : build_neighbors_device(c, nullptr);
       if (s) break;
     }
     s = lbfgs_minimize(c, c->d_X, &dp->lbfgs, &f, &it, &fev, &gn, &why);  // minimizer.cpp:548

@@ -68,6 +68,9 @@ enum : int { kStatusNonfinite = 1, kStatusOverflow = 2, kStatusTimeout = 4, kSta
 // less than half of it apart.
 constexpr double kFreeSpan = 64.0;
 
+// doubles of a context's pinned scratch, and where the list builds' reports start in it
+constexpr int kHostSmall = 32, kHostReport = 8;
+
 struct Mixed;   // mixed-precision buffers (k_mixed.cu)
 struct Lbfgs;   // L-BFGS buffers (lbfgs.cu)
 
@@ -112,9 +115,10 @@ struct a2c_gpp_ctx {
   a2c::Mixed *mixed;
   a2c::Lbfgs *lbfgs;
   void *snap;  // the snapshot in flight (api.cu)
+  void *list_work;  // scratch of the list builds (k_neighbors.cu), created on first use
   void *engine;     // the device-driven minimizer (batch.cu), created on first use
   int host_loop;    // L-BFGS driver, A2C_MINIMIZER_* (a2c_gpp_set_minimizer)
-  double *h_small;  // pinned: f and the status word of a host-pointer call
+  double *h_small;  // pinned (kHostSmall): f and the status word of a host-pointer call, list reports
   int last_mixed_iters, last_fp64_iters;
   double last_mixed_gnorm;
 };
@@ -186,16 +190,25 @@ a2c_status launch_macro_device(a2c_gpp_ctx *c, const double *d_x, const int *d_s
 a2c_status check_status_word(a2c_gpp_ctx *c);
 
 // k_neighbors.cu
-a2c_status build_neighbors_device(a2c_gpp_ctx *c, const double *h_X);
-// skin path (positions in c->d_X; h_X may be null): rebuild the extended
-// lists if needed, then re-filter at rc
-a2c_status update_neighbors_device(a2c_gpp_ctx *c, const double *h_X, int *rebuilt, int moved);
-// The skin path's new positions X (host memory; mX its device-visible view
-// when pinned, else null), checked on the device -- A2C_ERR_NONFINITE,
-// A2C_ERR_INVALID for a periodic coordinate outside [-L/2, 3L/2], d_X then
-// unchanged -- and moved into d_X; moved = 1 when a site moved more than
-// half the skin since the extended lists were built.
-a2c_status stage_positions(a2c_gpp_ctx *c, const double *X, const double *mX, int *moved);
+// What one pass over new positions finds: checks, extents, scale.
+constexpr int kPosMoved = 1, kPosNonfinite = 2, kPosOutside = 4;
+struct PosScan {
+  int flags;                        // kPos*
+  unsigned qmax_bits;               // largest |coordinate| as float bits, one ulp up
+  unsigned long long lo[3], hi[3];  // extents of the free directions, as ordered integers
+};
+// Positions in c->d_X; scan: what stage_positions found of them (null:
+// looked at here).  update: the skin path (rebuild the extended lists if
+// needed, then re-filter at rc).
+a2c_status build_neighbors_device(a2c_gpp_ctx *c, const PosScan *scan);
+a2c_status update_neighbors_device(a2c_gpp_ctx *c, const PosScan *scan, int *rebuilt);
+// New positions X (host memory; mX its device-visible view when pinned,
+// else null), checked on the device -- A2C_ERR_NONFINITE, A2C_ERR_INVALID
+// for a periodic coordinate outside [-L/2, 3L/2], d_X then unchanged -- and
+// moved into d_X; kPosMoved is set when a site moved more than half the skin
+// since the extended lists were built.
+a2c_status stage_positions(a2c_gpp_ctx *c, const double *X, const double *mX, PosScan *scan);
+void lists_free(a2c_gpp_ctx *c);
 
 // The span guard of the mixed form: per direction, how far a site may move
 // from the position the lists were built at before a listed pair could
