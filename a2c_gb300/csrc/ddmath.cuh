@@ -228,6 +228,53 @@ A2C_HD double from_words(int hi, int lo) {
 #endif
 }
 
+// a * b, correctly rounded, in integer operations: the 106-bit product of
+// the significands, normalized, rounded to nearest even by one chain of
+// carries that also adds the exponent and the sign.  Both factors and the
+// product must be normal (mul_int_ok).  About 28 instructions of the integer
+// pipes (four 32 x 32 + 64 multiply-adds among them), which a GB300
+// scheduler issues in the time its two-lane FP64 pipe needs for half an
+// instruction: a kernel bound by that pipe gains by moving multiplications
+// off it.
+A2C_HD double mul_int(double a, double b) {
+  const unsigned ah = (unsigned)hi_word(a), al = (unsigned)lo_word(a);
+  const unsigned bh = (unsigned)hi_word(b), bl = (unsigned)lo_word(b);
+  const unsigned ma = (ah & 0xfffffu) | 0x100000u;  // a's significand: 53 bits
+  const unsigned mb = (bh & 0xfffffu) | 0x100000u;
+  const unsigned nh = (mb << 11) | (bl >> 21), nl = bl << 11;  // b's, shifted to 64 bits
+  const unsigned long long p0 = (unsigned long long)al * nl;
+  const unsigned long long t = (unsigned long long)ma * nl + (p0 >> 32);
+  const unsigned long long u = (unsigned long long)al * nh + (unsigned)t;
+  const unsigned long long h = (unsigned long long)ma * nh + (t >> 32) + (u >> 32);  // 2^51 <= h < 2^53
+  const unsigned s = (unsigned)(h >> 32) < 0x100000u ? 1u : 0u;
+  const unsigned e = (ah & 0xfff00000u) + (bh & 0xfff00000u) - 0x3ff00000u - (s << 20);
+#if defined(__CUDA_ARCH__)
+  const unsigned hh = __funnelshift_l((unsigned)h, (unsigned)(h >> 32), s);
+  const unsigned hl = __funnelshift_l((unsigned)u, (unsigned)h, s);
+  const unsigned lh = __funnelshift_l((unsigned)p0, (unsigned)u, s);
+  const unsigned w = ((unsigned)p0 << s) | (hl & 1u);
+  unsigned rh, rl;
+  asm("{\n\t.reg .u32 c;\n\t"
+      "add.cc.u32 c, %2, 0xffffffff;\n\t"    // carry: bits below lh, or (a tie goes to even) an odd result
+      "addc.cc.u32 c, %3, 0x7fffffff;\n\t"   // carry: more than half, or half with the above
+      "addc.cc.u32 %0, %4, 0;\n\t"
+      "addc.u32 %1, %5, %6;\n\t}"
+      : "=r"(rl), "=r"(rh)
+      : "r"(w), "r"(lh), "r"(hl), "r"(hh), "r"(e));
+  return from_words((int)rh, (int)rl);
+#else
+  const unsigned long long lo = u << 32 | (unsigned)p0;
+  const unsigned long long hn = s ? h << 1 | lo >> 63 : h, ln = lo << s;
+  const unsigned long long up = ln > 0x8000000000000000ull || (ln == 0x8000000000000000ull && (hn & 1)) ? 1 : 0;
+  const unsigned long long r = hn + up + ((unsigned long long)e << 32);
+  return from_words((int)(r >> 32), (int)(unsigned)r);
+#endif
+}
+// |x| in [2^-511, 2^513): the product of two such values is normal
+A2C_HD bool mul_int_ok(double x) {
+  return (unsigned)((hi_word(x) & 0x7ff00000) - 0x20000000) < 0x40000000u;
+}
+
 // Adding 1.5 2^52 rounds |v| < 2^31 to an integer (ties to even), held in
 // the sum's low word.
 constexpr double kRoundShift = 6755399441055744.0;

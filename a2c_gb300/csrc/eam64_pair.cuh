@@ -12,7 +12,12 @@
 //     evaluations in place of five outside [2, 2.5) and [4, 5) A;
 //   * x / 5 by two operations and the other quotients by four, correctly
 //     rounded (div5, Divisor);
-//   * comparisons with the switch radii on the bits, by integer operations.
+//   * comparisons with the switch radii on the bits, by integer operations;
+//   * multiplications whose factors are known not to be zero on the integer
+//     pipes (ddmath.cuh mul_int).
+// Per point 221 FP64 instructions remain of about 330 (all pair types of a
+// bulk site, the additions included), at 83% of the pipe's two lanes, which
+// is what a chain of FMAs reaches: pass 2 at 262,144 sites 127 -> 106 ms.
 // The fast forms hold for kPairMin <= x < kPairMax (in_pair_range); callers
 // take eam64.cuh's functions elsewhere.
 #pragma once
@@ -45,7 +50,7 @@ A2C_EAM bool in_pair_range(double x) {
 // ulp from every midpoint of two doubles (x - 5 m is a multiple of 1/16 ulp
 // of x, and not zero, for a midpoint m), the sum below is within 2^-50 ulp
 // of it before its one rounding.
-A2C_EAM double div5(double x) { return fma(x, 0.2, x * -1.1102230246251565e-17); }
+A2C_EAM double div5(double x) { return fma(x, 0.2, dd::mul_int(x, -1.1102230246251565e-17)); }
 
 // Quotients by one divisor b, correctly rounded: z = 1/b rounded to
 // nearest, with its error zl a quotient q within one ulp, then Markstein's
@@ -77,55 +82,61 @@ A2C_EAM bool exact_for(double a) {
 // a / d.b for any a
 A2C_EAM double divide(double a, const Divisor &d) { return exact_for(a) ? quotient(a, d) : a / d.b; }
 
-// f_Pd as a function of r = x / 5 (potential.cpp:64-98)
+// f_Pd as a function of r = x / 5 (potential.cpp:64-98).  Multiplications
+// by mul_int where no factor can be zero: below the switch radius r <= 1,
+// the quadratics have no real root, and r meets 0.53 and 0.136 only.
 A2C_EAM double f_Pd_at(double r) {
-  const double x1 = r * 5.0;
+  using dd::mul_int;
+  const double x1 = mul_int(r, 5.0);
   if (above(x1, 5.0)) return 0.001510569378297 * dd::fexp(-0.077976566126292 / 0.001510569378297 * (x1 - 5.0));
-  double ra = r;
-  ra = ra * (r * (r - 2.7267629107325706) + 1.8716766113599643);
-  ra = ra * (r * (r - 2.50290548851635) + 1.668549182690922);
-  ra = ra * (r * (r - 2.0924467509943674) + 1.3150372774478005);
-  ra = ra * (r * (r - 1.564328475106985) + 0.8987511149780485);
-  ra = ra * (r * (r - 1.009780903403673) + 0.5124363774128722);
-  ra = ra * (r * (r - 0.5304054524800665) + 0.2169886022464641);
-  ra = ra * (r * (r - 0.1356566408715063) + 0.035852347523891395);
+  double ra = mul_int(r, mul_int(r - 2.7267629107325706, r) + 1.8716766113599643);
+  ra = mul_int(ra, mul_int(r - 2.50290548851635, r) + 1.668549182690922);
+  ra = mul_int(ra, mul_int(r - 2.0924467509943674, r) + 1.3150372774478005);
+  ra = mul_int(ra, mul_int(r - 1.564328475106985, r) + 0.8987511149780485);
+  ra = mul_int(ra, mul_int(r - 1.009780903403673, r) + 0.5124363774128722);
+  ra = mul_int(ra, r * (r - 0.5304054524800665) + 0.2169886022464641);
+  ra = mul_int(ra, r * (r - 0.1356566408715063) + 0.035852347523891395);
   return -0.02972698211669922 +
-         r * (0.6676807403564453 + r * (-255.8965835571289 + r * (14673.409149169922 + -2.597301181336601e7 * ra)));
+         r * (0.6676807403564453 +
+              r * (-255.8965835571289 + r * (14673.409149169922 + mul_int(ra, -2.597301181336601e7))));
 }
 // x1 / 5 for x1 = r * 5, r = x / 5: r itself where x's significand is 1.25
 // or more (see above)
 A2C_EAM double second_fifth(double x, double r) {
-  return (dd::hi_word(x) & 0xfffff) >= 0x40000 ? r : div5(r * 5.0);
+  return (dd::hi_word(x) & 0xfffff) >= 0x40000 ? r : div5(dd::mul_int(r, 5.0));
 }
-// phi_Pd with r = x / 5 and f = f_Pd(x1) (potential.cpp:126-155)
+// phi_Pd with r = x / 5 and f = f_Pd(x1) (potential.cpp:126-155).  Below
+// the switch radius r <= 1.01; the factor r - 0.424 can be zero, and then
+// so is the product from there on.
 A2C_EAM double phi_Pd_at(double r, double f) {
-  const double x1 = r * 5.0;
+  using dd::mul_int;
+  const double x1 = mul_int(r, 5.0);
   if (above(x1, 5.05)) return -0.016958780164980 * dd::fexp(0.089019679316328 / -0.016958780164980 * (x1 - 5.05));
-  double y = -79415.24035137112 * (r - 1.0699996145674568);
-  y = y * (r - 1.06015072612581);
+  double y = mul_int(r - 1.0699996145674568, -79415.24035137112);
+  y = mul_int(r - 1.06015072612581, y);
   y = y * (r - 0.42433991011376526);
-  y = y * (r + 0.06169160085238687);
-  y = y * (r * (r - 2.0586473420376348) + 1.0683922574015199);
-  y = y * (r * (r - 1.6696359816422877) + 0.7337878627470482);
-  y = y * (r * (r - 1.1690370066230809) + 0.3909805777737639);
-  y = y * (r * (r - 0.2635598721249787) + 0.033551116514910245);
+  if ((dd::hi_word(y) & 0x7fffffff) == 0) return 0.0 + (2 * 0.251546) * f;
+  y = mul_int(r + 0.06169160085238687, y);
+  y = mul_int(mul_int(r - 2.0586473420376348, r) + 1.0683922574015199, y);
+  y = mul_int(mul_int(r - 1.6696359816422877, r) + 0.7337878627470482, y);
+  y = mul_int(mul_int(r - 1.1690370066230809, r) + 0.3909805777737639, y);
+  y = mul_int(r * (r - 0.2635598721249787) + 0.033551116514910245, y);
   return y + (2 * 0.251546) * f;
 }
 A2C_EAM double f_Pd_pos(double x) { return f_Pd_at(div5(x)); }
 A2C_EAM double f_H_pos(double x) {
   if (above(x, 5.35)) return 0.009986990526578 * dd::fexp(-0.013075667086408 / 0.009986990526578 * (x - 5.35));
-  return 11.0025 * dd::fexp(-1.30927 * x);
+  return dd::mul_int(dd::fexp(dd::mul_int(x, -1.30927)), 11.0025);
 }
-A2C_EAM double phi_PdH_pos(double x) {
+// phi_PdH (potential.cpp:162-177) and phi_H (185-200): one form, constants
+// by pair type
+A2C_EAM double morse_pos(bool pdh, double x) {
   if (above(x, 5.35))
-    return -3.353001113951400e-04 * dd::fexp(7.147062196813336e-04 / -3.353001113951400e-04 * (x - 5.35));
-  const double D = 0.2494540, alpha = 4.82613, beta = 2.13158, r0 = 1.50964, t = x - r0;
-  return D * (beta * dd::fexp(-alpha * t) - alpha * dd::fexp(-beta * t));
-}
-A2C_EAM double phi_H_pos(double x) {
-  if (above(x, 5.35)) return -0.003702722457147 * dd::fexp(0.005465945471933 / -0.003702722457147 * (x - 5.35));
-  const double D = 0.0661496, alpha = 3.67263, beta = 1.47797, r0 = 2.51980, t = x - r0;
-  return D * (beta * dd::fexp(-alpha * t) - alpha * dd::fexp(-beta * t));
+    return pdh ? -3.353001113951400e-04 * dd::fexp(7.147062196813336e-04 / -3.353001113951400e-04 * (x - 5.35))
+               : -0.003702722457147 * dd::fexp(0.005465945471933 / -0.003702722457147 * (x - 5.35));
+  const double D = pdh ? 0.2494540 : 0.0661496, alpha = pdh ? 4.82613 : 3.67263, beta = pdh ? 2.13158 : 1.47797;
+  const double t = x - (pdh ? 1.50964 : 2.51980);
+  return D * (dd::mul_int(dd::fexp(-alpha * t), beta) - dd::mul_int(dd::fexp(-beta * t), alpha));
 }
 
 // What one quadrature point of a pair at distance s takes from the pair
@@ -147,26 +158,53 @@ A2C_EAM PairPoint pair_point(bool iPd, bool jPd, double s, double e, const Divis
     p.dphi = (iPd && jPd) ? phi_Pd_d(s, e) : (iPd || jPd) ? phi_PdH_d(s, e) : phi_H_d(s, e);
     return p;
   }
-  if (iPd && jPd) {
-    const double r = div5(s), rp = div5(xp), rm = div5(xm);
-    double fp = f_Pd_at(rp), fm = f_Pd_at(rm);
-    p.da = p.db = divide(fp - fm, h);
-    p.phi = phi_Pd_at(r, f_Pd_at(second_fifth(s, r)));
-    const double rp2 = second_fifth(xp, rp), rm2 = second_fifth(xm, rm);
-    if (rp2 != rp) fp = f_Pd_at(rp2);
-    if (rm2 != rm) fm = f_Pd_at(rm2);
-    p.dphi = divide(phi_Pd_at(rp, fp) - phi_Pd_at(rm, fm), h);
-  } else if (iPd || jPd) {
-    const double fP = divide(f_Pd_pos(xp) - f_Pd_pos(xm), h), fH = divide(f_H_pos(xp) - f_H_pos(xm), h);
-    p.da = jPd ? fP : fH;
-    p.db = iPd ? fP : fH;
-    p.phi = phi_PdH_pos(s);
-    p.dphi = divide(phi_PdH_pos(xp) - phi_PdH_pos(xm), h);
-  } else {
-    p.da = p.db = divide(f_H_pos(xp) - f_H_pos(xm), h);
-    p.phi = phi_H_pos(s);
-    p.dphi = divide(phi_H_pos(xp) - phi_H_pos(xm), h);
+  // s, then s + e and s - e in one rolled loop: with the functions written
+  // out for each the instruction caches did not hold the kernel (pass 2 at
+  // 262,144 sites 112 ms, rolled 106)
+  const bool pp = iPd && jPd, pdh = iPd != jPd;
+  double fP1 = 0.0, fH1 = 0.0, ph1 = 0.0, dP = 0.0, dH = 0.0;
+  p.phi = p.dphi = 0.0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+  for (int v = 0; v < 3; ++v) {
+    const double x = v == 0 ? s : v == 1 ? xp : xm;
+    double fP = 0.0, fH = 0.0, ph;
+    if (pp) {  // f_Pd at r (not needed at s itself), and where it differs at phi_Pd's own fifth
+      const double r = div5(x), r2 = second_fifth(x, r);
+      double at = v == 0 ? r2 : r, f;
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+      for (bool first = true;; first = false) {
+        f = f_Pd_at(at);
+        if (first) fP = f;
+        if (at == r2) break;
+        at = r2;
+      }
+      ph = phi_Pd_at(r, f);
+    } else {
+      if (v > 0) {
+        if (pdh) fP = f_Pd_at(div5(x));
+        fH = f_H_pos(x);
+      }
+      ph = morse_pos(pdh, x);
+    }
+    if (v == 0) {
+      p.phi = ph;
+    } else if (v == 1) {
+      fP1 = fP;
+      fH1 = fH;
+      ph1 = ph;
+    } else {
+      dP = fP1 - fP;
+      dH = fH1 - fH;
+      p.dphi = divide(ph1 - ph, h);
+    }
   }
+  const double fP = (iPd || jPd) ? divide(dP, h) : 0.0, fH = pp ? 0.0 : divide(dH, h);
+  p.da = jPd ? fP : fH;
+  p.db = iPd ? fP : fH;
   return p;
 }
 // the density a neighbor at distance s adds at one point

@@ -16,8 +16,8 @@
 // a 512-site system 16 warps, each with 960 points in a row.  S trades the
 // two ends (rho_sites_per_warp, grad_sites_per_warp).  With the pair
 // functions' fewer operations (eam64_pair.cuh) an evaluation takes, one
-// thread per site -> now: 15.3 -> 0.69 ms at 512 sites, 23.0 -> 8.7 ms at
-// 10,296, 210.6 -> 149.7 ms at 262,144.
+// thread per site -> now: 15.3 -> 0.69 ms at 512 sites, 23.0 -> 7.3 ms at
+// 10,296, 210.6 -> 124.2 ms at 262,144.
 //
 // Geometry: for quadrature point k = 2m (+sqrt(3)) or 2m+1 (-sqrt(3)) only
 // coordinate m of R^6 is non-zero, so r_k differs from the pair's base
@@ -101,10 +101,15 @@ constexpr double kSqrt2 = 1.4142135623730951, kSqrt3 = 1.7320508075688772;
 // in the reference's operation order.
 __device__ __forceinline__ double displacement(double sigma) { return (kSqrt2 * sigma) * kSqrt3; }
 
+// a * b by the integer pipes where both are in their range
+__device__ __forceinline__ double mul(double a, double b) {
+  return dd::mul_int_ok(a) && dd::mul_int_ok(b) ? dd::mul_int(a, b) : a * b;
+}
+
 // |r_k| of quadrature point k (quadrature.cpp:111-132 ordering): component m
 // of the pair vector replaced by rm.
 __device__ __forceinline__ double radius(int m, double rm, double d20, double d21, double d22) {
-  const double q = rm * rm;
+  const double q = mul(rm, rm);
   return sqrt((m == 0 ? q : d20) + (m == 1 ? q : d21) + (m == 2 ? q : d22));
 }
 
@@ -350,7 +355,8 @@ __global__ void __launch_bounds__(32 * kWarps) k_gradient64(SiteArgs a) {
           const double rm = k < 6 ? sh.qp[q / NB][2 * m + sgn] - sh.qj[m][q] : sh.D[m][q] - (sgn ? -u : u);
           const double s = radius(m, rm, sh.D2[0][q], sh.D2[1][q], sh.D2[2][q]);
           const eam64::PairPoint f = eam64::pair_point(pdmask >> q & 1u, jPd, s, eps, h);
-          double c[3] = {sh.A1[q] * f.da, sh.A2[q] * f.db, sh.A3[q] * f.dphi};
+          const double av = sh.AV[q], A[3] = {sh.A1[q], sh.A2[q], sh.A3[q]};
+          double c[3] = {mul(A[0], f.da), mul(A[1], f.db), mul(A[2], f.dphi)};
           if (eam64::in_pair_range(s)) {
             const eam64::Divisor ds = eam64::divisor(s);
 #pragma unroll
@@ -359,18 +365,32 @@ __global__ void __launch_bounds__(32 * kWarps) k_gradient64(SiteArgs a) {
 #pragma unroll
             for (int i = 0; i < 3; ++i) c[i] = c[i] / s;
           }
-          const double rx = m == 0 ? rm : sh.D[0][q], ry = m == 1 ? rm : sh.D[1][q], rz = m == 2 ? rm : sh.D[2][q];
+          const double r[3] = {m == 0 ? rm : sh.D[0][q], m == 1 ? rm : sh.D[1][q], m == 2 ? rm : sh.D[2][q]};
           const double xi0 = sgn ? -kSqrt3 : kSqrt3;
+          const bool fits = dd::mul_int_ok(c[0]) && dd::mul_int_ok(c[1]) && dd::mul_int_ok(c[2]) &&
+                            dd::mul_int_ok(r[0]) && dd::mul_int_ok(r[1]) && dd::mul_int_ok(r[2]);
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             double *o = sh.pt + 4 * i * kGradRow + p;
-            const double x = c[i] * rx, y = c[i] * ry, z = c[i] * rz;
+            double x, y, z;
+            if (fits) {
+              x = dd::mul_int(c[i], r[0]);
+              y = dd::mul_int(c[i], r[1]);
+              z = dd::mul_int(c[i], r[2]);
+            } else {
+              x = c[i] * r[0];
+              y = c[i] * r[1];
+              z = c[i] * r[2];
+            }
             o[0] = x;
             o[kGradRow] = y;
             o[2 * kGradRow] = z;
-            if (k < 6) o[3 * kGradRow] = (m == 0 ? x : m == 1 ? y : z) * xi0;
+            if (k < 6) {
+              const double v = m == 0 ? x : m == 1 ? y : z;
+              o[3 * kGradRow] = fits ? dd::mul_int(v, xi0) : v * xi0;
+            }
           }
-          sh.pt[(4 * (k % 3) + 3) * kGradRow + 12 * q + 6 + k / 3] = sh.AV[q] * f.phi;
+          sh.pt[(4 * (k % 3) + 3) * kGradRow + 12 * q + 6 + k / 3] = mul(av, f.phi);
         }
         __syncwarp();
         if (adds) {
@@ -458,7 +478,7 @@ __global__ void __launch_bounds__(kBlock) k_chem64(SiteArgs a, const double coeP
       const double sk = point(g, k, r, comp, xi0);
       const bool fast = eam64::in_pair_range(sk);
       sum = sum + WF * (fast ? eam64::f_H_pos(sk) : eam64::f_H(sk));
-      sum = sum + W * (fast ? eam64::phi_PdH_pos(sk) : eam64::phi_PdH(sk));
+      sum = sum + W * (fast ? eam64::morse_pos(true, sk) : eam64::phi_PdH(sk));
     }
     const int64_t bj = a.off[j], mj = bj + a.npd[j], ej = a.off[j + 1];
     sum = sum + ((T * coePd0) * coePd2) * (double)(mj - bj);
@@ -482,7 +502,7 @@ __global__ void __launch_bounds__(kBlock) k_chem64(SiteArgs a, const double coeP
       const double sk = point(g, k, r, comp, xi0);
       const bool fast = eam64::in_pair_range(sk);
       sum = sum + xWF * (fast ? eam64::f_H_pos(sk) : eam64::f_H(sk));
-      sum = sum + xW * (fast ? eam64::phi_H_pos(sk) : eam64::phi_H(sk));
+      sum = sum + xW * (fast ? eam64::morse_pos(false, sk) : eam64::phi_H(sk));
     }
     const int64_t bj = a.off[j], mj = bj + a.npd[j], ej = a.off[j + 1];
     sum = sum + (((xj * T) * coeH0) * coeH2) * (double)(mj - bj);
@@ -541,11 +561,12 @@ SiteArgs site_args(a2c_gpp_ctx *c, const double *dX) {
 // Sites per warp.  Few sites: a warp per site or two, all lanes on its
 // points, though one to eight lanes then do its additions; many: the
 // additions of 8 (32 in pass 1) sites fill the lanes.  Measured on a GB300
-// (152 SMs), pass 1 with 2 / 8 / 32 sites per warp: 512 sites 0.18 / 0.52 /
-// 1.84 ms, 10,296 1.35 / 1.38 / 1.84, 64,000 7.9 / 6.4 / 6.5, 262,144 31.9 /
-// 24.5 / 22.5 ms; pass 2 with 1 / 4 / 8: 512 sites 0.48 / 1.47 / 2.8 ms,
-// 2,744 2.06 / 2.50 / 3.21, 10,296 6.9 / 6.3 / 7.3, 32,768 21.9 / 17.3 /
-// 17.1, 262,144 174 / 133 / 127 ms.  Results do not depend on it.
+// (152 SMs) before multiplications moved to the integer pipes, pass 1 with 2
+// / 8 / 32 sites per warp: 512 sites 0.18 / 0.52 / 1.84 ms, 10,296 1.35 /
+// 1.38 / 1.84, 64,000 7.9 / 6.4 / 6.5, 262,144 31.9 / 24.5 / 22.5 ms; pass 2
+// with 1 / 4 / 8: 512 sites 0.48 / 1.47 / 2.8 ms, 2,744 2.06 / 2.50 / 3.21,
+// 10,296 6.9 / 6.3 / 7.3, 32,768 21.9 / 17.3 / 17.1, 262,144 174 / 133 / 127
+// ms.  Results do not depend on it.
 int rho_sites_per_warp(int64_t n, int sms) { return n < 64 * (int64_t)sms ? 2 : n < 512 * (int64_t)sms ? 8 : 32; }
 int grad_sites_per_warp(int64_t n, int sms) { return n < 32 * (int64_t)sms ? 1 : n < 128 * (int64_t)sms ? 4 : 8; }
 

@@ -1,10 +1,12 @@
 // Compares, bit for bit on the host, the fast FP64 forms of the device code
 // with the plain ones they stand for: ddmath.cuh's quick exp, log and pow
 // (where their rounding test settles the result) and fexp_mid, and
+// mul_int, and
 // eam64_pair.cuh's pair functions and quotients.  argv: form, count, seed.
 // Prints "<compared> <settled> <different>".
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <random>
 #include <string>
 
@@ -46,6 +48,17 @@ int main(int argc, char **argv) {
     } else if (form == "fexp") {
       const double x = i % 2 ? (U(g) - 0.5) * 1415.9 : (U(g) - 0.5) * std::ldexp(80.0, -(int)(g() % 70));
       tally(true, dd::fexp_mid(x), dd::fexp(x));
+    } else if (form == "mul") {  // both significands random, short, or all ones at the end
+      auto value = [&](long k) {
+        unsigned long long b = (g() >> 12) | (0x3ffull - 500 + g() % 1000) << 52 | g() << 63;
+        if (k % 4 == 1) b = b >> 26 << 26;
+        if (k % 4 == 2) b |= 0xfffffffffff00ull;
+        double x;
+        std::memcpy(&x, &b, sizeof(x));
+        return x;
+      };
+      const double a = value(i), b = value(i / 4);
+      tally(dd::mul_int_ok(a) && dd::mul_int_ok(b), dd::mul_int(a, b), a * b);
     } else if (form == "quotient") {
       const double b = std::ldexp(1.0 + U(g), (int)(g() % 8) - 4);
       double a = (U(g) - 0.5) * std::ldexp(1.0, (int)(g() % 900) - 450);

@@ -1,7 +1,7 @@
 """The fast FP64 forms of the device code against the plain ones, bit for
 bit, on the host (the headers compile as plain C++): the quick exp, log and
-pow of ddmath.cuh wherever Ziv's rounding test settles them, fexp_mid, the
-quotients and the pair functions of eam64_pair.cuh -- over their whole
+pow of ddmath.cuh wherever Ziv's rounding test settles them, fexp_mid, mul_int,
+the quotients and the pair functions of eam64_pair.cuh -- over their whole
 ranges and at the switch radii, a central-difference step to either side."""
 import subprocess
 from pathlib import Path
@@ -25,6 +25,7 @@ def check(tmp_path_factory):
 # take the series): all but 2^-10 in the mean, less for logarithms near 1
 @pytest.mark.parametrize("form,count,share", [("exp", 300_000, 0.999), ("log", 300_000, 0.8),
                                               ("pow", 200_000, 0.999), ("fexp", 1_000_000, 1.0),
+                                              ("mul", 2_000_000, 1.0),
                                               ("quotient", 1_000_000, 1.0), ("pair", 200_000, 1.0)])
 def test_fast_form_has_the_plain_bits(check, form, count, share):
     r = subprocess.run([str(check), form, str(count), "11"], capture_output=True, text=True, timeout=300)
