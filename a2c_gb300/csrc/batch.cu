@@ -33,6 +33,7 @@
 #include <new>
 #include <vector>
 
+#include "ddmath.cuh"
 #include "internal.cuh"
 
 namespace a2c {
@@ -49,7 +50,7 @@ enum : int { kPhaseMixed = 0, kPhaseFp64 = 1 };
 struct Inst {
   double f, fn, alpha, amax, gnorm, coef, gam_num, gam_den, f_noise, stall_rtol, mixed_gnorm;
   int state, phase, npairs, head, it, fev, ls, why, copy, steep, nhist, it0, mixed_iters, fp64_iters;
-  int fresh;  // a new direction awaits its first trial step length
+  unsigned arrived;  // reduction chunks of the running kernel that are done (see chunk_done)
 };
 
 struct Chunk {
@@ -61,6 +62,7 @@ struct Chunk {
 // Constants of one minimization.
 struct Cfg {
   int B, m, ring, max_it, max_fev, max_ls, polish, W;
+  int mixed;  // the minimization starts in the mixed form
   int64_t nec, nsc, n;  // element chunks, site chunks, vector length
   double gatol, c1, init_step, lb, max_step;
   double fn_mixed, fn_fp64, st_mixed, st_fp64;
@@ -88,44 +90,113 @@ __device__ __forceinline__ double wsum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ __forceinline__ double wmax(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 // block of kBlk threads: the warp tree, then warp 0 over the 8 warp sums
-template <bool MAX>
-__device__ __forceinline__ double bred(double v, double *sh) {
-  v = MAX ? wmax(v) : wsum(v);
+__device__ __forceinline__ double bsum(double v, double *sh) {
+  v = wsum(v);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (lane == 0) sh[w] = v;
   __syncthreads();
   v = (threadIdx.x < (blockDim.x >> 5)) ? sh[threadIdx.x] : 0.0;
-  if (w == 0) v = MAX ? wmax(v) : wsum(v);
+  if (w == 0) v = wsum(v);
   __syncthreads();
   return v;
 }
 
-__device__ __forceinline__ bool on_bound(int64_t t, const double *x, const double *g, double lb) {
-  return (t & 3) == 3 && x[t] <= lb && g[t] > 0.0;
+// The vector kernels are bound by the FP64 pipe (two lanes per SM and
+// clock: 1 M elements cost 1.7 us per operation), so what need not run on it
+// does not: products by the integer pipes (ddmath.cuh mul_int, the same
+// bits), magnitudes compared as integers, the width's bound tested on the
+// bits first.
+__device__ __forceinline__ double mul(double a, double b) {
+  return dd::mul_int_ok(a) && dd::mul_int_ok(b) ? dd::mul_int(a, b) : a * b;
+}
+// Magnitudes as integers: the same order as long as none is a NaN (then the
+// sums beside them are NaN, and decide).
+using Mag = unsigned long long;
+__device__ __forceinline__ Mag mag(double v) { return (Mag)__double_as_longlong(v) & 0x7fffffffffffffffull; }
+__device__ __forceinline__ double mag_value(Mag m) { return __longlong_as_double((long long)m); }
+__device__ __forceinline__ Mag wmax(Mag v) {
+  const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 32));
+  const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(v >> 32) == hi ? (unsigned)v : 0u);
+  return (Mag)hi << 32 | lo;
+}
+__device__ __forceinline__ Mag bmax(Mag v, double *sh) {
+  v = wmax(v);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (lane == 0) sh[w] = mag_value(v);
+  __syncthreads();
+  v = (threadIdx.x < (blockDim.x >> 5)) ? mag(sh[threadIdx.x]) : 0ull;
+  if (w == 0) v = wmax(v);
+  __syncthreads();
+  return v;
+}
+// v < lb, v <= lb for a positive lb; the FP64 comparison only where the bits
+// leave it open (a NaN)
+__device__ __forceinline__ bool below(double v, double lb) {
+  return __double_as_longlong(v) < __double_as_longlong(lb) && v < lb;
+}
+__device__ __forceinline__ bool at_or_below(double v, double lb) {
+  return __double_as_longlong(v) <= __double_as_longlong(lb) && v <= lb;
 }
 
 // sum over the instance's chunk partials part[c], c in [c0, c1), in order
+// (read past the L1: other blocks of the same kernel wrote them)
 __device__ __forceinline__ double chunk_total(const double *part, int c0, int c1, double *sh) {
   double s = 0.0;
-  for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) s += part[i];
-  return bred<false>(s, sh);
+  for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) s += __ldcg(&part[i]);
+  return bsum(s, sh);
 }
 __device__ __forceinline__ double chunk_max(const double *part, int c0, int c1, double *sh) {
-  double s = 0.0;
-  for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) s = fmax(s, part[i]);
-  return bred<true>(s, sh);
+  Mag s = 0;
+  for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) s = max(s, mag(__ldcg(&part[i])));
+  return mag_value(bmax(s, sh));
+}
+
+// Called by the whole block after a chunk of instance I is done and its
+// partials are written (by thread 0): true in the block that finishes the
+// last of the instance's `chunks`.  That block goes on to the instance's
+// totals, which spares a launch of one block per instance after every chunk
+// kernel -- no block waits for another.  The chunks of an instance are all
+// or none of them worked on by a kernel, so the count ends at `chunks`; it
+// is reset here.
+__device__ __forceinline__ bool chunk_done(Inst &I, int chunks, int *sh_last) {
+  if (threadIdx.x == 0) {
+    __threadfence();
+    const unsigned n = atomicAdd(&I.arrived, 1u) + 1u;
+    *sh_last = n == (unsigned)chunks;
+    if (n == (unsigned)chunks) I.arrived = 0u;
+  }
+  __syncthreads();
+  const bool last = *sh_last != 0;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// A chunk's kPer terms per thread, loaded together before they are used
+// (the loads of one term after the other left the vector kernels at the
+// latency of eight round trips); zeros past the chunk's end, which change
+// no sum.
+constexpr int kPer = kChunk / kBlk;
+__device__ __forceinline__ void load_chunk(const double *p, const Chunk &ch, double v[kPer]) {
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    const int i = threadIdx.x + e * kBlk;
+    v[e] = i < ch.len ? p[ch.start + i] : 0.0;
+  }
+}
+__device__ __forceinline__ void store_chunk(double *p, const Chunk &ch, const double v[kPer]) {
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    const int i = threadIdx.x + e * kBlk;
+    if (i < ch.len) p[ch.start + i] = v[e];
+  }
 }
 
 __device__ __forceinline__ int slot(int head, int k, int ring) { return ((head - 1 - k) % ring + ring) % ring; }
 
 // End of a phase: hand over to the FP64 polish, or retire.
-__device__ void end_phase(Inst &I, const Cfg &cf, int why) {
+__device__ void end_phase(Inst &I, const Cfg &cf, int why, int *cnt) {
   if (I.phase == kPhaseMixed) {
     I.mixed_iters = I.it;
     I.mixed_gnorm = I.gnorm;
@@ -143,6 +214,7 @@ __device__ void end_phase(Inst &I, const Cfg &cf, int why) {
     I.stall_rtol = cf.st_fp64;
   } else {
     I.state = kDone;
+    atomicSub(&cnt[kCntLeft], 1);
   }
 }
 
@@ -157,6 +229,7 @@ __global__ void k_init_state(Dev D, Cfg cf, int phase0) {
   I.f_noise = phase0 == kPhaseMixed ? cf.fn_mixed : cf.fn_fp64;
   I.stall_rtol = phase0 == kPhaseMixed ? cf.st_mixed : cf.st_fp64;
   D.st[b] = I;
+  if (b == 0) D.cnt[kCntLeft] = cf.B;
 }
 
 __global__ void k_project_all(double *x, int64_t n, double lb) {
@@ -171,8 +244,6 @@ __global__ void k_project_all(double *x, int64_t n, double lb) {
 constexpr int kPlanThreads = 1024;
 __global__ void __launch_bounds__(kPlanThreads) k_plan(Dev D, int B, int *listed, int *loff) {
   __shared__ int sh[7][kPlanThreads];
-  __shared__ int changed;
-  if (threadIdx.x == 0) changed = 0;
   const int per = (B + kPlanThreads - 1) / kPlanThreads;
   const int b0 = min(B, (int)threadIdx.x * per), b1 = min(B, b0 + per);
   int q[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -190,8 +261,10 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(Dev D, int B, int *listed
       q[6] += 1;
     }
   }
-  __syncthreads();
-  if (ch) atomicOr(&changed, 1);
+  if (!__syncthreads_or(ch)) {  // the lists and their lengths stand
+    if (threadIdx.x == 0) D.cnt[kCntChanged] = 0;
+    return;
+  }
   for (int k = 0; k < 7; ++k) sh[k][threadIdx.x] = q[k];
   __syncthreads();
   // inclusive Hillis-Steele scan of the per-thread sums
@@ -205,25 +278,23 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(Dev D, int B, int *listed
   int run[7];
   for (int k = 0; k < 7; ++k) run[k] = sh[k][threadIdx.x] - q[k];
   const int totPdM = sh[0][kPlanThreads - 1], totPdF = sh[2][kPlanThreads - 1];
-  if (changed) {
-    for (int b = b0; b < b1; ++b) {
-      const Inst &I = D.st[b];
-      const int code = I.state == kDone ? -1 : I.phase;
-      const InstGeo &g = D.geo[b];
-      int *o = loff + 6 * b;
-      o[0] = code == 0 ? run[0] : (code == 1 ? run[2] : -1);               // Pd sites
-      o[1] = code == 0 ? totPdM + run[1] : (code == 1 ? totPdF + run[3] : -1);  // H sites
-      o[2] = code >= 0 ? run[4] : -1;
-      o[3] = code >= 0 ? run[5] : -1;
-      o[4] = code;
-      if (code == 0) { run[0] += g.nPd; run[1] += g.nH; }
-      if (code == 1) { run[2] += g.nPd; run[3] += g.nH; }
-      if (code >= 0) {
-        run[4] += D.ecb[b + 1] - D.ecb[b];
-        run[5] += D.scb[b + 1] - D.scb[b];
-      }
-      listed[b] = code;
+  for (int b = b0; b < b1; ++b) {
+    const Inst &I = D.st[b];
+    const int code = I.state == kDone ? -1 : I.phase;
+    const InstGeo &g = D.geo[b];
+    int *o = loff + 6 * b;
+    o[0] = code == 0 ? run[0] : (code == 1 ? run[2] : -1);               // Pd sites
+    o[1] = code == 0 ? totPdM + run[1] : (code == 1 ? totPdF + run[3] : -1);  // H sites
+    o[2] = code >= 0 ? run[4] : -1;
+    o[3] = code >= 0 ? run[5] : -1;
+    o[4] = code;
+    if (code == 0) { run[0] += g.nPd; run[1] += g.nH; }
+    if (code == 1) { run[2] += g.nPd; run[3] += g.nH; }
+    if (code >= 0) {
+      run[4] += D.ecb[b + 1] - D.ecb[b];
+      run[5] += D.scb[b + 1] - D.scb[b];
     }
+    listed[b] = code;
   }
   if (threadIdx.x == kPlanThreads - 1) {
     D.cnt[kCntMixed] = sh[0][threadIdx.x] + sh[1][threadIdx.x];
@@ -231,7 +302,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_plan(Dev D, int B, int *listed
     D.cnt[kCntEch] = sh[4][threadIdx.x];
     D.cnt[kCntSch] = sh[5][threadIdx.x];
     D.cnt[kCntLive] = sh[6][threadIdx.x];
-    D.cnt[kCntChanged] = changed;
+    D.cnt[kCntChanged] = 1;
   }
 }
 
@@ -254,315 +325,248 @@ __global__ void k_fill(Dev D, int B, const int *loff, int *lm, int *lf, int *le,
   for (int i = threadIdx.x; i < ns; i += blockDim.x) ls[o[3] + i] = s0 + i;
 }
 
-__global__ void k_count_left(Dev D, int B) {
-  __shared__ double sh[kBlk / 32];
-  double v = 0.0;
-  for (int b = threadIdx.x; b < B; b += blockDim.x) v += D.st[b].state != kDone ? 1.0 : 0.0;
-  v = bred<false>(v, sh);
-  if (threadIdx.x == 0) D.cnt[kCntLeft] = (int)v;
-}
-
 // ------------------------------------------------------------ direction
 // Element-chunk kernels walk the live element chunks; a whole block takes
-// one chunk, so the per-instance tests below are block-uniform.
+// one chunk, so the per-instance tests below are block-uniform.  The block
+// that finishes an instance's last chunk (chunk_done) forms its totals and
+// takes the scalar step that follows.
 #define A2C_ECHUNKS(D)                                                     \
   for (int kk = blockIdx.x; kk < (D).cnt[kCntEch]; kk += gridDim.x) {       \
     const int c = (D).le[kk];                                             \
     const Chunk ch = (D).ech[c];                                          \
-    Inst &I = (D).st[ch.inst];
+    const int b = ch.inst;                                                \
+    Inst &I = (D).st[b];
 #define A2C_ECHUNKS_END }
 
-// pg = projected gradient; partials of |pg|^2 and max |pg|
+// pg = projected gradient, with |pg|^2 and max |pg|; the stopping tests
+// (TAO's gatol test and the caps); and, where there are pairs, the first
+// step of the two-loop recursion's first loop: q = pg, S_0 . q.
 __global__ void __launch_bounds__(kBlk) k_projgrad(Dev D, Cfg cf) {
   __shared__ double sh[kBlk / 32];
+  __shared__ int last;
   A2C_ECHUNKS(D)
   if (I.state != kNeedDir) continue;
-  double s = 0.0, mx = 0.0;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    const double v = on_bound(t, D.x, D.g, cf.lb) ? 0.0 : D.g[t];
-    D.pg[t] = v;
-    s += v * v;
-    mx = fmax(mx, fabs(v));
+  const bool pairs = I.npairs > 0;
+  const int sl = slot(I.head, 0, cf.ring);
+  double g[kPer], S[kPer];
+  load_chunk(D.g, ch, g);
+  if (pairs) load_chunk(D.S + (size_t)sl * cf.n, ch, S);
+  if ((threadIdx.x & 3) == 3) {  // a width (chunks start at a multiple of 4): zero where it rests on its bound
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const int i = threadIdx.x + e * kBlk;
+      if (i < ch.len && at_or_below(D.x[ch.start + i], cf.lb) && g[e] > 0.0) g[e] = 0.0;
+    }
   }
-  s = bred<false>(s, sh);
-  mx = bred<true>(mx, sh);
+  store_chunk(D.pg, ch, g);
+  if (pairs) store_chunk(D.d, ch, g);
+  double s = 0.0, q = 0.0;
+  Mag top = 0;
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    s += mul(g[e], g[e]);
+    top = max(top, mag(g[e]));
+    if (pairs) q += mul(S[e], g[e]);
+  }
+  s = bsum(s, sh);
+  double mx = mag_value(bmax(top, sh));
+  if (pairs) q = bsum(q, sh);
   if (threadIdx.x == 0) {
     D.part[c] = s;
     D.part[cf.nec + c] = mx;
+    D.part[2 * cf.nec + c] = q;
+  }
+  if (!chunk_done(I, D.ecb[b + 1] - D.ecb[b], &last)) continue;
+  s = chunk_total(D.part, D.ecb[b], D.ecb[b + 1], sh);
+  mx = chunk_max(D.part + cf.nec, D.ecb[b], D.ecb[b + 1], sh);
+  if (pairs) q = chunk_total(D.part + 2 * cf.nec, D.ecb[b], D.ecb[b + 1], sh);
+  if (threadIdx.x == 0) {
+    I.copy = 0;
+    I.gnorm = sqrt(s);
+    I.amax = mx;
+    I.steep = 0;
+    if (!isfinite(I.f) || !isfinite(I.gnorm)) end_phase(I, cf, A2C_DIVERGED_NAN, D.cnt);
+    else if (I.gnorm <= cf.gatol) end_phase(I, cf, A2C_CONVERGED_GATOL, D.cnt);
+    else if (I.it >= cf.max_it) end_phase(I, cf, A2C_DIVERGED_MAXITS, D.cnt);
+    else if (I.fev >= cf.max_fev) end_phase(I, cf, A2C_DIVERGED_MAXFCN, D.cnt);
+    else I.steep = pairs ? 0 : 1;
+    if (pairs) D.alph[b * cf.ring + sl] = q * D.rho[b * cf.ring + sl];
   }
   A2C_ECHUNKS_END
 }
 
-// gnorm and the stopping tests (TAO's gatol test and the caps)
-__global__ void __launch_bounds__(kBlk) k_dir_begin(Dev D, Cfg cf) {
-  __shared__ double sh[kBlk / 32];
-  const int b = blockIdx.x;
-  Inst &I = D.st[b];
-  if (threadIdx.x == 0) I.copy = 0;
-  if (I.state != kNeedDir) return;
-  const double s = chunk_total(D.part, D.ecb[b], D.ecb[b + 1], sh);
-  const double mx = chunk_max(D.part + cf.nec, D.ecb[b], D.ecb[b + 1], sh);
-  if (threadIdx.x != 0) return;
-  I.gnorm = sqrt(s);
-  I.amax = mx;
-  I.steep = 0;
-  if (!isfinite(I.f) || !isfinite(I.gnorm)) end_phase(I, cf, A2C_DIVERGED_NAN);
-  else if (I.gnorm <= cf.gatol) end_phase(I, cf, A2C_CONVERGED_GATOL);
-  else if (I.it >= cf.max_it) end_phase(I, cf, A2C_DIVERGED_MAXITS);
-  else if (I.fev >= cf.max_fev) end_phase(I, cf, A2C_DIVERGED_MAXFCN);
-  else I.steep = I.npairs == 0 ? 1 : 0;
-}
-
-// Two-loop recursion, first loop, step j (newest pair first): apply the
-// update of step j-1, then the partial dot S_j . q.
+// Two-loop recursion, first loop, step j >= 1 (newest pair first): apply
+// the update of step j-1, then the dot S_j . q.
 __global__ void __launch_bounds__(kBlk) k_loop1(Dev D, Cfg cf, int j) {
   __shared__ double sh[kBlk / 32];
-  A2C_ECHUNKS(D)
-  if (I.state != kNeedDir || I.steep) continue;
-  const int b = ch.inst, np = I.npairs;
-  const bool upd = j > 0 && j - 1 < np, dot = j < np;
-  if (j > 0 && !upd && !dot) continue;
-  const int slp = slot(I.head, j - 1, cf.ring), sl = slot(I.head, j, cf.ring);
-  const double a = upd ? D.alph[b * cf.ring + slp] : 0.0;
-  const double *Yp = D.Y + (size_t)slp * cf.n, *Sj = D.S + (size_t)sl * cf.n;
-  double s = 0.0;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    double q = j == 0 ? D.pg[t] : D.d[t];
-    if (upd) q -= a * Yp[t];
-    D.d[t] = q;
-    if (dot) s += Sj[t] * q;
-  }
-  s = bred<false>(s, sh);
-  if (threadIdx.x == 0) D.part[2 * cf.nec + c] = s;
-  A2C_ECHUNKS_END
-}
-
-__global__ void __launch_bounds__(kBlk) k_loop1_fin(Dev D, Cfg cf, int j) {
-  __shared__ double sh[kBlk / 32];
-  const int b = blockIdx.x;
-  Inst &I = D.st[b];
-  if (I.state != kNeedDir || I.steep || j >= I.npairs) return;
-  const double s = chunk_total(D.part + 2 * cf.nec, D.ecb[b], D.ecb[b + 1], sh);
-  if (threadIdx.x == 0) {
-    const int sl = slot(I.head, j, cf.ring);
-    D.alph[b * cf.ring + sl] = s * D.rho[b * cf.ring + sl];
-  }
-}
-
-// the pending update of the last first-loop step, then q *= s.y / y.y
-__global__ void __launch_bounds__(kBlk) k_scale(Dev D, Cfg cf) {
-  A2C_ECHUNKS(D)
-  if (I.state != kNeedDir || I.steep) continue;
-  const int b = ch.inst;
-  const bool upd = I.npairs == cf.m;
-  const int slp = slot(I.head, cf.m - 1, cf.ring);
-  const double a = upd ? D.alph[b * cf.ring + slp] : 0.0;
-  const double gam = I.gam_num / I.gam_den;
-  const double *Yp = D.Y + (size_t)slp * cf.n;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    double q = D.d[t];
-    if (upd) q -= a * Yp[t];
-    D.d[t] = q * gam;
-  }
-  A2C_ECHUNKS_END
-}
-
-// Second loop, step j (oldest pair first): apply the update of step j-1,
-// then the partial dot Y_j . q.
-__global__ void __launch_bounds__(kBlk) k_loop2(Dev D, Cfg cf, int j) {
-  __shared__ double sh[kBlk / 32];
+  __shared__ int last;
   A2C_ECHUNKS(D)
   if (I.state != kNeedDir || I.steep) continue;
   const int np = I.npairs;
-  const bool upd = j > 0 && j - 1 < np, dot = j < np;
-  if (!upd && !dot) continue;
-  const int slp = slot(I.head, np - j, cf.ring), sl = slot(I.head, np - 1 - j, cf.ring);
-  const double cp = I.coef;
-  const double *Sp = D.S + (size_t)slp * cf.n, *Yj = D.Y + (size_t)sl * cf.n;
+  if (j - 1 >= np) continue;
+  const bool dot = j < np;
+  const int slp = slot(I.head, j - 1, cf.ring), sl = slot(I.head, j, cf.ring);
+  const double a = D.alph[b * cf.ring + slp];
+  double q[kPer], Y[kPer], S[kPer];
+  load_chunk(D.d, ch, q);
+  load_chunk(D.Y + (size_t)slp * cf.n, ch, Y);
+  if (dot) load_chunk(D.S + (size_t)sl * cf.n, ch, S);
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) q[e] -= mul(a, Y[e]);
+  store_chunk(D.d, ch, q);
+  if (!dot) continue;
   double s = 0.0;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    double q = D.d[t];
-    if (upd) q += cp * Sp[t];
-    D.d[t] = q;
-    if (dot) s += Yj[t] * q;
-  }
-  s = bred<false>(s, sh);
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) s += mul(S[e], q[e]);
+  s = bsum(s, sh);
   if (threadIdx.x == 0) D.part[2 * cf.nec + c] = s;
+  if (!chunk_done(I, D.ecb[b + 1] - D.ecb[b], &last)) continue;
+  s = chunk_total(D.part + 2 * cf.nec, D.ecb[b], D.ecb[b + 1], sh);
+  if (threadIdx.x == 0) D.alph[b * cf.ring + sl] = s * D.rho[b * cf.ring + sl];
   A2C_ECHUNKS_END
 }
 
-__global__ void __launch_bounds__(kBlk) k_loop2_fin(Dev D, Cfg cf, int j) {
+// Second loop, step j (oldest pair first): apply the update of step j-1 --
+// at j = 0 the pending one of the first loop and the scaling by s.y / y.y
+// -- then the dot Y_j . q.
+__global__ void __launch_bounds__(kBlk) k_loop2(Dev D, Cfg cf, int j) {
   __shared__ double sh[kBlk / 32];
-  const int b = blockIdx.x;
-  Inst &I = D.st[b];
-  if (I.state != kNeedDir || I.steep || j >= I.npairs) return;
-  const double s = chunk_total(D.part + 2 * cf.nec, D.ecb[b], D.ecb[b + 1], sh);
-  if (threadIdx.x == 0) {
-    const int sl = slot(I.head, I.npairs - 1 - j, cf.ring);
-    I.coef = D.alph[b * cf.ring + sl] - D.rho[b * cf.ring + sl] * s;
+  __shared__ int last;
+  A2C_ECHUNKS(D)
+  if (I.state != kNeedDir || I.steep) continue;
+  const int np = I.npairs;
+  const bool upd = j > 0 ? j - 1 < np : np == cf.m, dot = j < np;
+  if (j > 0 && !upd) continue;
+  const int slp = j > 0 ? slot(I.head, np - j, cf.ring) : slot(I.head, cf.m - 1, cf.ring);
+  const int sl = slot(I.head, np - 1 - j, cf.ring);
+  double q[kPer], U[kPer], Y[kPer];
+  load_chunk(D.d, ch, q);
+  if (upd) load_chunk((j > 0 ? D.S : D.Y) + (size_t)slp * cf.n, ch, U);
+  if (dot) load_chunk(D.Y + (size_t)sl * cf.n, ch, Y);
+  if (j > 0) {
+    const double cp = I.coef;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) q[e] += mul(cp, U[e]);
+  } else {
+    const double a = upd ? D.alph[b * cf.ring + slp] : 0.0, gam = I.gam_num / I.gam_den;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      if (upd) q[e] -= mul(a, U[e]);
+      q[e] = mul(q[e], gam);
+    }
   }
+  store_chunk(D.d, ch, q);
+  if (!dot) continue;
+  double s = 0.0;
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) s += mul(Y[e], q[e]);
+  s = bsum(s, sh);
+  if (threadIdx.x == 0) D.part[2 * cf.nec + c] = s;
+  if (!chunk_done(I, D.ecb[b + 1] - D.ecb[b], &last)) continue;
+  s = chunk_total(D.part + 2 * cf.nec, D.ecb[b], D.ecb[b + 1], sh);
+  if (threadIdx.x == 0) I.coef = D.alph[b * cf.ring + sl] - D.rho[b * cf.ring + sl] * s;
+  A2C_ECHUNKS_END
 }
 
-// d = -q off the active set (or the scaled steepest descent); partial g.d
+// d = -q off the active set (or the scaled steepest descent), g.d and max
+// |d|; then the descent test -- not a descent direction: drop the memory
+// and fall back to steepest descent, which the trial kernel forms -- and the
+// first trial step length min(1, max_step / max|d|).
 __global__ void __launch_bounds__(kBlk) k_finish(Dev D, Cfg cf) {
   __shared__ double sh[kBlk / 32];
+  __shared__ int last;
   A2C_ECHUNKS(D)
   if (I.state != kNeedDir) continue;
   const bool steep = I.steep != 0;
   const bool upd = !steep && I.npairs == cf.m;
   const int slp = slot(I.head, 0, cf.ring);
   const double cp = I.coef, sc = -cf.init_step / I.amax;
-  const double *Sp = D.S + (size_t)slp * cf.n;
-  double s = 0.0, mx = 0.0;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    double v;
+  double g[kPer], v[kPer], S[kPer];
+  load_chunk(D.g, ch, g);
+  load_chunk(steep ? D.pg : D.d, ch, v);
+  if (upd) load_chunk(D.S + (size_t)slp * cf.n, ch, S);
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
     if (steep) {
-      v = D.pg[t] * sc;
+      v[e] = mul(v[e], sc);
     } else {
-      double q = D.d[t];
-      if (upd) q += cp * Sp[t];
-      v = on_bound(t, D.x, D.g, cf.lb) ? 0.0 : -q;
+      if (upd) v[e] += mul(cp, S[e]);
+      v[e] = -v[e];
     }
-    D.d[t] = v;
-    s += D.g[t] * v;
-    mx = fmax(mx, fabs(v));
   }
-  s = bred<false>(s, sh);
-  mx = bred<true>(mx, sh);
+  if (!steep && (threadIdx.x & 3) == 3) {
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      const int i = threadIdx.x + e * kBlk;
+      if (i < ch.len && at_or_below(D.x[ch.start + i], cf.lb) && g[e] > 0.0) v[e] = 0.0;
+    }
+  }
+  store_chunk(D.d, ch, v);
+  double s = 0.0;
+  Mag top = 0;
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    s += mul(g[e], v[e]);
+    top = max(top, mag(v[e]));
+  }
+  s = bsum(s, sh);
+  const double mx = mag_value(bmax(top, sh));
   if (threadIdx.x == 0) {
     D.part[3 * cf.nec + c] = s;
     D.part[cf.nec + c] = mx;  // the slot of max |pg|, read before this kernel
   }
-  A2C_ECHUNKS_END
-}
-
-// not a descent direction: drop the memory, fall back to steepest descent
-__global__ void __launch_bounds__(kBlk) k_dir_end(Dev D, Cfg cf) {
-  __shared__ double sh[kBlk / 32];
-  const int b = blockIdx.x;
-  Inst &I = D.st[b];
-  if (I.state != kNeedDir) return;
+  if (!chunk_done(I, D.ecb[b + 1] - D.ecb[b], &last)) continue;
   const double gd = chunk_total(D.part + 3 * cf.nec, D.ecb[b], D.ecb[b + 1], sh);
-  if (threadIdx.x != 0) return;
-  if (!(gd < 0.0)) {
-    I.npairs = 0;
-    I.head = 0;
-    I.steep = 2;
-  } else {
-    I.steep = 0;
+  double dmax = chunk_max(D.part + cf.nec, D.ecb[b], D.ecb[b + 1], sh);
+  if (threadIdx.x == 0) {
+    if (!(gd < 0.0)) {
+      I.npairs = 0;
+      I.head = 0;
+      I.steep = 2;
+      dmax = fabs(I.amax * sc);  // max |pg sc|: rounding keeps the order
+    } else {
+      I.steep = 0;
+    }
+    I.alpha = cf.max_step > 0.0 && dmax > cf.max_step ? cf.max_step / dmax : 1.0;
+    I.ls = 0;
+    I.state = kLineSearch;
   }
-  I.alpha = 1.0;
-  I.ls = 0;
-  I.fresh = 1;
-  I.state = kLineSearch;
-}
-
-__global__ void __launch_bounds__(kBlk) k_steep(Dev D, Cfg cf) {
-  __shared__ double sh[kBlk / 32];
-  A2C_ECHUNKS(D)
-  if (I.steep != 2) continue;
-  const double sc = -cf.init_step / I.amax;
-  double mx = 0.0;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    const double v = D.pg[t] * sc;
-    D.d[t] = v;
-    mx = fmax(mx, fabs(v));
-  }
-  mx = bred<true>(mx, sh);
-  if (threadIdx.x == 0) D.part[cf.nec + c] = mx;
   A2C_ECHUNKS_END
-}
-
-// first trial step length: min(1, max_step / max|d|)
-__global__ void __launch_bounds__(kBlk) k_alpha0(Dev D, Cfg cf) {
-  __shared__ double sh[kBlk / 32];
-  const int b = blockIdx.x;
-  Inst &I = D.st[b];
-  if (I.state != kLineSearch || !I.fresh) return;
-  const double dmax = chunk_max(D.part + cf.nec, D.ecb[b], D.ecb[b + 1], sh);
-  if (threadIdx.x != 0) return;
-  I.fresh = 0;
-  if (cf.max_step > 0.0 && dmax > cf.max_step) I.alpha = cf.max_step / dmax;
 }
 
 // ------------------------------------------------------------ trial / decide
-// xn = P(x + alpha d) (line search) or xn = x (first evaluation of a
-// phase); partial g.(xn - x)
+// xn = P(x + alpha d) (line search; after a failed descent test d = the
+// steepest descent first) or xn = x (first evaluation of a phase); partial
+// g.(xn - x)
 __global__ void __launch_bounds__(kBlk) k_trial(Dev D, Cfg cf) {
   __shared__ double sh[kBlk / 32];
   A2C_ECHUNKS(D)
   if (I.state != kLineSearch && I.state != kNeedEval) continue;
-  const bool ls = I.state == kLineSearch;
-  const double al = I.alpha;
+  (void)b;
+  const bool ls = I.state == kLineSearch, steep = I.steep == 2;
+  const double al = I.alpha, sc = -cf.init_step / I.amax;
+  double x[kPer], d[kPer], g[kPer];
+  load_chunk(D.x, ch, x);
   double s = 0.0;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    double v = D.x[t];
-    if (ls) {
-      v = D.x[t] + al * D.d[t];
-      if ((t & 3) == 3 && v < cf.lb) v = cf.lb;
-      s += D.g[t] * (v - D.x[t]);
+  if (ls) {
+    load_chunk(steep ? D.pg : D.d, ch, d);
+    load_chunk(D.g, ch, g);
+    if (steep) {
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) d[e] = mul(d[e], sc);
     }
-    D.xn[t] = v;
+#pragma unroll
+    for (int e = 0; e < kPer; ++e) {
+      double v = x[e] + mul(al, d[e]);
+      if ((threadIdx.x & 3) == 3 && below(v, cf.lb)) v = cf.lb;
+      s += mul(g[e], v - x[e]);
+      x[e] = v;
+    }
   }
-  s = bred<false>(s, sh);
+  store_chunk(D.xn, ch, x);
+  s = bsum(s, sh);
   if (threadIdx.x == 0) D.part[4 * cf.nec + c] = s;
   A2C_ECHUNKS_END
-}
-
-// candidate pair into the free ring slot; partials gn.s, s.y, y.y
-__global__ void __launch_bounds__(kBlk) k_post(Dev D, Cfg cf) {
-  __shared__ double sh[kBlk / 32];
-  A2C_ECHUNKS(D)
-  if (I.state != kLineSearch) continue;
-  double *Sh = D.S + (size_t)I.head * cf.n, *Yh = D.Y + (size_t)I.head * cf.n;
-  double dn = 0.0, sy = 0.0, yy = 0.0;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    const double s = D.xn[t] - D.x[t], y = D.gn[t] - D.g[t];
-    Sh[t] = s;
-    Yh[t] = y;
-    dn += D.gn[t] * s;
-    sy += s * y;
-    yy += y * y;
-  }
-  dn = bred<false>(dn, sh);
-  sy = bred<false>(sy, sh);
-  yy = bred<false>(yy, sh);
-  if (threadIdx.x == 0) {
-    D.part[5 * cf.nec + c] = dn;
-    D.part[6 * cf.nec + c] = sy;
-    D.part[7 * cf.nec + c] = yy;
-  }
-  A2C_ECHUNKS_END
-}
-
-// site-chunk partials of the energy and sigma-entropy sums
-__global__ void __launch_bounds__(kBlk) k_objpart(Dev D, Cfg cf, int all) {
-  __shared__ double sh[kBlk / 32];
-  for (int kk = blockIdx.x; kk < D.cnt[kCntSch]; kk += gridDim.x) {
-    const int c = D.ls[kk];
-    const Chunk ch = D.sch[c];
-    const Inst &I = D.st[ch.inst];
-    if (!all && I.state != kLineSearch && I.state != kNeedEval) continue;
-    double v = 0.0, s = 0.0;
-    for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-      v += D.Vs[ch.start + i];
-      s += D.Ss[ch.start + i];
-    }
-    v = bred<false>(v, sh);
-    s = bred<false>(s, sh);
-    if (threadIdx.x == 0) {
-      D.part[8 * cf.nec + c] = v;
-      D.part[8 * cf.nec + cf.nsc + c] = s;
-    }
-  }
 }
 
 // f = (1/T) sum V - 3 kB sum sigma  (minimizer.cpp:353)
@@ -579,22 +583,23 @@ __global__ void __launch_bounds__(kBlk) k_objective(Dev D, Cfg cf, double *f) {
   if (threadIdx.x == 0) f[b] = v;
 }
 
-// The line-search decision (lbfgs.cu, one instance per block).
-__global__ void __launch_bounds__(kBlk) k_decide(Dev D, Cfg cf) {
-  __shared__ double sh[kBlk / 32];
-  const int b = blockIdx.x;
+// The line-search decision (lbfgs.cu) of instance b, by a whole block.
+__device__ __forceinline__ void decide(const Dev &D, const Cfg &cf, int b, double *sh) {
   Inst &I = D.st[b];
-  if (I.state != kLineSearch && I.state != kNeedEval) return;
   const double fn = objective(D, cf, b, sh);
   const int e0 = D.ecb[b], e1 = D.ecb[b + 1];
-  const double dec = chunk_total(D.part + 4 * cf.nec, e0, e1, sh);
-  const double dn = chunk_total(D.part + 5 * cf.nec, e0, e1, sh);
-  const double sy = chunk_total(D.part + 6 * cf.nec, e0, e1, sh);
-  const double yy = chunk_total(D.part + 7 * cf.nec, e0, e1, sh);
+  const bool first = I.state == kNeedEval;
+  double dec = 0.0, dn = 0.0, sy = 0.0, yy = 0.0;
+  if (!first) {
+    dec = chunk_total(D.part + 4 * cf.nec, e0, e1, sh);
+    dn = chunk_total(D.part + 5 * cf.nec, e0, e1, sh);
+    sy = chunk_total(D.part + 6 * cf.nec, e0, e1, sh);
+    yy = chunk_total(D.part + 7 * cf.nec, e0, e1, sh);
+  }
   if (threadIdx.x != 0) return;
   I.fev += 1;
   I.fn = fn;
-  if (I.state == kNeedEval) {
+  if (first) {
     I.f = fn;
     I.copy = 2;
     I.nhist = 0;
@@ -620,7 +625,7 @@ __global__ void __launch_bounds__(kBlk) k_decide(Dev D, Cfg cf) {
       h[I.nhist % (W + 1)] = fn;
       I.nhist += 1;
       if (I.nhist > W && h[(I.nhist - 1 - W) % (W + 1)] - fn <= I.stall_rtol * fabs(fn)) {
-        end_phase(I, cf, A2C_CONVERGED_STALLED);
+        end_phase(I, cf, A2C_CONVERGED_STALLED, D.cnt);
         return;
       }
     }
@@ -636,21 +641,93 @@ __global__ void __launch_bounds__(kBlk) k_decide(Dev D, Cfg cf) {
       I.head = 0;
       I.state = kNeedDir;
     } else {
-      end_phase(I, cf, I.fev >= cf.max_fev ? A2C_DIVERGED_MAXFCN : A2C_DIVERGED_LS_FAILURE);
+      end_phase(I, cf, I.fev >= cf.max_fev ? A2C_DIVERGED_MAXFCN : A2C_DIVERGED_LS_FAILURE, D.cnt);
     }
+  }
+}
+
+// site-chunk partials of the energy and sigma-entropy sums
+__device__ __forceinline__ void objective_chunk(const Dev &D, const Cfg &cf, int c, const Chunk &ch, double *sh) {
+  double V[kPer], S[kPer];
+  load_chunk(D.Vs, ch, V);
+  load_chunk(D.Ss, ch, S);
+  double v = 0.0, s = 0.0;
+#pragma unroll
+  for (int e = 0; e < kPer; ++e) {
+    v += V[e];
+    s += S[e];
+  }
+  v = bsum(v, sh);
+  s = bsum(s, sh);
+  if (threadIdx.x == 0) {
+    D.part[8 * cf.nec + c] = v;
+    D.part[8 * cf.nec + cf.nsc + c] = s;
+  }
+}
+__global__ void __launch_bounds__(kBlk) k_objpart(Dev D, Cfg cf) {
+  __shared__ double sh[kBlk / 32];
+  for (int kk = blockIdx.x; kk < D.cnt[kCntSch]; kk += gridDim.x) objective_chunk(D, cf, D.ls[kk], D.sch[D.ls[kk]], sh);
+}
+
+// After the evaluation, one launch: blocks below `eblocks` take the element
+// chunks (the candidate pair into the free ring slot; gn.s, s.y, y.y), the
+// rest the site chunks (the objective's sums); the block that finishes an
+// instance's last chunk of either kind takes its line-search decision.
+__global__ void __launch_bounds__(kBlk) k_post(Dev D, Cfg cf, int eblocks) {
+  __shared__ double sh[kBlk / 32];
+  __shared__ int last;
+  const bool elements = (int)blockIdx.x < eblocks;
+  const int first = elements ? blockIdx.x : blockIdx.x - eblocks, step = elements ? eblocks : gridDim.x - eblocks;
+  const int n = elements ? D.cnt[kCntEch] : D.cnt[kCntSch];
+  for (int kk = first; kk < n; kk += step) {
+    const int c = elements ? D.le[kk] : D.ls[kk];
+    const Chunk ch = elements ? D.ech[c] : D.sch[c];
+    const int b = ch.inst;
+    Inst &I = D.st[b];
+    if (I.state != kLineSearch && I.state != kNeedEval) continue;
+    if (!elements) {
+      objective_chunk(D, cf, c, ch, sh);
+    } else if (I.state == kLineSearch) {
+      double s[kPer], y[kPer], x[kPer], g[kPer];
+      load_chunk(D.xn, ch, s);
+      load_chunk(D.x, ch, x);
+      load_chunk(D.gn, ch, g);
+      load_chunk(D.g, ch, y);
+      double dn = 0.0, sy = 0.0, yy = 0.0;
+#pragma unroll
+      for (int e = 0; e < kPer; ++e) {
+        s[e] = s[e] - x[e];
+        y[e] = g[e] - y[e];
+        dn += mul(g[e], s[e]);
+        sy += mul(s[e], y[e]);
+        yy += mul(y[e], y[e]);
+      }
+      store_chunk(D.S + (size_t)I.head * cf.n, ch, s);
+      store_chunk(D.Y + (size_t)I.head * cf.n, ch, y);
+      dn = bsum(dn, sh);
+      sy = bsum(sy, sh);
+      yy = bsum(yy, sh);
+      if (threadIdx.x == 0) {
+        D.part[5 * cf.nec + c] = dn;
+        D.part[6 * cf.nec + c] = sy;
+        D.part[7 * cf.nec + c] = yy;
+      }
+    }
+    if (chunk_done(I, D.ecb[b + 1] - D.ecb[b] + D.scb[b + 1] - D.scb[b], &last)) decide(D, cf, b, sh);
   }
 }
 
 // accepted step: x <- xn, g <- gn; first evaluation of a phase: g <- gn
 __global__ void __launch_bounds__(kBlk) k_copy(Dev D, Cfg cf) {
   A2C_ECHUNKS(D)
+  (void)b;
   if (!I.copy) continue;
   const bool both = I.copy == 1;
-  for (int i = threadIdx.x; i < ch.len; i += kBlk) {
-    const int64_t t = ch.start + i;
-    if (both) D.x[t] = D.xn[t];
-    D.g[t] = D.gn[t];
-  }
+  double x[kPer], g[kPer];
+  load_chunk(D.gn, ch, g);
+  if (both) load_chunk(D.xn, ch, x);
+  store_chunk(D.g, ch, g);
+  if (both) store_chunk(D.x, ch, x);
   A2C_ECHUNKS_END
 }
 
@@ -759,9 +836,11 @@ Dev dev_view(a2c_gpp_batch *b) {
 
 BatchView view(a2c_gpp_batch *b, int which) {
   BatchView v;
-  v.inst = b->inst;
   v.geo = b->geo;
-  v.list = which == 0 ? b->lm : b->lf;
+  if (b->B > 1) {  // one instance: while it is live its list is every site in order
+    v.inst = b->inst;
+    v.list = which == 0 ? b->lm : b->lf;
+  }
   v.count = b->cnt + (which == 0 ? kCntMixed : kCntFp64);
   return v;
 }
@@ -782,41 +861,29 @@ a2c_status plan(a2c_gpp_batch *b, const Dev &D) {
 
 Tile batch_tile(a2c_gpp_batch *b) { return effective_tile(b->tile, b->c->N, device_sms(b->c->device)); }
 
-// Evaluation of every listed site at xn into gn (both forms; a form with
-// an empty list costs an empty launch).
-a2c_status eval_lists(a2c_gpp_batch *b, const double *X, double *G, const Tile &tile) {
-  A2C_TRY(mixed_eval_list(b->c, X, G, view(b, 0), tile));
-  A2C_TRY(launch_eval64_list(b->c, X, G, view(b, 1)));
+// Evaluation of every listed site at X into G.  Both forms where a mixed
+// minimization ends in the FP64 polish (a form with an empty list costs an
+// empty launch); else only the form the minimization runs in.
+a2c_status eval_lists(a2c_gpp_batch *b, const double *X, double *G, const Cfg &cf, const Tile &tile) {
+  if (cf.mixed) A2C_TRY(mixed_eval_list(b->c, X, G, view(b, 0), tile));
+  if (!cf.mixed || cf.polish) A2C_TRY(launch_eval64_list(b->c, X, G, view(b, 1)));
   return A2C_OK;
 }
 
-// One tick (see the file comment); the same launches whether captured or not.
+// One tick (see the file comment); the same launches whether captured or
+// not.  262,144 sites, one instance, 5 pairs: MEASURED_TICK.
 a2c_status tick(a2c_gpp_batch *b, const Dev &D, const Cfg &cf, const Tile &tps) {
   cudaStream_t s = b->c->stream;
-  const int ge = chunk_grid(cf.nec), gs = chunk_grid(cf.nsc), B = cf.B;
+  const int ge = chunk_grid(cf.nec), gs = chunk_grid(cf.nsc);
   k_projgrad<<<ge, kBlk, 0, s>>>(D, cf);
-  k_dir_begin<<<B, kBlk, 0, s>>>(D, cf);
-  for (int j = 0; j < cf.m; ++j) {
-    k_loop1<<<ge, kBlk, 0, s>>>(D, cf, j);
-    k_loop1_fin<<<B, kBlk, 0, s>>>(D, cf, j);
-  }
-  k_scale<<<ge, kBlk, 0, s>>>(D, cf);
-  for (int j = 0; j < cf.m; ++j) {
-    k_loop2<<<ge, kBlk, 0, s>>>(D, cf, j);
-    k_loop2_fin<<<B, kBlk, 0, s>>>(D, cf, j);
-  }
+  for (int j = 1; j < cf.m; ++j) k_loop1<<<ge, kBlk, 0, s>>>(D, cf, j);
+  for (int j = 0; j < cf.m; ++j) k_loop2<<<ge, kBlk, 0, s>>>(D, cf, j);
   k_finish<<<ge, kBlk, 0, s>>>(D, cf);
-  k_dir_end<<<B, kBlk, 0, s>>>(D, cf);
-  k_steep<<<ge, kBlk, 0, s>>>(D, cf);
-  k_alpha0<<<B, kBlk, 0, s>>>(D, cf);
   A2C_TRY(plan(b, D));
   k_trial<<<ge, kBlk, 0, s>>>(D, cf);
-  A2C_TRY(eval_lists(b, b->xn, b->gn, tps));
-  k_post<<<ge, kBlk, 0, s>>>(D, cf);
-  k_objpart<<<gs, kBlk, 0, s>>>(D, cf, 0);
-  k_decide<<<B, kBlk, 0, s>>>(D, cf);
+  A2C_TRY(eval_lists(b, b->xn, b->gn, cf, tps));
+  k_post<<<ge + gs, kBlk, 0, s>>>(D, cf, ge);
   k_copy<<<ge, kBlk, 0, s>>>(D, cf);
-  k_count_left<<<1, kBlk, 0, s>>>(D, B);
   A2C_CUDA(cudaGetLastError());
   return A2C_OK;
 }
@@ -892,9 +959,11 @@ a2c_status init_tables(a2c_gpp_batch *b, const a2c_gpp_params *params, int n, bo
     for (int d = 0; d < 3; ++d) {
       G.S[d] = p.periodic[d] ? p.box[d] : kFreeSpan;
       G.sc[d] = (float)(G.S[d] / 4294967296.0);
+      G.unit[d] = 4294967296.0 / G.S[d];
     }
     set_limits(b, k, G);
     G.T = p.T;
+    G.invT = 1.0 / p.T;
     G.start = (int)s0;
     G.nPd = p.nPd;
     G.nH = p.nH;
@@ -960,6 +1029,7 @@ a2c_status setup_min(a2c_gpp_batch *b, const a2c_lbfgs_params *lp, Cfg &cf, Tile
   cf.max_ls = lp->max_ls;
   cf.polish = b->precision == A2C_MIXED ? lp->polish : 0;
   cf.W = lp->stall_window;
+  cf.mixed = b->precision == A2C_MIXED ? 1 : 0;
   cf.nec = b->nec;
   cf.nsc = b->nsc;
   cf.n = 4 * N;
@@ -1287,9 +1357,10 @@ a2c_status a2c_gpp_batch_eval(a2c_gpp_batch *b, const double *X, double *f, doub
   if (!st) st = plan(b, D);
   if (!st && cudaMemcpyAsync(c->d_X, X, sizeof(double) * 4 * N, cudaMemcpyHostToDevice, s) != cudaSuccess)
     st = A2C_ERR_CUDA;
-  if (!st) st = eval_lists(b, c->d_X, c->d_G, batch_tile(b));
+  cf.mixed = phase == kPhaseMixed ? 1 : 0;
+  if (!st) st = eval_lists(b, c->d_X, c->d_G, cf, batch_tile(b));
   if (!st) {
-    k_objpart<<<chunk_grid(b->nsc), kBlk, 0, s>>>(D, cf, 1);
+    k_objpart<<<chunk_grid(b->nsc), kBlk, 0, s>>>(D, cf);
     k_objective<<<b->B, kBlk, 0, s>>>(D, cf, df);
     if (cudaGetLastError() != cudaSuccess) st = A2C_ERR_CUDA;
   }

@@ -26,16 +26,24 @@ struct InstGeo {
   float sc[3];   // S / 2^32 (one fixed-point unit of the mixed form)
   int start;     // first site
   int nPd, nH;
+  double unit[3];       // 2^32 / S (the mixed form's fixed-point units per A)
+  double invT;          // 1 / T
   float lim[3];  // free direction: how far a site may move from its list position (span guard); else +inf
 };
 
 // What a list-driven evaluator launch reads: the instance of every site,
 // the per-instance geometry, and the sites to evaluate (count on device).
+// One instance alone has neither list nor inst: item k is site k of
+// instance 0.
 struct BatchView {
   const uint16_t *inst = nullptr;
   const InstGeo *geo = nullptr;
   const int *list = nullptr;
   const int *count = nullptr;
+#if defined(__CUDACC__)
+  __device__ __forceinline__ int64_t site(int64_t k) const { return list ? list[k] : k; }
+  __device__ __forceinline__ const InstGeo &geo_of(int64_t s) const { return geo[inst ? inst[s] : 0]; }
+#endif
 };
 
 // Device pointers and scalars one FP64 kernel launch needs.

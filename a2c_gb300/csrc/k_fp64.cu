@@ -125,8 +125,8 @@ __device__ __forceinline__ Site64 site64(const SiteArgs &a, int64_t k, int64_t n
   Site64 r;
   r.live = k < n;
   if (LIST) {
-    r.s = r.live ? a.bv.list[k] : 0;
-    const InstGeo &g = a.bv.geo[r.live ? a.bv.inst[r.s] : 0];
+    r.s = r.live ? a.bv.site(k) : 0;
+    const InstGeo &g = a.bv.geo_of(r.s);
     r.iPd = r.s - g.start < g.nPd;
     r.box = g.S;
     r.T = g.T;

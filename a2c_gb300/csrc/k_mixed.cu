@@ -169,22 +169,22 @@ struct SiteRef {
   int64_t s;
   bool iPd;
   float3 sc;
-  double T;
+  double invT;
 };
 template <bool LIST>
 __device__ __forceinline__ SiteRef<LIST> site_ref(const MixArgs &a, int64_t k) {
   SiteRef<LIST> r;
   if (LIST) {
-    r.s = a.bv.list[k];
-    const InstGeo &g = a.bv.geo[a.bv.inst[r.s]];
+    r.s = a.bv.site(k);
+    const InstGeo &g = a.bv.geo_of(r.s);
     r.iPd = r.s - g.start < g.nPd;
     r.sc = make_float3(g.sc[0], g.sc[1], g.sc[2]);
-    r.T = g.T;
+    r.invT = g.invT;
   } else {
     r.s = k;
     r.iPd = k < a.nPd;
     r.sc = make_float3(a.sc[0], a.sc[1], a.sc[2]);
-    r.T = a.T;
+    r.invT = 1.0 / a.T;
   }
   return r;
 }
@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_mixed(
     tot[k] = (double)v;
   }
   if (live && lane == 0) {
-    const double x = xi, sg = sigi, invT = 1.0 / R.T;
+    const double x = xi, sg = sigi, invT = R.invT;
     a.G[4 * s] = tot[0] * (invT * x);
     a.G[4 * s + 1] = tot[1] * (invT * x);
     a.G[4 * s + 2] = tot[2] * (invT * x);
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(M
     tot[k] = (double)v;
   }
   if (live && lane == 0) {  // the site's own share (16-byte stores: Gown is the library's); k_grad_recv completes G
-    const double x = xi, sg = sigi, invT = 1.0 / R.T;
+    const double x = xi, sg = sigi, invT = R.invT;
     double2 *own = reinterpret_cast<double2 *>(a.Gown + 4 * s);
     own[0] = make_double2(tot[0] * (invT * x), tot[1] * (invT * x));
     own[1] = make_double2(tot[2] * (invT * x),
@@ -832,7 +832,7 @@ __global__ void __launch_bounds__(kBlock) k_grad_recv(MixArgs a) {
     // where scattered 8-byte stores are slow)
     static_assert(TPS >= 4, "one lane per gradient component");
     if (live && lane < 4) {
-      const double x = a.occ[s], invT = 1.0 / R.T;
+      const double x = a.occ[s], invT = R.invT;
       const double v = lane == 0 ? tot[0] : lane == 1 ? tot[1] : lane == 2 ? tot[2] : tot[3];
       const double scale = lane == 3 ? 1.7320508075688772 * 1.4142135623730951 * invT * x : invT * x;
       a.G[4 * s + lane] = a.Gown[4 * s + lane] + v * scale;
@@ -1009,13 +1009,13 @@ __global__ void k_prep_list(const double *X, const double *occ, BatchView bv, in
                             int *status) {
   const int n = *bv.count;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    const int64_t s = bv.list[k];
-    const InstGeo &g = bv.geo[bv.inst[s]];
+    const int64_t s = bv.site(k);
+    const InstGeo &g = bv.geo_of(s);
     const double4 x = make_double4(X[4 * s], X[4 * s + 1], X[4 * s + 2], X[4 * s + 3]);
     span_check(x, xl, s, g.lim[0], g.lim[1], g.lim[2], status);
-    const long long u0 = __double2ll_rn(x.x * (4294967296.0 / g.S[0]));
-    const long long u1 = __double2ll_rn(x.y * (4294967296.0 / g.S[1]));
-    const long long u2 = __double2ll_rn(x.z * (4294967296.0 / g.S[2]));
+    const long long u0 = __double2ll_rn(x.x * g.unit[0]);
+    const long long u1 = __double2ll_rn(x.y * g.unit[1]);
+    const long long u2 = __double2ll_rn(x.z * g.unit[2]);
     P[s] = make_int4((int)(unsigned)u0, (int)(unsigned)u1, (int)(unsigned)u2, __float_as_int((float)x.w));
     occf[s] = (float)occ[s];
   }
@@ -1316,8 +1316,15 @@ int mixed_threads_per_site(a2c_gpp_ctx *c) { return (c->mixed && c->mixed->tps) 
 Tile effective_tile(const Tile &t, int64_t n_sites, int sms) {
   Tile e;
   e.tps = t.tps ? t.tps : default_threads_per_site(n_sites, sms);
-  e.rho_block = t.rho_block ? t.rho_block : kBlock;
-  e.grad_block = t.grad_block ? t.grad_block : kBlock;
+  // Block sizes when none was chosen (they change no result).  Pass 1: two
+  // blocks fit an SM whatever their size, so 512 threads double its warps
+  // (262,144 sites at 4 threads per site: 178 -> 141 us; 33,592: 31 -> 27;
+  // 512: 15.4 either way), except with one thread per site (373,248 sites:
+  // 233 us at 256, 266 at 512).  Pass 2: 128 threads while there are few
+  // blocks to spread (512 sites: 27 against 29 us, 33,592: 54 against 56;
+  // 92,160: 115 against 113).
+  e.rho_block = t.rho_block ? t.rho_block : e.tps > 1 ? 512 : kBlock;
+  e.grad_block = t.grad_block ? t.grad_block : n_sites < 256 * (int64_t)sms ? 128 : kBlock;
   return e;
 }
 
