@@ -76,8 +76,9 @@ enum : int { kStatusNonfinite = 1, kStatusOverflow = 2, kStatusTimeout = 4, kSta
 // less than half of it apart.
 constexpr double kFreeSpan = 64.0;
 
-// doubles of a context's pinned scratch, and where the list builds' reports start in it
-constexpr int kHostSmall = 32, kHostReport = 8;
+// doubles of a context's pinned scratch: f and the status word of an
+// evaluation (0, 1), and where the other results start in it
+constexpr int kHostSmall = 32, kHostStatus = 2, kHostMacro = 4, kHostReport = 8;
 
 struct Mixed;   // mixed-precision buffers (k_mixed.cu)
 struct Lbfgs;   // L-BFGS buffers (lbfgs.cu)
@@ -123,6 +124,7 @@ struct a2c_gpp_ctx {
   a2c::Mixed *mixed;
   a2c::Lbfgs *lbfgs;
   void *snap;  // the snapshot in flight (api.cu)
+  void *hscratch;   // scratch of the occupancy calls (api.cu), created on first use
   void *list_work;  // scratch of the list builds (k_neighbors.cu), created on first use
   void *engine;     // the device-driven minimizer (batch.cu), created on first use
   int host_loop;    // L-BFGS driver, A2C_MINIMIZER_* (a2c_gpp_set_minimizer)
@@ -191,11 +193,15 @@ a2c_status launch_diffuse(a2c_gpp_ctx *c, const double *d_gamma, const int *d_fu
                           double Qm, double xLb, double xUb, double *d_x);
 a2c_status launch_dirichlet(a2c_gpp_ctx *c, const int *d_sites, int n, double gamma_bd, double xUb, double *d_gamma,
                             int *d_full);
+// waits, and checks the status word
 a2c_status launch_macro(a2c_gpp_ctx *c, const double *d_x, const int *d_surf_flags, int nSurf, double *h_xH,
                         double *h_xHint);
 // the same reduction into d_out[2] on the device (stream-ordered, capturable)
 a2c_status launch_macro_device(a2c_gpp_ctx *c, const double *d_x, const int *d_surf_flags, int nSurf, double *d_out);
+a2c_status launch_flags(a2c_gpp_ctx *c, const int *d_sites, int n, int *d_flags);
+// waits for the stream and reads (and clears) the device status word
 a2c_status check_status_word(a2c_gpp_ctx *c);
+a2c_status status_of(const void *word);  // what a status word read back says
 
 // k_neighbors.cu
 // What one pass over new positions finds: checks, extents, scale.

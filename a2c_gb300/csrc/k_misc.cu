@@ -3,6 +3,7 @@
 // diffusion step and the macro results.  Compiled with -fmad=false.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "ddmath.cuh"
 #include "internal.cuh"
@@ -96,9 +97,15 @@ __global__ void k_dirichlet(const int *sites, int n, double gamma_bd, double xUb
     atomicOr(status, kStatusBadIndex);
     return;
   }
-  gamma[i] = gamma_bd;
-  full[i] = 1;
+  if (gamma) gamma[i] = gamma_bd;  // null: the host entry point sets the caller's arrays
+  if (full) full[i] = 1;
   xH[i] = xUb;
+}
+
+// flags of the listed sites (those in range), 0 elsewhere
+__global__ void k_flags(const int *sites, int n, int nH, int *flags) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n && sites[t] >= 0 && sites[t] < nH) flags[sites[t]] = 1;
 }
 
 // integrate.cpp:26-81: explicit Euler step of the hop-rate master equation
@@ -251,29 +258,44 @@ a2c_status launch_macro_device(a2c_gpp_ctx *c, const double *d_x, const int *d_s
   return A2C_OK;
 }
 
+a2c_status launch_flags(a2c_gpp_ctx *c, const int *d_sites, int n, int *d_flags) {
+  A2C_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * c->p.nH, c->stream));
+  if (n > 0) {
+    k_flags<<<grid_for(n, 256), 256, 0, c->stream>>>(d_sites, n, c->p.nH, d_flags);
+    A2C_CUDA(cudaGetLastError());
+  }
+  return A2C_OK;
+}
+
 a2c_status launch_macro(a2c_gpp_ctx *c, const double *d_x, const int *d_surf_flags, int nSurf, double *h_xH,
                         double *h_xHint) {
   double *out = c->d_red + 2 * kRedGrid + 4;
   A2C_TRY(launch_macro_device(c, d_x, d_surf_flags, nSurf, out));
-  double h[2];
-  A2C_CUDA(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-  A2C_CUDA(cudaStreamSynchronize(c->stream));
-  *h_xH = h[0];
-  *h_xHint = h[1];
-  return A2C_OK;
+  A2C_CUDA(cudaMemcpyAsync(c->h_small + kHostMacro, out, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  const a2c_status st = check_status_word(c);
+  *h_xH = c->h_small[kHostMacro];
+  *h_xHint = c->h_small[kHostMacro + 1];
+  return st;
 }
 
-a2c_status check_status_word(a2c_gpp_ctx *c) {
+a2c_status status_of(const void *word) {
   int st = 0;
-  A2C_CUDA(cudaMemcpyAsync(&st, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-  A2C_CUDA(cudaStreamSynchronize(c->stream));
-  A2C_CUDA(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
+  std::memcpy(&st, word, sizeof(int));
   if (st & kStatusBadIndex) return A2C_ERR_INVALID;
   if (st & kStatusOverflow) return A2C_ERR_NEIGHBOR_OVERFLOW;
   if (st & kStatusTimeout) return A2C_ERR_TIMEOUT;
   if (st & kStatusNonfinite) return A2C_ERR_NONFINITE;
   if (st & kStatusSpan) return A2C_ERR_LISTS_STALE;
   return A2C_OK;
+}
+
+// Waits for the stream; the word comes through pinned memory, cleared on
+// the device in the same order.
+a2c_status check_status_word(a2c_gpp_ctx *c) {
+  A2C_CUDA(cudaMemcpyAsync(c->h_small + kHostStatus, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  A2C_CUDA(cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream));
+  A2C_CUDA(cudaStreamSynchronize(c->stream));
+  return status_of(c->h_small + kHostStatus);
 }
 
 }  // namespace a2c
