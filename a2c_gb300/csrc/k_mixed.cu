@@ -30,9 +30,14 @@
 // beyond 5.35 A are C1 continuations, selected branch-free); F and F' per
 // site from FP32 Hermite tables in rho.
 //
-// Mapping: TPS threads per site (1, 2, 4 or 8), each taking every TPS-th
+// Mapping: V threads per site (1, 2, 4 or 8), each taking every V-th
 // neighbor, first among the Pd then among the H neighbors (so the lanes of a
-// warp evaluate the same pair type together), combined by shuffles.
+// warp evaluate the same pair type together), combined by shuffles.  V sets
+// the order of a site's sums.  Where that many lanes leave the device idle
+// (few sites) or serve it badly (one lane per site), TPS > V lanes evaluate
+// the site's neighbors TPS at a time and hand the terms round, each lane
+// adding those its V-th part would have met, in the same order: the same
+// bits (walk_together, add_pairs; effective_tile says when).
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -152,6 +157,14 @@ __device__ __forceinline__ float rsq(float x) {
 }
 __device__ __forceinline__ void kahan(float &s, float &c, float v) {
   const float y = v - c;
+  const float t = s + y;
+  c = (t - s) - y;
+  s = t;
+}
+
+// The same for the product a b, rounded once with the compensation.
+__device__ __forceinline__ void kahan_product(float &s, float &c, float a, float b) {
+  const float y = fmaf(a, b, -c);
   const float t = s + y;
   c = (t - s) - y;
   s = t;
@@ -279,6 +292,39 @@ __device__ __forceinline__ void walk_neighbors(const MixArgs &a, int64_t begin, 
   }
 }
 
+// The same for a site whose TPS lanes stand for V lanes of R = TPS / V
+// neighbors each (see "Mapping"): the lanes step together, TPS neighbors at
+// a time; body(valid, t, first, ...) runs in all of them, t = first + lane.
+template <int TPS, bool OCC, bool FP, class Body>
+__device__ __forceinline__ void walk_together(const MixArgs &a, int64_t begin, int64_t end, int lane, Body body) {
+  int64_t t = begin + lane;
+  int64_t j0 = t < end ? __ldg(&a.nbr[t]) & kIdMask : 0;
+  int4 p0 = __ldg(&a.P[j0]);
+  float x0 = OCC ? __ldg(&a.occ[j0]) : 1.0f;
+  float f0 = FP ? __ldg(&a.FF[j0].x) : 0.0f;
+  uint32_t e1 = t + TPS < end ? __ldg(&a.nbr[t + TPS]) : 0u;
+  for (int64_t first = begin; first < end; first += TPS, t += TPS) {
+    int4 p1 = p0;
+    float x1 = x0, f1 = f0;
+    if (t + TPS < end) {
+      const int64_t j1 = e1 & kIdMask;
+      p1 = __ldg(&a.P[j1]);
+      if (OCC) x1 = __ldg(&a.occ[j1]);
+      if (FP) f1 = __ldg(&a.FF[j1].x);
+    }
+    if (t + 2 * TPS < end) e1 = __ldg(&a.nbr[t + 2 * TPS]);
+    body(t < end, t, first, p0, x0, f0);
+    p0 = p1;
+    x0 = x1;
+    f0 = f1;
+  }
+}
+// The lanes of this site's group within the warp.
+template <int TPS>
+__device__ __forceinline__ unsigned site_lanes() {
+  return TPS == 32 ? 0xffffffffu : ((1u << (TPS & 31)) - 1u) << ((threadIdx.x % 32) & ~(TPS - 1));
+}
+
 // The per-site finish of pass 1: rho = W * (sum of the density terms), then
 // F'(rho) and F(rho) from the embedding table of the site's species.
 __device__ __forceinline__ void rho_finish(const MixArgs &a, int64_t s, bool iPd, float tot) {
@@ -314,15 +360,53 @@ constexpr int kGradCopies = A2C_GRAD_COPIES;
 constexpr int kGradTabN = kTabN;  // phi_Pd is -3e-4 eV at 5.8 A: every interval
 constexpr size_t kGradSmem = 2 * sizeof(float4) * kGradTabN * kGradCopies;
 
-template <int TPS, bool LIST, int BLOCK>
+// The density terms of one neighbor: f_Pd from the table (COPIES copies,
+// this lane's from sF), or f_H.
+template <int COPIES>
+__device__ __forceinline__ float rho_terms_Pd(const float4 *sF, float3 D, float ui, float uj) {
+  const float D2 = fmaf(D.x, D.x, fmaf(D.y, D.y, D.z * D.z));
+  const float Ai = fmaf(ui, ui, D2), Aj = fmaf(uj, uj, D2);
+  float part = 0.0f;
+  const float Dv[3] = {D.x, D.y, D.z};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    A2C_RADII(c, Dv[c])
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float r = s2[q] * rsq(s2[q]);
+      float tt;
+      const int i = tab_index<kRhoTabN>(r, tt);
+      part += hv(sF[COPIES * i], tt);
+    }
+  }
+  return part;
+}
+__device__ __forceinline__ float rho_terms_H(const ExpTerms &ex, float3 D, float ui, float uj) {
+  const float D2 = fmaf(D.x, D.x, fmaf(D.y, D.y, D.z * D.z));
+  const float Ai = fmaf(ui, ui, D2), Aj = fmaf(uj, uj, D2);
+  float part = 0.0f;
+  const float Dv[3] = {D.x, D.y, D.z};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    A2C_RADII(c, Dv[c])
+#pragma unroll
+    for (int q = 0; q < 4; ++q) part += fH(ex, s2[q] * rsq(s2[q]));
+  }
+  return part;
+}
+
+// V lanes per site in the order of its sums, TPS in the work (see
+// "Mapping"); one copy of the table where few sites share a block (TPS =
+// 32: its 98 KB took longer to fill than the lookups' bank conflicts cost).
+template <int V, int TPS, bool LIST, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, rho_min_blocks<BLOCK>()) k_rho_mixed(MixArgs a) {
-  constexpr int kSitesPerBlock = BLOCK / TPS;
+  constexpr int kSitesPerBlock = BLOCK / TPS, kCopies = TPS == 32 ? 1 : kRhoCopies;
   const int64_t n = LIST ? (int64_t)*a.bv.count : a.N;
   if ((int64_t)blockIdx.x * kSitesPerBlock >= n) return;
   extern __shared__ float4 sF8[];
-  for (int i = threadIdx.x; i < kRhoTabN * kRhoCopies; i += blockDim.x) sF8[i] = __ldg(&a.tabPair[i / kRhoCopies]);
+  for (int i = threadIdx.x; i < kRhoTabN * kCopies; i += blockDim.x) sF8[i] = __ldg(&a.tabPair[i / kCopies]);
   __syncthreads();
-  const float4 *sF = sF8 + (threadIdx.x % kRhoCopies);  // this lane's copy: interval i at sF[8 i]
+  const float4 *sF = sF8 + (threadIdx.x % kCopies);  // this lane's copy: interval i at sF[kCopies i]
   for (int64_t base = (int64_t)blockIdx.x * kSitesPerBlock; base < n;
        base += (int64_t)gridDim.x * kSitesPerBlock) {
   const int64_t k = base + threadIdx.x / TPS;
@@ -334,47 +418,45 @@ __global__ void __launch_bounds__(BLOCK, rho_min_blocks<BLOCK>()) k_rho_mixed(Mi
   float acc = 0.0f, cmp = 0.0f;
   if (live) {
     const int4 pi = a.P[s];
-    const float ui = kSqrt6 * __int_as_float(pi.w), ui2 = ui * ui;
+    const float ui = kSqrt6 * __int_as_float(pi.w);
     const int64_t b = a.off[s], m = b + a.npd[s], e = a.off[s + 1];
-    walk_neighbors<false, false>(a, b + lane, m, TPS, [&](int64_t, int4 pj, float, float) {  // Pd neighbors: f_Pd
-      const float3 D = pair_vec(R.sc, pi, pj);
-      const float uj = kSqrt6 * __int_as_float(pj.w);
-      const float D2 = fmaf(D.x, D.x, fmaf(D.y, D.y, D.z * D.z));
-      const float Ai = D2 + ui2, Aj = fmaf(uj, uj, D2);
-      float part = 0.0f;
-      const float Dv[3] = {D.x, D.y, D.z};
+    if constexpr (V == TPS) {
+      walk_neighbors<false, false>(a, b + lane, m, TPS, [&](int64_t, int4 pj, float, float) {  // Pd neighbors: f_Pd
+        const float3 D = pair_vec(R.sc, pi, pj);
+        kahan(acc, cmp, rho_terms_Pd<kCopies>(sF, D, ui, kSqrt6 * __int_as_float(pj.w)));
+      });
+      walk_neighbors<true, false>(a, m + lane, e, TPS, [&](int64_t, int4 pj, float xj, float) {  // H: x_j f_H
+        const float3 D = pair_vec(R.sc, pi, pj);
+        const float part = rho_terms_H(a.ex, D, ui, kSqrt6 * __int_as_float(pj.w));
+        kahan_product(acc, cmp, part, xj);
+      });
+    } else {
+      const unsigned group = site_lanes<TPS>();
+      walk_together<TPS, false, false>(a, b, m, lane, [&](bool valid, int64_t, int64_t first, int4 pj, float, float) {
+        float part = 0.0f;
+        if (valid) part = rho_terms_Pd<kCopies>(sF, pair_vec(R.sc, pi, pj), ui, kSqrt6 * __int_as_float(pj.w));
+        __syncwarp(group);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        A2C_RADII(c, Dv[c])
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const float r = s2[q] * rsq(s2[q]);
-          float tt;
-          const int i = tab_index<kRhoTabN>(r, tt);
-          part += hv(sF[kRhoCopies * i], tt);
+        for (int q = 0; q < TPS; q += V) {
+          const float v = __shfl_sync(group, part, q + lane % V, TPS);
+          if (first + q + lane % V < m) kahan(acc, cmp, v);
         }
-      }
-      kahan(acc, cmp, part);
-    });
-    walk_neighbors<true, false>(a, m + lane, e, TPS, [&](int64_t, int4 pj, float xj, float) {  // H neighbors: x_j f_H
-      const float3 D = pair_vec(R.sc, pi, pj);
-      const float uj = kSqrt6 * __int_as_float(pj.w);
-      const float D2 = fmaf(D.x, D.x, fmaf(D.y, D.y, D.z * D.z));
-      const float Ai = D2 + ui2, Aj = fmaf(uj, uj, D2);
-      float part = 0.0f;
-      const float Dv[3] = {D.x, D.y, D.z};
+      });
+      walk_together<TPS, true, false>(a, m, e, lane, [&](bool valid, int64_t, int64_t first, int4 pj, float xj, float) {
+        float part = 0.0f;
+        if (valid) part = rho_terms_H(a.ex, pair_vec(R.sc, pi, pj), ui, kSqrt6 * __int_as_float(pj.w));
+        __syncwarp(group);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        A2C_RADII(c, Dv[c])
-#pragma unroll
-        for (int q = 0; q < 4; ++q) part += fH(a.ex, s2[q] * rsq(s2[q]));
-      }
-      kahan(acc, cmp, part * xj);
-    });
+        for (int q = 0; q < TPS; q += V) {
+          const float v = __shfl_sync(group, part, q + lane % V, TPS), x = __shfl_sync(group, xj, q + lane % V, TPS);
+          if (first + q + lane % V < e) kahan_product(acc, cmp, v, x);
+        }
+      });
+    }
   }
   float tot = acc;
 #pragma unroll
-  for (int o = TPS / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+  for (int o = V / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
   if (live && lane == 0) rho_finish(a, s, R.iPd, tot);
   }
 }
@@ -473,7 +555,7 @@ __device__ __forceinline__ void add_pair(SiteAcc &A, const PairAcc &p, float3 D,
   A.s[1] = fmaf(wx, fmaf(D.y, p.csum, p.e[1]), A.s[1]);
   A.s[2] = fmaf(wx, fmaf(D.z, p.csum, p.e[2]), A.s[2]);
   A.s[3] = fmaf(wx, p.sig, A.s[3]);
-  kahan(A.s[4], A.c[4], vx * p.v);
+  kahan_product(A.s[4], A.c[4], vx, p.v);
 }
 
 // The objective of a single system, f = (1/T) sum_i V_i - 3 kB sum_i x_i
@@ -713,7 +795,31 @@ __device__ __forceinline__ void send_share(const MixArgs &a, uint32_t slot, cons
                              -w * fmaf(D.z, p.csum, p.e[2]), w * p.sigj);
 }
 
-template <int TPS, bool LIST, int BLOCK>
+// The neighbors of one step added in the order of V lanes (V < TPS): lane l
+// adds those at l % V, l % V + V, ... of the step, as lane l % V alone would.
+template <int V, int TPS, bool OCC>
+__device__ __forceinline__ void add_pairs(SiteAcc &A, const PairAcc &p, float3 D, float W, float w, float xj,
+                                          unsigned group, int lane, int64_t first, int64_t end) {
+  const float ux = fmaf(D.x, p.csum, p.e[0]), uy = fmaf(D.y, p.csum, p.e[1]), uz = fmaf(D.z, p.csum, p.e[2]);
+  __syncwarp(group);
+#pragma unroll
+  for (int q = 0; q < TPS; q += V) {
+    const int src = q + lane % V;
+    const float x = __shfl_sync(group, ux, src, TPS), y = __shfl_sync(group, uy, src, TPS),
+                z = __shfl_sync(group, uz, src, TPS), g = __shfl_sync(group, p.sig, src, TPS),
+                v = __shfl_sync(group, p.v, src, TPS), o = OCC ? __shfl_sync(group, xj, src, TPS) : 1.0f;
+    if (first + src < end) {
+      const float wx = OCC ? W * o : W, vx = OCC ? w * o : w;
+      A.s[0] = fmaf(wx, x, A.s[0]);
+      A.s[1] = fmaf(wx, y, A.s[1]);
+      A.s[2] = fmaf(wx, z, A.s[2]);
+      A.s[3] = fmaf(wx, g, A.s[3]);
+      kahan_product(A.s[4], A.c[4], vx, v);
+    }
+  }
+}
+
+template <int V, int TPS, bool LIST, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(MixArgs a) {
   constexpr int kSitesPerBlock = BLOCK / TPS;
   const int64_t n = LIST ? (int64_t)*a.bv.count : a.N;
@@ -747,38 +853,74 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(M
     const bool iPd = R.iPd;
     const int64_t b = a.off[s], m = b + a.npd[s], p = b + a.npre[s];
     const float w = a.W * xi;  // the neighbor's share and the pair energy carry W x_i
-    walk_neighbors<false, true>(a, b + lane, m < p ? m : p, TPS, [&](int64_t t, int4 pj, float, float Fb) {
-      const uint32_t slot = __ldg(&a.rev[t]);
-      const float3 D = pair_vec(R.sc, pi, pj);
-      const float uj = kSqrt6 * __int_as_float(pj.w);
-      PairAcc q;
-      if (iPd) {
-        pair_terms<0>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
-      } else if (pair_inside(D, ui, uj)) {
-        pair_terms<2, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
-      } else {
-        pair_terms<2, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
-      }
-      add_pair(A, q, D, a.W, w);
-      send_share(a, slot, q, D, w);
-    });
-    walk_neighbors<true, true>(a, m + lane, p, TPS, [&](int64_t t, int4 pj, float xj, float Fb) {  // H site, H j < i
-      const uint32_t slot = __ldg(&a.rev[t]);
-      const float3 D = pair_vec(R.sc, pi, pj);
-      const float uj = kSqrt6 * __int_as_float(pj.w);
-      PairAcc q;
-      if (pair_inside(D, ui, uj)) pair_terms<3, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
-      else pair_terms<3, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
-      add_pair(A, q, D, a.W * xj, w * xj);
-      send_share(a, slot, q, D, w);
-    });
+    const int64_t mp = m < p ? m : p;
+    if constexpr (V == TPS) {
+      walk_neighbors<false, true>(a, b + lane, mp, TPS, [&](int64_t t, int4 pj, float, float Fb) {
+        const uint32_t slot = __ldg(&a.rev[t]);
+        const float3 D = pair_vec(R.sc, pi, pj);
+        const float uj = kSqrt6 * __int_as_float(pj.w);
+        PairAcc q;
+        if (iPd) {
+          pair_terms<0>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+        } else if (pair_inside(D, ui, uj)) {
+          pair_terms<2, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+        } else {
+          pair_terms<2, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+        }
+        add_pair(A, q, D, a.W, w);
+        send_share(a, slot, q, D, w);
+      });
+      walk_neighbors<true, true>(a, m + lane, p, TPS, [&](int64_t t, int4 pj, float xj, float Fb) {  // H site, H j < i
+        const uint32_t slot = __ldg(&a.rev[t]);
+        const float3 D = pair_vec(R.sc, pi, pj);
+        const float uj = kSqrt6 * __int_as_float(pj.w);
+        PairAcc q;
+        if (pair_inside(D, ui, uj)) pair_terms<3, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+        else pair_terms<3, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+        add_pair(A, q, D, a.W * xj, w * xj);
+        send_share(a, slot, q, D, w);
+      });
+    } else {
+      const unsigned group = site_lanes<TPS>();
+      walk_together<TPS, false, true>(a, b, mp, lane,
+                                      [&](bool valid, int64_t t, int64_t first, int4 pj, float, float Fb) {
+        const float3 D = pair_vec(R.sc, pi, pj);
+        PairAcc q{};
+        if (valid) {
+          const uint32_t slot = __ldg(&a.rev[t]);
+          const float uj = kSqrt6 * __int_as_float(pj.w);
+          if (iPd) {
+            pair_terms<0>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          } else if (pair_inside(D, ui, uj)) {
+            pair_terms<2, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          } else {
+            pair_terms<2, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          }
+          send_share(a, slot, q, D, w);
+        }
+        add_pairs<V, TPS, false>(A, q, D, a.W, w, 1.0f, group, lane, first, mp);
+      });
+      walk_together<TPS, true, true>(a, m, p, lane,
+                                     [&](bool valid, int64_t t, int64_t first, int4 pj, float xj, float Fb) {
+        const float3 D = pair_vec(R.sc, pi, pj);
+        PairAcc q{};
+        if (valid) {
+          const uint32_t slot = __ldg(&a.rev[t]);
+          const float uj = kSqrt6 * __int_as_float(pj.w);
+          if (pair_inside(D, ui, uj)) pair_terms<3, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          else pair_terms<3, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          send_share(a, slot, q, D, w);
+        }
+        add_pairs<V, TPS, true>(A, q, D, a.W, w, xj, group, lane, first, p);
+      });
+    }
   }
   double tot[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
     float v = A.s[k] - A.c[k];
 #pragma unroll
-    for (int o = TPS / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = V / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     tot[k] = (double)v;
   }
   if (live && lane == 0) {  // the site's own share (16-byte stores: Gown is the library's); k_grad_recv completes G
@@ -1104,35 +1246,72 @@ inline unsigned persistent_grid(int64_t n_items, int per_block, int cap) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n_items + per_block - 1) / per_block, cap));
 }
 
-template <int TPS, bool LIST, int B>
+template <int V, int TPS, bool LIST, int B>
 void launch_rho(const MixArgs &a, cudaStream_t st) {
-  const void *fn = (const void *)k_rho_mixed<TPS, LIST, B>;
-  k_rho_mixed<TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, kRhoSmem)), B, kRhoSmem, st>>>(a);
+  const void *fn = (const void *)k_rho_mixed<V, TPS, LIST, B>;
+  constexpr size_t smem = TPS == 32 ? kRhoSmem / kRhoCopies : kRhoSmem;
+  k_rho_mixed<V, TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, smem)), B, smem, st>>>(a);
+}
+template <int V, int TPS, bool LIST, int B>
+void launch_once(const MixArgs &a, cudaStream_t st) {
+  const void *fn = (const void *)k_grad_once<V, TPS, LIST, B>;
+  k_grad_once<V, TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, kGradSmem)), B, kGradSmem, st>>>(a);
 }
 template <int TPS, bool LIST, int B>
 void launch_grad(const MixArgs &a, cudaStream_t st, bool once) {
   if (once) {
-    const void *fn = (const void *)k_grad_once<TPS, LIST, B>;
-    k_grad_once<TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, kGradSmem)), B, kGradSmem, st>>>(a);
+    launch_once<TPS, TPS, LIST, B>(a, st);
   } else {
     const void *fn = (const void *)k_grad_mixed<TPS, LIST, B>;
     k_grad_mixed<TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, kGradSmem)), B, kGradSmem, st>>>(a);
   }
 }
 
-template <int TPS, bool LIST>
-void launch_pair_kernels(const MixArgs &a, cudaStream_t st, cudaEvent_t *ev, bool once, const Tile &t) {
+// Pass 1 at V lanes per site in its sums' order, on the lanes the size asks
+// for (see spread).
+template <int V, bool LIST>
+void launch_pass1(const MixArgs &a, cudaStream_t st, const Tile &t) {
+  if (t.wide) {
+    launch_rho<V, 32, LIST, 128>(a, st);
+    return;
+  }
+  if constexpr (V == 1) {
+    if (t.twin) {
+      launch_rho<1, 2, LIST, 512>(a, st);
+      return;
+    }
+  }
   switch (t.rho_block) {
-    case 512: launch_rho<TPS, LIST, 512>(a, st); break;
-    case 768: launch_rho<TPS, LIST, 768>(a, st); break;
-    default: launch_rho<TPS, LIST, 256>(a, st); break;
+    case 512: launch_rho<V, V, LIST, 512>(a, st); break;
+    case 768: launch_rho<V, V, LIST, 768>(a, st); break;
+    default: launch_rho<V, V, LIST, 256>(a, st); break;
   }
-  if (ev) cudaEventRecord(ev[2], st);
+}
+
+template <int V, bool LIST>
+void launch_pass2(const MixArgs &a, cudaStream_t st, bool once, const Tile &t) {
+  if (once && t.wide) {
+    launch_once<V, 32, LIST, 128>(a, st);
+    return;
+  }
+  if constexpr (V == 1) {
+    if (once && t.twin) {
+      launch_once<1, 2, LIST, 256>(a, st);
+      return;
+    }
+  }
   switch (t.grad_block) {
-    case 128: launch_grad<TPS, LIST, 128>(a, st, once); break;
-    case 512: launch_grad<TPS, LIST, 512>(a, st, once); break;
-    default: launch_grad<TPS, LIST, 256>(a, st, once); break;
+    case 128: launch_grad<V, LIST, 128>(a, st, once); break;
+    case 512: launch_grad<V, LIST, 512>(a, st, once); break;
+    default: launch_grad<V, LIST, 256>(a, st, once); break;
   }
+}
+
+template <int V, bool LIST>
+void launch_pair_kernels(const MixArgs &a, cudaStream_t st, cudaEvent_t *ev, bool once, const Tile &t) {
+  launch_pass1<V, LIST>(a, st, t);
+  if (ev) cudaEventRecord(ev[2], st);
+  launch_pass2<V, LIST>(a, st, once, t);
   if (once) {
     const void *fn = (const void *)k_grad_recv<kRecvTps, LIST>;
     k_grad_recv<kRecvTps, LIST><<<persistent_grid(a.N, kBlock / kRecvTps, grid_cap(fn, kBlock, 0)), kBlock, 0, st>>>(a);
@@ -1323,6 +1502,16 @@ Tile effective_tile(const Tile &t, int64_t n_sites, int sms) {
   // 233 us at 256, 266 at 512).  Pass 2: 128 threads while there are few
   // blocks to spread (512 sites: 27 against 29 us, 33,592: 54 against 56;
   // 92,160: 115 against 113).
+  // More lanes per site than its sums' order asks for, where no block size
+  // was chosen: a warp for a site while there are few (passes 1 and 2 with
+  // 4 / 32 lanes, 512 sites: 16.4 + 26.8 / 8.1 + 18.9 us, 4,096: 16.4 + 26.8
+  // / 14.3 + 25.2, 8,000: 16.4 + 29.3 / 19.8 + 37.1), two lanes in place of
+  // one (512,000 sites: 315 + 614 / 303 + 580 us, 2,097,152: 1215 + 2559 /
+  // 1131 + 2399).
+  if (!t.rho_block && !t.grad_block) {
+    e.wide = n_sites <= 27 * (int64_t)sms;
+    e.twin = !e.wide && e.tps == 1;
+  }
   e.rho_block = t.rho_block ? t.rho_block : e.tps > 1 ? 512 : kBlock;
   e.grad_block = t.grad_block ? t.grad_block : n_sites < 256 * (int64_t)sms ? 128 : kBlock;
   return e;
@@ -1499,12 +1688,10 @@ a2c_status mixed_chem(a2c_gpp_ctx *c, const double *dX, double *d_send, const in
   a.T = c->p.T;
   // the state's fixed-point form and pass 1 (F and F' of every site)
   k_prep<<<grid_for(N, 256), 256, 0, c->stream>>>(dX, c->d_occ, N, k[0], k[1], k[2], M->P, M->occ, span_args(c));
-  const Tile t = effective_tile(mixed_tile(c), N, device_sms(c->device));
-  switch (t.rho_block) {
-    case 512: launch_rho<1, false, 512>(a, c->stream); break;
-    case 768: launch_rho<1, false, 768>(a, c->stream); break;
-    default: launch_rho<1, false, 256>(a, c->stream); break;
-  }
+  Tile one = mixed_tile(c);
+  one.tps = 1;
+  const Tile t = effective_tile(one, N, device_sms(c->device));
+  launch_pass1<1, false>(a, c->stream, t);
   const double *cp = c->p.coe_Pd, *ch = c->p.coe_H;
   k_chem_mixed<<<grid_for(nH, kBlock), kBlock, 0, c->stream>>>(a, nH, cp[0], cp[2], cp[3], ch[0], ch[1], ch[2], ch[3],
                                                                c->d_occ, d_full, d_send);
