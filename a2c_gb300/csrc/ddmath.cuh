@@ -304,11 +304,96 @@ A2C_HD double fexp_mid(double x) {
   return from_words(hi_word(v) + (int)((unsigned)(ni >> 6) << 20), lo_word(v));
 }
 
+// The same values again with three FP64 operations, for 2^-8 <= |x| < 708
+// (else fexp_mid): n and the reduced argument in integers, and the four
+// inner steps of the polynomial, whose results keep to one binade each, as
+// fixed-point sums rounded like the FMAs they stand for.  About 210 integer
+// instructions for ten FP64 ones: the kernels of the plain form are bound by
+// the FP64 pipe (see mul_int).
+//
+// r = |x| - n ln2/64: the head of ln2/64 is a multiple of 2^-59 and |x| of
+// 2^-60, so r before the tail is an exact 64-bit integer in 2^-60; less n
+// times the tail, in 2^-114, rounded to 53 bits.  |r| >= 2^-20 is asked for
+// (one in 6,000 arguments is nearer a multiple of ln2/64).
+#if defined(__CUDACC__)
+#define A2C_CALL static __host__ __device__ __noinline__
+#else
+#define A2C_CALL inline
+#endif
+struct FixedStep {  // c + r * f, rounded: c and the result in units of 2^u
+  // f = fl 2^(ef-63) with fl left-justified; ml: |r| left-justified, with d
+  // the shift that brings the product's head into units of 2^u
+  static A2C_HD unsigned long long go(unsigned long long c, unsigned long long fl, unsigned long long ml, int d,
+                                      bool neg) {
+    const unsigned __int128 p = (unsigned __int128)ml * fl;
+    const unsigned long long t = (unsigned long long)(p >> 64);
+    unsigned long long q = t >> d, f = (t << (64 - d)) | ((unsigned long long)p != 0 ? 1ull : 0ull);
+    if (neg) {  // minus (q.f)
+      f = 0ull - f;
+      q = c - q - (f != 0 ? 1ull : 0ull);
+    } else {
+      q = c + q;
+    }
+    return q + (f > 0x8000000000000000ull || (f == 0x8000000000000000ull && (q & 1)) ? 1ull : 0ull);
+  }
+};
+A2C_CALL double fexp_fixed(double x) {
+  const unsigned hx = (unsigned)hi_word(x), ah = hx & 0x7fffffffu, lx = (unsigned)lo_word(x);
+  if (ah - 0x3f700000u >= 0x40862000u - 0x3f700000u) return fexp_mid(x);
+  const bool sx = hx >> 31;
+  // n = rint(|x| * 64/ln2)
+  const double p = mul_int(from_words((int)ah, (int)lx), 92.33248261689366);
+  const unsigned hp = (unsigned)hi_word(p), lp = (unsigned)lo_word(p);
+  const unsigned s = 1043u - (hp >> 20);  // 4 to 22: the unit's place in the high word
+  const unsigned mp = (hp & 0xfffffu) | 0x100000u;
+  const unsigned fr = mp << (32u - s);
+  unsigned n = mp >> s;
+  n += fr > 0x80000000u || (fr == 0x80000000u && (lp != 0 || (n & 1u))) ? 1u : 0u;
+  // r in 2^-60, then in 2^-114
+  const unsigned long long m = ((unsigned long long)((ah & 0xfffffu) | 0x100000u) << 32) | lx;
+  const long long r0 = (long long)((m << ((ah >> 20) - 1015u)) - (unsigned long long)n * 12486629536330718ull);
+  const __int128 v = ((__int128)r0 << 54) - (__int128)((unsigned __int128)n * 7525737178955839ull);
+  const bool neg = v < 0;
+  const unsigned __int128 w = neg ? -(unsigned __int128)v : (unsigned __int128)v;
+  const unsigned long long wh = (unsigned long long)(w >> 64);
+  if (wh < (1ull << 30)) return fexp_mid(x);
+#if defined(__CUDA_ARCH__)
+  const int lz = __clzll((long long)wh);
+#else
+  const int lz = __builtin_clzll(wh);
+#endif
+  const unsigned __int128 nv = w << lz;
+  const unsigned long long nh = (unsigned long long)(nv >> 64) | ((unsigned long long)nv != 0 ? 1ull : 0ull);
+  const unsigned long long mr = (nh + 0x3ff + ((nh >> 11) & 1)) >> 11;  // |r| = mr 2^(-39 - lz)
+  if (mr == 0) return fexp_mid(x);                                      // rounded up to a power of two and wrapped
+  const unsigned long long ml = mr << 11;
+  const bool sr = neg != sx;
+  // 1/120 + r/720, 1/24 + r (.), 1/6 + r (.), 1/2 + r (.)
+  unsigned long long c = FixedStep::go(4803839602528529ull, 6405119470038039ull << 11, ml, lz, sr);
+  c = FixedStep::go(6004799503160661ull, c << 11, ml, lz - 1, sr);
+  c = FixedStep::go(6004799503160661ull, c << 11, ml, lz - 1, sr);
+  c = FixedStep::go(sr ? 1ull << 53 : 1ull << 52, c << 11, ml, sr ? lz - 2 : lz - 1, sr);
+  const unsigned long long hb = c + ((sr ? 1020ull : 1021ull) << 52);
+  const double half = from_words((int)(hb >> 32), (int)(unsigned)hb);
+  const unsigned long long rb = mr + ((unsigned long long)(1035 - lz) << 52);
+  const double r = from_words((int)((unsigned)(rb >> 32) | (sr ? 0x80000000u : 0u)), (int)(unsigned)rb);
+  const double q = fma(mul_int(r, r), half, r);
+  const int ns = sx ? -(int)n : (int)n, j = ns & 63;
+#if defined(__CUDA_ARCH__)
+  const double2 e = *reinterpret_cast<const double2 *>(kExp2TabDev[j]);
+  const double th = e.x, tl = e.y;
+#else
+  const double th = kExp2TabHost[j][0], tl = kExp2TabHost[j][1];
+#endif
+  const double y = th + fma(th, q, tl);
+  return from_words(hi_word(y) + (int)((unsigned)(ns >> 6) << 20), lo_word(y));
+}
+
 // Results below 2^-1021 are flushed to zero (no argument of the potential
 // comes near), above 709.78 overflow to +inf; NaN propagates.
 A2C_HD double fexp(double x) {
 #if defined(__CUDA_ARCH__)
-  if ((hi_word(x) & 0x7fffffff) < 0x40862000) return fexp_mid(x);  // |x| < 708
+  if ((hi_word(x) & 0x7fffffff) < 0x40862000) return fexp_fixed(x);  // |x| < 708
 #endif
   if (!(x > -708.0)) return (x != x) ? x : 0.0;
   if (x > 709.78) return HUGE_VAL;
@@ -329,6 +414,11 @@ A2C_HD double fexp(double x) {
   const double th = kExp2TabHost[j][0], tl = kExp2TabHost[j][1];
 #endif
   return ldexp(th + fma(th, p, tl), k);
+}
+
+// fexp's values by fexp_mid wherever that serves
+A2C_HD double fexp_soon(double x) {
+  return (hi_word(x) & 0x7fffffff) < 0x40862000 ? fexp_mid(x) : fexp(x);
 }
 
 // e^(a.hi + a.lo) = 2^k (v.hi + v.lo) with relative error below 2^-70, for

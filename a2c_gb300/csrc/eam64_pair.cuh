@@ -15,9 +15,14 @@
 //   * comparisons with the switch radii on the bits, by integer operations;
 //   * multiplications whose factors are known not to be zero on the integer
 //     pipes (ddmath.cuh mul_int).
-// Per point 221 FP64 instructions remain of about 330 (all pair types of a
-// bulk site, the additions included), at 83% of the pipe's two lanes, which
-// is what a chain of FMAs reaches: pass 2 at 262,144 sites 127 -> 106 ms.
+//   * the exponentials mostly on the integer pipes (ddmath.cuh fexp_fixed).
+// FP64 instructions per point, all pair types of a bulk site and the
+// additions included, and pass 2 at 262,144 sites: about 330 / 127 ms with
+// the first three, 221 / 106 ms with the fourth (the pipe at 83% of its two
+// lanes, what a chain of FMAs reaches), 170 / 92 ms with all, where the
+// pipe, the integer pipes and the latency of both hold each other up: fewer
+// FP64 instructions still (the points' products by mul_int: 161) take
+// longer (99 ms).
 // The fast forms hold for kPairMin <= x < kPairMax (in_pair_range); callers
 // take eam64.cuh's functions elsewhere.
 #pragma once
@@ -82,13 +87,23 @@ A2C_EAM bool exact_for(double a) {
 // a / d.b for any a
 A2C_EAM double divide(double a, const Divisor &d) { return exact_for(a) ? quotient(a, d) : a / d.b; }
 
+// e^x: FIXED, the form with three FP64 operations and a long chain of
+// integer ones, for kernels whose warps wait for the FP64 pipe; else the one
+// with 13, which is done sooner where a scheduler has one warp to run (512
+// sites, pass 2: 0.51 against 0.55 ms).
+template <bool FIXED>
+A2C_EAM double exp_of(double x) {
+  return FIXED ? dd::fexp(x) : dd::fexp_soon(x);
+}
+
 // f_Pd as a function of r = x / 5 (potential.cpp:64-98).  Multiplications
 // by mul_int where no factor can be zero: below the switch radius r <= 1,
 // the quadratics have no real root, and r meets 0.53 and 0.136 only.
+template <bool FIXED>
 A2C_EAM double f_Pd_at(double r) {
   using dd::mul_int;
   const double x1 = mul_int(r, 5.0);
-  if (above(x1, 5.0)) return 0.001510569378297 * dd::fexp(-0.077976566126292 / 0.001510569378297 * (x1 - 5.0));
+  if (above(x1, 5.0)) return 0.001510569378297 * exp_of<FIXED>(-0.077976566126292 / 0.001510569378297 * (x1 - 5.0));
   double ra = mul_int(r, mul_int(r - 2.7267629107325706, r) + 1.8716766113599643);
   ra = mul_int(ra, mul_int(r - 2.50290548851635, r) + 1.668549182690922);
   ra = mul_int(ra, mul_int(r - 2.0924467509943674, r) + 1.3150372774478005);
@@ -108,10 +123,11 @@ A2C_EAM double second_fifth(double x, double r) {
 // phi_Pd with r = x / 5 and f = f_Pd(x1) (potential.cpp:126-155).  Below
 // the switch radius r <= 1.01; the factor r - 0.424 can be zero, and then
 // so is the product from there on.
+template <bool FIXED>
 A2C_EAM double phi_Pd_at(double r, double f) {
   using dd::mul_int;
   const double x1 = mul_int(r, 5.0);
-  if (above(x1, 5.05)) return -0.016958780164980 * dd::fexp(0.089019679316328 / -0.016958780164980 * (x1 - 5.05));
+  if (above(x1, 5.05)) return -0.016958780164980 * exp_of<FIXED>(0.089019679316328 / -0.016958780164980 * (x1 - 5.05));
   double y = mul_int(r - 1.0699996145674568, -79415.24035137112);
   y = mul_int(r - 1.06015072612581, y);
   y = y * (r - 0.42433991011376526);
@@ -123,20 +139,23 @@ A2C_EAM double phi_Pd_at(double r, double f) {
   y = mul_int(r * (r - 0.2635598721249787) + 0.033551116514910245, y);
   return y + (2 * 0.251546) * f;
 }
-A2C_EAM double f_Pd_pos(double x) { return f_Pd_at(div5(x)); }
+template <bool FIXED>
+A2C_EAM double f_Pd_pos(double x) { return f_Pd_at<FIXED>(div5(x)); }
+template <bool FIXED>
 A2C_EAM double f_H_pos(double x) {
-  if (above(x, 5.35)) return 0.009986990526578 * dd::fexp(-0.013075667086408 / 0.009986990526578 * (x - 5.35));
-  return dd::mul_int(dd::fexp(dd::mul_int(x, -1.30927)), 11.0025);
+  if (above(x, 5.35)) return 0.009986990526578 * exp_of<FIXED>(-0.013075667086408 / 0.009986990526578 * (x - 5.35));
+  return dd::mul_int(exp_of<FIXED>(dd::mul_int(x, -1.30927)), 11.0025);
 }
 // phi_PdH (potential.cpp:162-177) and phi_H (185-200): one form, constants
 // by pair type
+template <bool FIXED>
 A2C_EAM double morse_pos(bool pdh, double x) {
   if (above(x, 5.35))
-    return pdh ? -3.353001113951400e-04 * dd::fexp(7.147062196813336e-04 / -3.353001113951400e-04 * (x - 5.35))
-               : -0.003702722457147 * dd::fexp(0.005465945471933 / -0.003702722457147 * (x - 5.35));
+    return pdh ? -3.353001113951400e-04 * exp_of<FIXED>(7.147062196813336e-04 / -3.353001113951400e-04 * (x - 5.35))
+               : -0.003702722457147 * exp_of<FIXED>(0.005465945471933 / -0.003702722457147 * (x - 5.35));
   const double D = pdh ? 0.2494540 : 0.0661496, alpha = pdh ? 4.82613 : 3.67263, beta = pdh ? 2.13158 : 1.47797;
   const double t = x - (pdh ? 1.50964 : 2.51980);
-  return D * (dd::mul_int(dd::fexp(-alpha * t), beta) - dd::mul_int(dd::fexp(-beta * t), alpha));
+  return D * (dd::mul_int(exp_of<FIXED>(-alpha * t), beta) - dd::mul_int(exp_of<FIXED>(-beta * t), alpha));
 }
 
 // What one quadrature point of a pair at distance s takes from the pair
@@ -147,17 +166,29 @@ A2C_EAM double morse_pos(bool pdh, double x) {
 struct PairPoint {
   double da, db, phi, dphi;
 };
+#if defined(__CUDACC__)
+#define A2C_COLD static __host__ __device__ __noinline__
+#else
+#define A2C_COLD inline
+#endif
+// outside the fast forms' range: the plain functions, out of line
+A2C_COLD PairPoint pair_point_plain(bool iPd, bool jPd, double s, double e) {
+  PairPoint p;
+  const double fP = (iPd || jPd) ? f_Pd_d(s, e) : 0.0, fH = (iPd && jPd) ? 0.0 : f_H_d(s, e);
+  p.da = jPd ? fP : fH;
+  p.db = iPd ? fP : fH;
+  p.phi = (iPd && jPd) ? phi_Pd(s) : (iPd || jPd) ? phi_PdH(s) : phi_H(s);
+  p.dphi = (iPd && jPd) ? phi_Pd_d(s, e) : (iPd || jPd) ? phi_PdH_d(s, e) : phi_H_d(s, e);
+  return p;
+}
+A2C_COLD double density_plain(bool jPd, double s) { return jPd ? f_Pd(s) : f_H(s); }
+#undef A2C_COLD
+
+template <bool FIXED = true>
 A2C_EAM PairPoint pair_point(bool iPd, bool jPd, double s, double e, const Divisor &h) {
   const double xp = s + e, xm = s - e;
   PairPoint p;
-  if (!in_pair_range(xp) || !in_pair_range(xm)) {
-    const double fP = (iPd || jPd) ? f_Pd_d(s, e) : 0.0, fH = (iPd && jPd) ? 0.0 : f_H_d(s, e);
-    p.da = jPd ? fP : fH;
-    p.db = iPd ? fP : fH;
-    p.phi = (iPd && jPd) ? phi_Pd(s) : (iPd || jPd) ? phi_PdH(s) : phi_H(s);
-    p.dphi = (iPd && jPd) ? phi_Pd_d(s, e) : (iPd || jPd) ? phi_PdH_d(s, e) : phi_H_d(s, e);
-    return p;
-  }
+  if (!in_pair_range(xp) || !in_pair_range(xm)) return pair_point_plain(iPd, jPd, s, e);
   // s, then s + e and s - e in one rolled loop: with the functions written
   // out for each the instruction caches did not hold the kernel (pass 2 at
   // 262,144 sites 112 ms, rolled 106)
@@ -177,18 +208,18 @@ A2C_EAM PairPoint pair_point(bool iPd, bool jPd, double s, double e, const Divis
 #pragma unroll 1
 #endif
       for (bool first = true;; first = false) {
-        f = f_Pd_at(at);
+        f = f_Pd_at<FIXED>(at);
         if (first) fP = f;
         if (at == r2) break;
         at = r2;
       }
-      ph = phi_Pd_at(r, f);
+      ph = phi_Pd_at<FIXED>(r, f);
     } else {
       if (v > 0) {
-        if (pdh) fP = f_Pd_at(div5(x));
-        fH = f_H_pos(x);
+        if (pdh) fP = f_Pd_at<FIXED>(div5(x));
+        fH = f_H_pos<FIXED>(x);
       }
-      ph = morse_pos(pdh, x);
+      ph = morse_pos<FIXED>(pdh, x);
     }
     if (v == 0) {
       p.phi = ph;
@@ -208,9 +239,10 @@ A2C_EAM PairPoint pair_point(bool iPd, bool jPd, double s, double e, const Divis
   return p;
 }
 // the density a neighbor at distance s adds at one point
+template <bool FIXED = true>
 A2C_EAM double density_point(bool jPd, double s) {
-  if (!in_pair_range(s)) return jPd ? f_Pd(s) : f_H(s);
-  return jPd ? f_Pd_pos(s) : f_H_pos(s);
+  if (!in_pair_range(s)) return density_plain(jPd, s);
+  return jPd ? f_Pd_pos<FIXED>(s) : f_H_pos<FIXED>(s);
 }
 
 }  // namespace eam64

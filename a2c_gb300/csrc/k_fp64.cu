@@ -16,8 +16,9 @@
 // a 512-site system 16 warps, each with 960 points in a row.  S trades the
 // two ends (rho_sites_per_warp, grad_sites_per_warp).  With the pair
 // functions' fewer operations (eam64_pair.cuh) an evaluation takes, one
-// thread per site -> now: 15.3 -> 0.69 ms at 512 sites, 23.0 -> 7.3 ms at
-// 10,296, 210.6 -> 124.2 ms at 262,144.
+// thread per site -> now: 15.3 -> 0.70 ms at 512 sites, 23.0 -> 5.5 ms at
+// 10,296, 210.6 -> 108.5 ms at 262,144.  Five blocks of pass 2 per SM: 10,296
+// sites then fit at once (5.6 -> 4.6 ms).
 //
 // Geometry: for quadrature point k = 2m (+sqrt(3)) or 2m+1 (-sqrt(3)) only
 // coordinate m of R^6 is non-zero, so r_k differs from the pair's base
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_density64(SiteArgs a) {
           const int m = (k < 6 ? k : k - 6) >> 1, sgn = k & 1;
           const double u = sh.uj[q];
           const double rm = k < 6 ? sh.qp[q / NB][2 * m + sgn] - sh.qj[m][q] : sh.D[m][q] - (sgn ? -u : u);
-          const double f = eam64::density_point(jPd, radius(m, rm, sh.D2[0][q], sh.D2[1][q], sh.D2[2][q]));
+          const double f = eam64::density_point<(S > 2)>(jPd, radius(m, rm, sh.D2[0][q], sh.D2[1][q], sh.D2[2][q]));
           sh.term[q * kRhoRow + k] = (jPd ? f : sh.xj[q] * f) * W;
         }
         __syncwarp();
@@ -283,7 +284,7 @@ struct GradShared {
 };
 
 template <int S, bool LIST>
-__global__ void __launch_bounds__(32 * kWarps) k_gradient64(SiteArgs a) {
+__global__ void __launch_bounds__(32 * kWarps, 5) k_gradient64(SiteArgs a) {
   constexpr int NB = kGradPairs / S;
   extern __shared__ double2 smem64[];
   GradShared &sh = reinterpret_cast<GradShared *>(smem64)[threadIdx.x / 32];
@@ -354,7 +355,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_gradient64(SiteArgs a) {
           const double u = sh.uj[q];
           const double rm = k < 6 ? sh.qp[q / NB][2 * m + sgn] - sh.qj[m][q] : sh.D[m][q] - (sgn ? -u : u);
           const double s = radius(m, rm, sh.D2[0][q], sh.D2[1][q], sh.D2[2][q]);
-          const eam64::PairPoint f = eam64::pair_point(pdmask >> q & 1u, jPd, s, eps, h);
+          const eam64::PairPoint f = eam64::pair_point<(S > 1)>(pdmask >> q & 1u, jPd, s, eps, h);
           const double av = sh.AV[q], A[3] = {sh.A1[q], sh.A2[q], sh.A3[q]};
           double c[3] = {mul(A[0], f.da), mul(A[1], f.db), mul(A[2], f.dphi)};
           if (eam64::in_pair_range(s)) {
@@ -367,28 +368,14 @@ __global__ void __launch_bounds__(32 * kWarps) k_gradient64(SiteArgs a) {
           }
           const double r[3] = {m == 0 ? rm : sh.D[0][q], m == 1 ? rm : sh.D[1][q], m == 2 ? rm : sh.D[2][q]};
           const double xi0 = sgn ? -kSqrt3 : kSqrt3;
-          const bool fits = dd::mul_int_ok(c[0]) && dd::mul_int_ok(c[1]) && dd::mul_int_ok(c[2]) &&
-                            dd::mul_int_ok(r[0]) && dd::mul_int_ok(r[1]) && dd::mul_int_ok(r[2]);
 #pragma unroll
           for (int i = 0; i < 3; ++i) {
             double *o = sh.pt + 4 * i * kGradRow + p;
-            double x, y, z;
-            if (fits) {
-              x = dd::mul_int(c[i], r[0]);
-              y = dd::mul_int(c[i], r[1]);
-              z = dd::mul_int(c[i], r[2]);
-            } else {
-              x = c[i] * r[0];
-              y = c[i] * r[1];
-              z = c[i] * r[2];
-            }
+            const double x = c[i] * r[0], y = c[i] * r[1], z = c[i] * r[2];
             o[0] = x;
             o[kGradRow] = y;
             o[2 * kGradRow] = z;
-            if (k < 6) {
-              const double v = m == 0 ? x : m == 1 ? y : z;
-              o[3 * kGradRow] = fits ? dd::mul_int(v, xi0) : v * xi0;
-            }
+            if (k < 6) o[3 * kGradRow] = (m == 0 ? x : m == 1 ? y : z) * xi0;
           }
           sh.pt[(4 * (k % 3) + 3) * kGradRow + 12 * q + 6 + k / 3] = mul(av, f.phi);
         }
@@ -477,8 +464,8 @@ __global__ void __launch_bounds__(kBlock) k_chem64(SiteArgs a, const double coeP
       int comp;
       const double sk = point(g, k, r, comp, xi0);
       const bool fast = eam64::in_pair_range(sk);
-      sum = sum + WF * (fast ? eam64::f_H_pos(sk) : eam64::f_H(sk));
-      sum = sum + W * (fast ? eam64::morse_pos(true, sk) : eam64::phi_PdH(sk));
+      sum = sum + WF * (fast ? eam64::f_H_pos<true>(sk) : eam64::f_H(sk));
+      sum = sum + W * (fast ? eam64::morse_pos<true>(true, sk) : eam64::phi_PdH(sk));
     }
     const int64_t bj = a.off[j], mj = bj + a.npd[j], ej = a.off[j + 1];
     sum = sum + ((T * coePd0) * coePd2) * (double)(mj - bj);
@@ -501,8 +488,8 @@ __global__ void __launch_bounds__(kBlock) k_chem64(SiteArgs a, const double coeP
       int comp;
       const double sk = point(g, k, r, comp, xi0);
       const bool fast = eam64::in_pair_range(sk);
-      sum = sum + xWF * (fast ? eam64::f_H_pos(sk) : eam64::f_H(sk));
-      sum = sum + xW * (fast ? eam64::morse_pos(false, sk) : eam64::phi_H(sk));
+      sum = sum + xWF * (fast ? eam64::f_H_pos<true>(sk) : eam64::f_H(sk));
+      sum = sum + xW * (fast ? eam64::morse_pos<true>(false, sk) : eam64::phi_H(sk));
     }
     const int64_t bj = a.off[j], mj = bj + a.npd[j], ej = a.off[j + 1];
     sum = sum + (((xj * T) * coeH0) * coeH2) * (double)(mj - bj);
@@ -561,14 +548,19 @@ SiteArgs site_args(a2c_gpp_ctx *c, const double *dX) {
 // Sites per warp.  Few sites: a warp per site or two, all lanes on its
 // points, though one to eight lanes then do its additions; many: the
 // additions of 8 (32 in pass 1) sites fill the lanes.  Measured on a GB300
-// (152 SMs) before multiplications moved to the integer pipes, pass 1 with 2
-// / 8 / 32 sites per warp: 512 sites 0.18 / 0.52 / 1.84 ms, 10,296 1.35 /
-// 1.38 / 1.84, 64,000 7.9 / 6.4 / 6.5, 262,144 31.9 / 24.5 / 22.5 ms; pass 2
-// with 1 / 4 / 8: 512 sites 0.48 / 1.47 / 2.8 ms, 2,744 2.06 / 2.50 / 3.21,
-// 10,296 6.9 / 6.3 / 7.3, 32,768 21.9 / 17.3 / 17.1, 262,144 174 / 133 / 127
-// ms.  Results do not depend on it.
-int rho_sites_per_warp(int64_t n, int sms) { return n < 64 * (int64_t)sms ? 2 : n < 512 * (int64_t)sms ? 8 : 32; }
-int grad_sites_per_warp(int64_t n, int sms) { return n < 32 * (int64_t)sms ? 1 : n < 128 * (int64_t)sms ? 4 : 8; }
+// (152 SMs), ms for the choices named:
+//   pass 1, 2 / 8 / 32 sites: 512 sites 0.18 / 0.54 / 1.9, 5,832 0.65 / 0.71
+//     / 1.9, 8,000 0.92 / 0.71 / 1.9, 32,768 3.5 / 2.33 / 2.42, 64,000 6.7 /
+//     4.55 / 4.38, 110,592 11.5 / 7.3 / 6.6;
+//   pass 2, 1 / 2 / 4 / 8 sites: 512 sites 0.51 / 0.98 / 1.7 / 3.3, 1,728
+//     1.13 / 1.28 / 1.7 / 3.3, 2,744 1.9 / 1.7 / 2.2 / 3.7, 5,832 3.7 / 2.7 /
+//     3.0 / 4.3, 8,000 5.5 / 4.1 / 3.8 / 4.5, 13,824 8.5 / 6.9 / 6.9 / 6.0,
+//     110,592 67 / 49 / 42 / 40.
+// Results do not depend on it.
+int rho_sites_per_warp(int64_t n, int sms) { return n < 42 * (int64_t)sms ? 2 : n < 330 * (int64_t)sms ? 8 : 32; }
+int grad_sites_per_warp(int64_t n, int sms) {
+  return n < 16 * (int64_t)sms ? 1 : n < 46 * (int64_t)sms ? 2 : n < 80 * (int64_t)sms ? 4 : 8;
+}
 
 // Blocks resident on the device at once for a kernel with its shared
 // memory, asked once per kernel and device under a lock.
@@ -614,6 +606,7 @@ template <bool LIST>
 a2c_status gradient64(a2c_gpp_ctx *c, const SiteArgs &a, int64_t n) {
   switch (grad_sites_per_warp(n, device_sms(c->device))) {
     case 1: return launch_warps<GradShared>(k_gradient64<1, LIST>, 1, a, n, LIST, c);
+    case 2: return launch_warps<GradShared>(k_gradient64<2, LIST>, 2, a, n, LIST, c);
     case 4: return launch_warps<GradShared>(k_gradient64<4, LIST>, 4, a, n, LIST, c);
     default: return launch_warps<GradShared>(k_gradient64<8, LIST>, 8, a, n, LIST, c);
   }

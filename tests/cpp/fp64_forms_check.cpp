@@ -48,6 +48,10 @@ int main(int argc, char **argv) {
     } else if (form == "fexp") {
       const double x = i % 2 ? (U(g) - 0.5) * 1415.9 : (U(g) - 0.5) * std::ldexp(80.0, -(int)(g() % 70));
       tally(true, dd::fexp_mid(x), dd::fexp(x));
+      // near multiples of ln2/64, where the reduced argument is small
+      const double y = (double)((long)(g() % 80000) - 40000) * 0.010830424696249145 + (U(g) - 0.5) * std::ldexp(1.0, -(int)(g() % 30));
+      tally(true, dd::fexp_fixed(x), dd::fexp(x));
+      if (std::fabs(y) < 708) tally(true, dd::fexp_fixed(y), dd::fexp(y));
     } else if (form == "mul") {  // both significands random, short, or all ones at the end
       auto value = [&](long k) {
         unsigned long long b = (g() >> 12) | (0x3ffull - 500 + g() % 1000) << 52 | g() << 63;
