@@ -160,6 +160,7 @@ int current_device_sms();
 struct Tile {
   int tps = 0, rho_block = 0, grad_block = 0;
   bool wide = false, twin = false;  // a warp, or two lanes, for a site's tps lanes (effective_tile)
+  bool copies = false;              // pass 2 with eight copies of its tables (effective_tile)
   bool operator==(const Tile &o) const { return tps == o.tps && rho_block == o.rho_block && grad_block == o.grad_block; }
 };
 inline bool valid_tile(int tps, int rho_block, int grad_block) {

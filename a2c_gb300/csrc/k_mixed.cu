@@ -348,17 +348,46 @@ constexpr int kRhoTabN = 768;
 constexpr int kRhoCopies = 8;
 constexpr size_t kRhoSmem = sizeof(float4) * kRhoTabN * kRhoCopies;  // 98,304 B: two blocks per SM
 
-// Pass 2 reads two tables (f_Pd' and phi_Pd).  Interleaved copies cost it
-// occupancy (8 copies of both: one 256-thread block per SM; 4: two), and
-// pass 2 needs the resident warps more than conflict-free lookups: on a
-// GB300 at 262,144 sites pass 2 took 0.329 ms with one copy (four blocks
-// per SM), 0.375 ms with 4 copies and 0.530 ms with 8.  So one copy.
-#ifndef A2C_GRAD_COPIES
-#define A2C_GRAD_COPIES 1
-#endif
-constexpr int kGradCopies = A2C_GRAD_COPIES;
+// Pass 2 reads two tables, f_Pd' (Pd-Pd and H-Pd pairs) and phi_Pd (Pd-Pd
+// pairs, a fifth of the lookups).  One copy of both leaves the blocks any
+// size, but its lookups meet bank conflicts: 22.6 M of the 61 M wavefronts of
+// the load/store data pipe at 262,144 sites, which is 81% busy.  Eight copies
+// of f_Pd', as in pass 1, and two of phi_Pd under one block of 1024 threads
+// per SM leave 6.5 M (the pipe 61% busy, the issue slots 59%) and the L1 as
+// large as four blocks with one copy each: 289 us -> 264 with the fetched
+// items below.  Eight copies of both left 28 KB of L1 for the gathers:
+// 301 us.  f_Pd' ends at 5.8 A there, as f_Pd does in pass 1: its last
+// interval, where f_Pd' is below 1e-19 and the phi' that it is added to
+// above 1e-7, holds zeros (the same bits).
 constexpr int kGradTabN = kTabN;  // phi_Pd is -3e-4 eV at 5.8 A: every interval
-constexpr size_t kGradSmem = 2 * sizeof(float4) * kGradTabN * kGradCopies;
+template <int COPIES>
+constexpr int kForceTabN = COPIES == 1 ? kTabN : kRhoTabN;
+template <int COPIES>
+constexpr int kPhiCopies = COPIES == 1 ? 1 : 2;
+template <int COPIES>
+constexpr size_t grad_smem() {  // 30,720 B or 129,024 B
+  return sizeof(float4) * (COPIES * kForceTabN<COPIES> + kPhiCopies<COPIES> * kGradTabN);
+}
+// This block's tables: f_Pd' quadratics, then phi_Pd cubics, each interval
+// COPIES times; sF and sP point at this thread's copies.
+template <int COPIES>
+__device__ __forceinline__ void load_grad_tables(const float4 *tabPair, float4 *sTab, const float4 *&sF,
+                                                 const float4 *&sP) {
+  constexpr int kN = kForceTabN<COPIES>;
+  for (int i = threadIdx.x; i < kN * COPIES; i += blockDim.x)
+    sTab[i] = COPIES > 1 && i / COPIES == kN - 1 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f)
+                                                 : __ldg(&tabPair[2 * kTabN + i / COPIES]);
+  for (int i = threadIdx.x; i < kGradTabN * kPhiCopies<COPIES>; i += blockDim.x)
+    sTab[kN * COPIES + i] = __ldg(&tabPair[kTabN + i / kPhiCopies<COPIES>]);
+  __syncthreads();
+  sF = sTab + threadIdx.x % COPIES;
+  sP = sTab + kN * COPIES + threadIdx.x % kPhiCopies<COPIES>;
+}
+// The f_Pd' entry of interval i.
+template <int COPIES>
+__device__ __forceinline__ float4 force_entry(const float4 *sF, int i) {
+  return sF[COPIES * (COPIES == 1 ? i : min(i, kRhoTabN - 1))];
+}
 
 // The density terms of one neighbor: f_Pd from the table (COPIES copies,
 // this lane's from sF), or f_H.
@@ -487,7 +516,7 @@ __device__ __forceinline__ bool pair_inside(float3 D, float ui, float uj) {
 
 // TAIL = false: every point is inside the switch radius (pair_inside), so
 // the Morse terms skip the per-point branch selection.
-template <int TYPE, bool TAIL = true>  // 0 Pd-Pd, 1 Pd i / H j, 2 H i / Pd j, 3 H-H
+template <int TYPE, bool TAIL, int COPIES>  // 0 Pd-Pd, 1 Pd i / H j, 2 H i / Pd j, 3 H-H
 __device__ __forceinline__ void pair_terms(const ExpTerms &x, const float4 *sF, const float4 *sP, float Fa, float Fb,
                                            float3 D, float ui, float uj, PairAcc &p) {
   const float D2 = fmaf(D.x, D.x, fmaf(D.y, D.y, D.z * D.z));
@@ -508,8 +537,8 @@ __device__ __forceinline__ void pair_terms(const ExpTerms &x, const float4 *sF, 
       float g, phi;
       if (TYPE == 0) {
         float tt;
-        const int i = kGradCopies * tab_index<kGradTabN>(r, tt);
-        const float4 cf = sF[i], cp = sP[i];
+        const int i = tab_index<kGradTabN>(r, tt);
+        const float4 cf = force_entry<COPIES>(sF, i), cp = sP[kPhiCopies<COPIES> * i];
         // phi and h phi' share one Horner chain
         const float hp = fmaf(cp.w, tt, cp.z), hq = fmaf(hp, tt, cp.y);
         phi = fmaf(hq, tt, cp.x);
@@ -522,8 +551,8 @@ __device__ __forceinline__ void pair_terms(const ExpTerms &x, const float4 *sF, 
         g = fmaf(-(Fa + Fb), nfhd, dphi);
       } else {
         float tt;
-        const int i = kGradCopies * tab_index<kGradTabN>(r, tt);
-        const float fpd = dq(sF[i], tt) * (float)kTabInvH;
+        const int i = tab_index<kGradTabN>(r, tt);
+        const float fpd = dq(force_entry<COPIES>(sF, i), tt) * (float)kTabInvH;
         const float nfhd = fHd_neg(x, r);
         float dphi;
         if (TAIL) morse(x.pdh, r, phi, dphi);
@@ -702,13 +731,9 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_mixed(
   constexpr int kSitesPerBlock = BLOCK / TPS;
   const int64_t n = LIST ? (int64_t)*a.bv.count : a.N;
   if ((int64_t)blockIdx.x * kSitesPerBlock >= n) return;
-  extern __shared__ float4 sTab[];  // f_Pd' quadratics, then phi_Pd cubics, kGradCopies-way interleaved
-  for (int i = threadIdx.x; i < kGradTabN * kGradCopies; i += blockDim.x) {
-    sTab[i] = __ldg(&a.tabPair[2 * kTabN + i / kGradCopies]);
-    sTab[kGradTabN * kGradCopies + i] = __ldg(&a.tabPair[kTabN + i / kGradCopies]);
-  }
-  __syncthreads();
-  const float4 *sF = sTab + threadIdx.x % kGradCopies, *sP = sF + kGradTabN * kGradCopies;
+  extern __shared__ float4 sTab[];
+  const float4 *sF, *sP;
+  load_grad_tables<1>(a.tabPair, sTab, sF, sP);
   for (int64_t base = (int64_t)blockIdx.x * kSitesPerBlock; base < n;
        base += (int64_t)gridDim.x * kSitesPerBlock) {
   const int64_t k = base + threadIdx.x / TPS;
@@ -736,11 +761,11 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_mixed(
       const float uj = kSqrt6 * __int_as_float(pj.w);
       PairAcc p;
       if (iPd) {
-        pair_terms<0>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
+        pair_terms<0, true, 1>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
       } else if (pair_inside(D, ui, uj)) {
-        pair_terms<2, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
+        pair_terms<2, false, 1>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
       } else {
-        pair_terms<2, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
+        pair_terms<2, true, 1>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
       }
       add_pair(A, p, D, a.W, hw);
     });
@@ -750,11 +775,11 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_mixed(
       PairAcc p;
       const bool in = pair_inside(D, ui, uj);
       if (iPd) {
-        if (in) pair_terms<1, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
-        else pair_terms<1, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
+        if (in) pair_terms<1, false, 1>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
+        else pair_terms<1, true, 1>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
       } else {
-        if (in) pair_terms<3, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
-        else pair_terms<3, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
+        if (in) pair_terms<3, false, 1>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
+        else pair_terms<3, true, 1>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, p);
       }
       add_pair(A, p, D, a.W * xj, hw * xj);
     });
@@ -819,23 +844,78 @@ __device__ __forceinline__ void add_pairs(SiteAcc &A, const PairAcc &p, float3 D
   }
 }
 
-template <int V, int TPS, bool LIST, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(MixArgs a) {
-  constexpr int kSitesPerBlock = BLOCK / TPS;
-  const int64_t n = LIST ? (int64_t)*a.bv.count : a.N;
-  if ((int64_t)blockIdx.x * kSitesPerBlock >= n) return;
-  extern __shared__ float4 sTab[];  // f_Pd' quadratics, then phi_Pd cubics, kGradCopies-way interleaved
-  for (int i = threadIdx.x; i < kGradTabN * kGradCopies; i += blockDim.x) {
-    sTab[i] = __ldg(&a.tabPair[2 * kTabN + i / kGradCopies]);
-    sTab[kGradTabN * kGradCopies + i] = __ldg(&a.tabPair[kTabN + i / kGradCopies]);
+// How the sites reach the warps of the shape with table copies.  An item is
+// the sites of one warp.  The H sites come first, then the Pd sites (an H
+// site owns the pairs with all its Pd neighbors and takes about three times
+// a Pd site's time): every block gets the same number of items of either
+// kind, in rounds of neighboring items, and its warps fetch them one by one,
+// so that the last ones to run are short.  With the fixed rounds of the other
+// shapes the SMs' shares differed (idle 11% of the kernel at 262,144 sites,
+// 281 -> 264 us; 2,097,152: 2,303 -> 2,145); those shapes, whose blocks are
+// many or hold an item per warp, lost 1 to 3% by fetching.
+struct Items {
+  unsigned whole[2], share[2], count[2];  // items in whole rounds, per block in the last one, of this block
+  unsigned next;                          // the next item of this block
+};
+// The H and the Pd sites of a launch (a work list of many instances: all its
+// sites as one kind).
+template <bool LIST>
+__device__ __forceinline__ void site_kinds(const MixArgs &a, unsigned &nH, unsigned &nPd) {
+  const unsigned n = LIST ? (unsigned)*a.bv.count : (unsigned)a.N;
+  nPd = LIST ? (a.bv.list ? 0u : min((unsigned)a.bv.geo[0].nPd, n)) : (unsigned)a.nPd;
+  nH = n - nPd;
+}
+// Called by every thread; false if the block has nothing to do.
+template <int WARPS, int UNIT>
+__device__ __forceinline__ bool share_items(Items &q, unsigned nH, unsigned nPd) {
+  if (threadIdx.x < 2) {
+    const unsigned n = threadIdx.x ? nPd : nH, items = (n + UNIT - 1) / UNIT;
+    const unsigned full = items / (gridDim.x * WARPS), left = items - full * gridDim.x * WARPS;
+    const unsigned share = (left + gridDim.x - 1) / gridDim.x, before = blockIdx.x * share;
+    q.whole[threadIdx.x] = full * WARPS;
+    q.share[threadIdx.x] = share;
+    q.count[threadIdx.x] = full * WARPS + (before < left ? min(share, left - before) : 0u);
+    if (threadIdx.x == 0) q.next = 0u;
   }
   __syncthreads();
-  const float4 *sF = sTab + threadIdx.x % kGradCopies, *sP = sF + kGradTabN * kGradCopies;
-  for (int64_t base = (int64_t)blockIdx.x * kSitesPerBlock; base < n;
+  return q.count[0] + q.count[1] > 0u;
+}
+// The first site of the warp's next item and the end of its kind.
+template <int WARPS, int UNIT>
+__device__ __forceinline__ bool next_item(Items &q, unsigned nH, unsigned nPd, int64_t &first, int64_t &end) {
+  unsigned u = 0;
+  if (threadIdx.x % 32 == 0) u = atomicAdd(&q.next, 1u);
+  u = __shfl_sync(0xffffffffu, u, 0);
+  const int kind = u >= q.count[0];
+  if (kind) u -= q.count[0];
+  if (u >= q.count[kind]) return false;
+  const unsigned whole = q.whole[kind];
+  const unsigned item = u < whole ? u / WARPS * (gridDim.x * WARPS) + blockIdx.x * WARPS + u % WARPS
+                                  : whole * gridDim.x + blockIdx.x * q.share[kind] + (u - whole);
+  first = (int64_t)item * UNIT + (kind ? 0 : nPd);
+  end = kind ? nPd : nPd + nH;
+  return true;
+}
+
+template <int V, int TPS, bool LIST, int BLOCK, int COPIES>
+__global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(MixArgs a) {
+  constexpr int kUnit = 32 / TPS, kWarps = BLOCK / 32, kSitesPerBlock = BLOCK / TPS;
+  constexpr bool kFetch = COPIES > 1;
+  __shared__ Items items;
+  unsigned nH, nPd;
+  site_kinds<LIST>(a, nH, nPd);
+  if (kFetch ? !share_items<kWarps, kUnit>(items, nH, nPd) : (int64_t)blockIdx.x * kSitesPerBlock >= nH + nPd) return;
+  extern __shared__ float4 sTab[];
+  const float4 *sF, *sP;
+  load_grad_tables<COPIES>(a.tabPair, sTab, sF, sP);
+  int64_t k = 0, end = nH + nPd;
+  for (int64_t base = (int64_t)blockIdx.x * kSitesPerBlock;
+       kFetch ? next_item<kWarps, kUnit>(items, nH, nPd, k, end) : base < end;
        base += (int64_t)gridDim.x * kSitesPerBlock) {
-  const int64_t k = base + threadIdx.x / TPS;
+  if (kFetch) k += threadIdx.x % 32 / TPS;
+  else k = base + threadIdx.x / TPS;
   const int lane = (int)(threadIdx.x % TPS);
-  const bool live = k < n;
+  const bool live = k < end;
   SiteRef<LIST> R{};
   if (live) R = site_ref<LIST>(a, k);
   const int64_t s = R.s;
@@ -861,11 +941,11 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(M
         const float uj = kSqrt6 * __int_as_float(pj.w);
         PairAcc q;
         if (iPd) {
-          pair_terms<0>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          pair_terms<0, true, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
         } else if (pair_inside(D, ui, uj)) {
-          pair_terms<2, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          pair_terms<2, false, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
         } else {
-          pair_terms<2, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          pair_terms<2, true, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
         }
         add_pair(A, q, D, a.W, w);
         send_share(a, slot, q, D, w);
@@ -875,8 +955,8 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(M
         const float3 D = pair_vec(R.sc, pi, pj);
         const float uj = kSqrt6 * __int_as_float(pj.w);
         PairAcc q;
-        if (pair_inside(D, ui, uj)) pair_terms<3, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
-        else pair_terms<3, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+        if (pair_inside(D, ui, uj)) pair_terms<3, false, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+        else pair_terms<3, true, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
         add_pair(A, q, D, a.W * xj, w * xj);
         send_share(a, slot, q, D, w);
       });
@@ -890,11 +970,11 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(M
           const uint32_t slot = __ldg(&a.rev[t]);
           const float uj = kSqrt6 * __int_as_float(pj.w);
           if (iPd) {
-            pair_terms<0>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+            pair_terms<0, true, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
           } else if (pair_inside(D, ui, uj)) {
-            pair_terms<2, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+            pair_terms<2, false, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
           } else {
-            pair_terms<2, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+            pair_terms<2, true, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
           }
           send_share(a, slot, q, D, w);
         }
@@ -907,8 +987,8 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(M
         if (valid) {
           const uint32_t slot = __ldg(&a.rev[t]);
           const float uj = kSqrt6 * __int_as_float(pj.w);
-          if (pair_inside(D, ui, uj)) pair_terms<3, false>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
-          else pair_terms<3, true>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          if (pair_inside(D, ui, uj)) pair_terms<3, false, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
+          else pair_terms<3, true, COPIES>(a.ex, sF, sP, ffi.x, Fb, D, ui, uj, q);
           send_share(a, slot, q, D, w);
         }
         add_pairs<V, TPS, true>(A, q, D, a.W, w, xj, group, lane, first, p);
@@ -1252,10 +1332,11 @@ void launch_rho(const MixArgs &a, cudaStream_t st) {
   constexpr size_t smem = TPS == 32 ? kRhoSmem / kRhoCopies : kRhoSmem;
   k_rho_mixed<V, TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, smem)), B, smem, st>>>(a);
 }
-template <int V, int TPS, bool LIST, int B>
+template <int V, int TPS, bool LIST, int B, int COPIES = 1>
 void launch_once(const MixArgs &a, cudaStream_t st) {
-  const void *fn = (const void *)k_grad_once<V, TPS, LIST, B>;
-  k_grad_once<V, TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, kGradSmem)), B, kGradSmem, st>>>(a);
+  const void *fn = (const void *)k_grad_once<V, TPS, LIST, B, COPIES>;
+  constexpr size_t smem = grad_smem<COPIES>();
+  k_grad_once<V, TPS, LIST, B, COPIES><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, smem)), B, smem, st>>>(a);
 }
 template <int TPS, bool LIST, int B>
 void launch_grad(const MixArgs &a, cudaStream_t st, bool once) {
@@ -1263,7 +1344,7 @@ void launch_grad(const MixArgs &a, cudaStream_t st, bool once) {
     launch_once<TPS, TPS, LIST, B>(a, st);
   } else {
     const void *fn = (const void *)k_grad_mixed<TPS, LIST, B>;
-    k_grad_mixed<TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, kGradSmem)), B, kGradSmem, st>>>(a);
+    k_grad_mixed<TPS, LIST, B><<<persistent_grid(a.N, B / TPS, grid_cap(fn, B, grad_smem<1>())), B, grad_smem<1>(), st>>>(a);
   }
 }
 
@@ -1296,9 +1377,14 @@ void launch_pass2(const MixArgs &a, cudaStream_t st, bool once, const Tile &t) {
   }
   if constexpr (V == 1) {
     if (once && t.twin) {
-      launch_once<1, 2, LIST, 256>(a, st);
+      if (t.copies) launch_once<1, 2, LIST, 1024, 8>(a, st);
+      else launch_once<1, 2, LIST, 256>(a, st);
       return;
     }
+  }
+  if (once && t.copies) {
+    launch_once<V, V, LIST, 1024, 8>(a, st);
+    return;
   }
   switch (t.grad_block) {
     case 128: launch_grad<V, LIST, 128>(a, st, once); break;
@@ -1514,6 +1600,13 @@ Tile effective_tile(const Tile &t, int64_t n_sites, int sms) {
   }
   e.rho_block = t.rho_block ? t.rho_block : e.tps > 1 ? 512 : kBlock;
   e.grad_block = t.grad_block ? t.grad_block : n_sites < 256 * (int64_t)sms ? 128 : kBlock;
+  // Pass 2's shape of 256 threads (kBlock, or nothing chosen) has eight
+  // copies of f_Pd' under one block of 1024 threads per SM where its warps
+  // come near 32 per SM (pass 2 without / with them, 2 threads per site:
+  // 33,592 sites 59 / 83 us, 92,160: 125 / 109, 262,144: 293 / 266; 4 threads:
+  // 21,952: 45 / 51, 33,592: 58 / 53, 2,097,152: 2,076 / 1,891; two lanes for
+  // one: 33,592: 76 / 96, 92,160: 156 / 123).
+  e.copies = !e.wide && (!t.grad_block || t.grad_block == kBlock) && n_sites * (e.twin ? 2 : e.tps) >= 25 * 32 * (int64_t)sms;
   return e;
 }
 
