@@ -64,10 +64,10 @@ int current_device_sms() {
   return device_sms(dev);
 }
 
-a2c_status eval_device_impl(a2c_gpp_ctx *c, const double *dX, double *d_f, double *dG, cudaEvent_t *ev) {
+a2c_status eval_device_impl(a2c_gpp_ctx *c, const double *dX, double *d_f, double *dG, cudaEvent_t *ev, double *keep) {
   if (!c->has_neighbors) return A2C_ERR_STATE;
   if (c->p.precision == A2C_MIXED) {
-    A2C_TRY(mixed_eval(c, dX, d_f, dG, ev));
+    A2C_TRY(mixed_eval(c, dX, d_f, dG, ev, keep));
   } else {
     if (ev) cudaEventRecord(ev[0], c->stream);
     if (ev) cudaEventRecord(ev[1], c->stream);
@@ -77,6 +77,7 @@ a2c_status eval_device_impl(a2c_gpp_ctx *c, const double *dX, double *d_f, doubl
     if (ev) cudaEventRecord(ev[3], c->stream);
     A2C_TRY(reduce_objective(c, d_f));
     if (ev) cudaEventRecord(ev[4], c->stream);
+    if (keep) A2C_CUDA(cudaMemcpyAsync(keep, dX, sizeof(double) * 4 * c->N, cudaMemcpyDeviceToDevice, c->stream));
   }
   c->has_density = (c->p.precision != A2C_MIXED);
   return A2C_OK;
@@ -812,9 +813,7 @@ a2c_status a2c_gpp_get_shell_counts(a2c_gpp_ctx *c, int *PdPdnum) {
 a2c_status a2c_gpp_eval_device(a2c_gpp_ctx *c, const double *dX, double *df, double *dG) {
   if (!c || (!dX && c->N > 0) || !df || (!dG && c->N > 0)) return A2C_ERR_INVALID;
   DeviceGuard g(c->device);
-  A2C_TRY(eval_device_impl(c, dX, df, dG));
-  if (dX != c->d_X && c->N > 0)
-    A2C_CUDA(cudaMemcpyAsync(c->d_X, dX, sizeof(double) * 4 * c->N, cudaMemcpyDeviceToDevice, c->stream));
+  A2C_TRY(eval_device_impl(c, dX, df, dG, nullptr, dX != c->d_X && c->N > 0 ? c->d_X : nullptr));
   c->has_state = true;
   return A2C_OK;
 }

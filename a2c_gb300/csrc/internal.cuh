@@ -292,6 +292,7 @@ a2c_status lbfgs_minimize(a2c_gpp_ctx *c, double *dX, const a2c_lbfgs_params *lp
 void lbfgs_free(a2c_gpp_ctx *c);
 
 // api.cu
-a2c_status eval_device_impl(a2c_gpp_ctx *c, const double *dX, double *d_f, double *dG, cudaEvent_t *ev = nullptr);
+a2c_status eval_device_impl(a2c_gpp_ctx *c, const double *dX, double *d_f, double *dG, cudaEvent_t *ev = nullptr,
+                            double *keep = nullptr);
 
 }  // namespace a2c

@@ -73,7 +73,7 @@ struct Mixed {
   int *npre = nullptr;
   float4 *recv = nullptr;
   double *Gown = nullptr;  // 4 per site: the owner's share of the gradient (k_grad_once)
-  void *fpart = nullptr;     // the objective's block sums: one ObjSum per block of k_objective
+  void *fpart = nullptr;     // the objective's block sums: one ObjSum per block
   unsigned *fcount = nullptr;
   int64_t sym_entries = 0, sym_sites = 0;  // capacities
   uint64_t sym_version = ~0ull;            // list version the index was built for
@@ -134,7 +134,7 @@ struct MixArgs {
   const int *npre;
   float4 *recv;
   double *Gown;
-  // A single system's objective (k_objective): per block its sums, the
+  // A single system's objective: per block its sums, the
   // count of blocks done, f and its two sums.
   ObjSum *fpart;
   unsigned *fcount;
@@ -588,11 +588,15 @@ __device__ __forceinline__ void add_pair(SiteAcc &A, const PairAcc &p, float3 D,
 }
 
 // The objective of a single system, f = (1/T) sum_i V_i - 3 kB sum_i x_i
-// ln sigma_i (minimizer.cpp:353), in one launch: every block sums a
-// stride of the per-site terms and the last block to finish adds the block
-// sums (15 us at 262,144 sites on a GB300, where the two-kernel FP64
-// reduction the plain form keeps took 18 us; appended to k_grad_once the
-// same tail cost its main loop 8%, to k_grad_recv 25 us).  The sums do not
+// ln sigma_i (minimizer.cpp:353): every block sums a stride of the per-site
+// terms and the last block to finish adds the block sums.  Pass 2 wrote the
+// terms, so with pairs evaluated once the first blocks of k_grad_recv do it
+// while the others sum the received shares (an evaluation of 512 sites 41 ->
+// 31 us, with X kept by k_prep instead of a copy of its own; 262,144: 428 ->
+// 414); else, and where the stages are timed, it has a launch of its own
+// (12 us at 262,144 sites on a GB300, where the two-kernel FP64 reduction
+// the plain form keeps took 18 us; as a tail of k_grad_once it cost that
+// kernel's main loop 8%, as one of k_grad_recv's blocks 25 us).  The sums do not
 // depend on the order of their terms, so neither the tile, the grid nor
 // the order in which blocks finish changes a bit: every term is added as a
 // 64.64 fixed-point number (a signed 128-bit integer in units of 2^-64,
@@ -682,11 +686,12 @@ __device__ __forceinline__ ObjSum obj_block(ObjSum a, ObjSum *sh) {
   return a;
 }
 
-__global__ void __launch_bounds__(kBlock) k_objective(MixArgs a) {
+// blocks 0 ... blocks - 1 of a grid, all threads of each
+__device__ __forceinline__ void objective(const MixArgs &a, unsigned blocks) {
   __shared__ ObjSum sh[32];
   __shared__ bool last;
   ObjSum o{};
-  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < a.N; s += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < a.N; s += (int64_t)blocks * blockDim.x) {
     obj_term(o, a.Vs[s], false);
     obj_term(o, a.Ss[s], true);
   }
@@ -694,13 +699,13 @@ __global__ void __launch_bounds__(kBlock) k_objective(MixArgs a) {
   if (threadIdx.x == 0) {
     a.fpart[blockIdx.x] = o;
     __threadfence();
-    last = atomicAdd(a.fcount, 1u) == gridDim.x - 1;
+    last = atomicAdd(a.fcount, 1u) == blocks - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
   ObjSum t{};
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
+  for (int i = threadIdx.x; i < (int)blocks; i += blockDim.x) {
     const volatile ObjSum *q = a.fpart + i;
     ObjSum b;
     b.v.lo = q->v.lo;
@@ -719,12 +724,13 @@ __global__ void __launch_bounds__(kBlock) k_objective(MixArgs a) {
     a.fsums[0] = sa;
     a.fsums[1] = sb;
     *a.fcount = 0u;
-    if (a.hout) {  // every other kernel of the evaluation has finished: its status bits are in
+    if (a.hout) {  // k_prep, which alone sets status bits, has finished
       a.hout[0] = f;
       *reinterpret_cast<int *>(a.hout + 1) = atomicExch(a.status, 0);
     }
   }
 }
+__global__ void __launch_bounds__(kBlock) k_objective(MixArgs a) { objective(a, gridDim.x); }
 
 template <int TPS, bool LIST, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_mixed(MixArgs a) {
@@ -1017,13 +1023,18 @@ __global__ void __launch_bounds__(BLOCK, grad_min_blocks<BLOCK>()) k_grad_once(M
 
 // The shares a site received (its list entries after the first npre),
 // summed in list order with compensation and added to its own share: G is
-// written once (it may be the caller's host-mapped memory).
+// written once (it may be the caller's host-mapped memory).  The first `obj`
+// blocks compute the objective instead.
 template <int TPS, bool LIST>
-__global__ void __launch_bounds__(kBlock) k_grad_recv(MixArgs a) {
+__global__ void __launch_bounds__(kBlock) k_grad_recv(MixArgs a, unsigned obj) {
   constexpr int kSitesPerBlock = kBlock / TPS;
+  if (!LIST && blockIdx.x < obj) {
+    objective(a, obj);
+    return;
+  }
   const int64_t n = LIST ? (int64_t)*a.bv.count : a.N;
-  for (int64_t base = (int64_t)blockIdx.x * kSitesPerBlock; base < n;
-       base += (int64_t)gridDim.x * kSitesPerBlock) {
+  for (int64_t base = (int64_t)(blockIdx.x - obj) * kSitesPerBlock; base < n;
+       base += (int64_t)(gridDim.x - obj) * kSitesPerBlock) {
     const int64_t k = base + threadIdx.x / TPS;
     const int lane = (int)(threadIdx.x % TPS);
     const bool live = k < n;
@@ -1194,11 +1205,13 @@ struct SpanArgs {
   int *status;
 };
 
+// keep: the context's own copy of the state, null where X is that already.
 __global__ void k_prep(const double *X, const double *occ, int64_t N, double k0, double k1, double k2, int4 *P,
-                       float *occf, SpanArgs sg) {
+                       float *occf, double *keep, SpanArgs sg) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= N) return;
   const double4 x = make_double4(X[4 * s], X[4 * s + 1], X[4 * s + 2], X[4 * s + 3]);
+  if (keep) *reinterpret_cast<double4 *>(keep + 4 * s) = x;
   span_check(x, sg.xl, s, sg.lim[0], sg.lim[1], sg.lim[2], sg.status);
   const long long u0 = __double2ll_rn(x.x * k0);
   const long long u1 = __double2ll_rn(x.y * k1);
@@ -1295,9 +1308,13 @@ const ExpTerms &exp_consts() {
 // ms at 2 threads per site) -- its share traffic costs more than the
 // arithmetic it saves.
 constexpr int kRecvTps = 8;  // lanes per site summing the received shares
-// k_objective's grid: blocks per SM at most (at 262,144 sites 2 per SM took
+// The objective's grid: blocks per SM at most (at 262,144 sites 2 per SM took
 // 12.3 us, 8 per SM 17.9 us: the last-block count is one contended atomic)
 constexpr int kObjBlocksPerSm = 2;
+unsigned objective_blocks(int64_t n) {
+  const int64_t most = kObjBlocksPerSm * (int64_t)current_device_sms();
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + kBlock - 1) / kBlock, most));
+}
 // Persistent grid size of a kernel at a block size on the current device
 // (resident blocks x SMs), computed once per (kernel, block, device) under
 // a lock, with the dynamic shared-memory limit raised on that device first.
@@ -1394,32 +1411,35 @@ void launch_pass2(const MixArgs &a, cudaStream_t st, bool once, const Tile &t) {
 }
 
 template <int V, bool LIST>
-void launch_pair_kernels(const MixArgs &a, cudaStream_t st, cudaEvent_t *ev, bool once, const Tile &t) {
+void launch_pair_kernels(const MixArgs &a, cudaStream_t st, cudaEvent_t *ev, bool once, const Tile &t, bool fold) {
   launch_pass1<V, LIST>(a, st, t);
   if (ev) cudaEventRecord(ev[2], st);
   launch_pass2<V, LIST>(a, st, once, t);
   if (once) {
     const void *fn = (const void *)k_grad_recv<kRecvTps, LIST>;
-    k_grad_recv<kRecvTps, LIST><<<persistent_grid(a.N, kBlock / kRecvTps, grid_cap(fn, kBlock, 0)), kBlock, 0, st>>>(a);
+    const unsigned obj = fold ? objective_blocks(a.N) : 0u;
+    k_grad_recv<kRecvTps, LIST>
+        <<<obj + persistent_grid(a.N, kBlock / kRecvTps, grid_cap(fn, kBlock, 0)), kBlock, 0, st>>>(a, obj);
   }
   if (ev) cudaEventRecord(ev[3], st);
 }
 
 // Dispatch on threads per site.
-void launch_tile(const MixArgs &a, cudaStream_t st, cudaEvent_t *ev, bool once, const Tile &t, bool list) {
+void launch_tile(const MixArgs &a, cudaStream_t st, cudaEvent_t *ev, bool once, const Tile &t, bool list,
+                 bool fold = false) {
   if (list) {
     switch (t.tps) {
-      case 1: launch_pair_kernels<1, true>(a, st, ev, once, t); break;
-      case 2: launch_pair_kernels<2, true>(a, st, ev, once, t); break;
-      case 4: launch_pair_kernels<4, true>(a, st, ev, once, t); break;
-      default: launch_pair_kernels<8, true>(a, st, ev, once, t); break;
+      case 1: launch_pair_kernels<1, true>(a, st, ev, once, t, false); break;
+      case 2: launch_pair_kernels<2, true>(a, st, ev, once, t, false); break;
+      case 4: launch_pair_kernels<4, true>(a, st, ev, once, t, false); break;
+      default: launch_pair_kernels<8, true>(a, st, ev, once, t, false); break;
     }
   } else {
     switch (t.tps) {
-      case 1: launch_pair_kernels<1, false>(a, st, ev, once, t); break;
-      case 2: launch_pair_kernels<2, false>(a, st, ev, once, t); break;
-      case 4: launch_pair_kernels<4, false>(a, st, ev, once, t); break;
-      default: launch_pair_kernels<8, false>(a, st, ev, once, t); break;
+      case 1: launch_pair_kernels<1, false>(a, st, ev, once, t, fold); break;
+      case 2: launch_pair_kernels<2, false>(a, st, ev, once, t, fold); break;
+      case 4: launch_pair_kernels<4, false>(a, st, ev, once, t, fold); break;
+      default: launch_pair_kernels<8, false>(a, st, ev, once, t, fold); break;
     }
   }
 }
@@ -1670,31 +1690,34 @@ a2c_status mixed_eval(a2c_gpp_ctx *c, const double *dX, double *d_f, double *dG,
   a.npre = M->npre;
   a.recv = M->recv;
   a.Gown = M->Gown;
-  a.fpart = (ObjSum *)M->fpart;  // k_objective
+  a.fpart = (ObjSum *)M->fpart;
   a.fcount = M->fcount;
   a.f = d_f;
   a.fsums = c->d_red + 2 * 1024;
   a.hout = h_out;
   a.status = c->d_status;
+  bool fold = false;
   if (ev) cudaEventRecord(ev[0], c->stream);
   if (N > 0) {
     const SpanArgs sg = span_args(c);
-    if (Xcopy)
+    if (Xcopy && h_out)
       k_prep_copy<<<grid_for(N, 256), 256, 0, c->stream>>>(dX, c->d_occ, N, k[0], k[1], k[2], M->P, M->occ, Xcopy,
                                                            sg);
     else
-      k_prep<<<grid_for(N, 256), 256, 0, c->stream>>>(dX, c->d_occ, N, k[0], k[1], k[2], M->P, M->occ, sg);
+      k_prep<<<grid_for(N, 256), 256, 0, c->stream>>>(dX, c->d_occ, N, k[0], k[1], k[2], M->P, M->occ, Xcopy, sg);
     A2C_CUDA(cudaGetLastError());
     if (ev) cudaEventRecord(ev[1], c->stream);
-    launch_tile(a, c->stream, ev, once, effective_tile(mixed_tile(c), N, device_sms(c->device)), false);
+    // the objective goes with the received shares unless the stages are timed
+    fold = once && !ev;
+    launch_tile(a, c->stream, ev, once, effective_tile(mixed_tile(c), N, device_sms(c->device)), false, fold);
     A2C_CUDA(cudaGetLastError());
   } else if (ev) {
     for (int k2 = 1; k2 < 4; ++k2) cudaEventRecord(ev[k2], c->stream);
   }
-  k_objective<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(grid_for(N, kBlock),
-                                                                  kObjBlocksPerSm * (int64_t)device_sms(c->device))),
-                kBlock, 0, c->stream>>>(a);
-  A2C_CUDA(cudaGetLastError());
+  if (!fold) {
+    k_objective<<<objective_blocks(N), kBlock, 0, c->stream>>>(a);
+    A2C_CUDA(cudaGetLastError());
+  }
   if (ev) cudaEventRecord(ev[4], c->stream);
   return A2C_OK;
 }
@@ -1780,7 +1803,7 @@ a2c_status mixed_chem(a2c_gpp_ctx *c, const double *dX, double *d_send, const in
   a.FF = M->FF;
   a.T = c->p.T;
   // the state's fixed-point form and pass 1 (F and F' of every site)
-  k_prep<<<grid_for(N, 256), 256, 0, c->stream>>>(dX, c->d_occ, N, k[0], k[1], k[2], M->P, M->occ, span_args(c));
+  k_prep<<<grid_for(N, 256), 256, 0, c->stream>>>(dX, c->d_occ, N, k[0], k[1], k[2], M->P, M->occ, nullptr, span_args(c));
   Tile one = mixed_tile(c);
   one.tps = 1;
   const Tile t = effective_tile(one, N, device_sms(c->device));
@@ -1986,7 +2009,7 @@ extern "C" a2c_status a2c_gpp_eval_mixed_noalloc(a2c_gpp_ctx *c, const double *d
   }
   if (N > 0) {
     k_prep<<<grid_for(N, 256), 256, 0, c->stream>>>(dX, c->d_occ, N, k[0], k[1], k[2], (int4 *)(base + kNaP),
-                                                     (float *)(base + kNaOcc), span_args(c));
+                                                     (float *)(base + kNaOcc), nullptr, span_args(c));
     launch_tile(a, c->stream, nullptr, once, effective_tile(mixed_tile(c), N, device_sms(c->device)), false);
   }
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(kNaRedGrid, (N + kNaRedBlock - 1) / kNaRedBlock));
