@@ -645,6 +645,42 @@ A2C_HD bool quick_cr_exp(double x, double &out) {
   out = scale_normal(out, k);
   return ok;
 }
+// e^x and e^-x, |x| < 700, each with its own test (bits 0 and 1 of the
+// result): quick_exp's steps with the reduction shared and the degree-7 tail
+// split into its even and odd part, whose rounding stays some 2^-78 of 1.
+A2C_HD int quick_cr_exp_both(double x, double &up, double &down) {
+  const double t = x * 92.33248261689366 + kRoundShift;
+  const double n = t - kRoundShift;
+  const int ni = lo_word(t);
+  const double r1 = fma(-n, 0.010830424696223417, x);
+  const double p = n * 2.572804622327669e-14, pe = fma(n, 2.572804622327669e-14, -p);
+  D2 r = two_sum(r1, -p);
+  r = quick_two_sum(r.hi, r.lo - pe);
+  const double v = r.hi * r.hi, ve = fma(r.hi, r.hi, -v), vh = 0.5 * v;
+  const double odd = fma(v, fma(v, 1.984126984126984e-04, 8.333333333333333e-03), 1.6666666666666666e-01);
+  const double even = fma(v, 1.388888888888889e-03, 4.1666666666666664e-02);
+  const double w = fma(r.hi, r.lo, 0.5 * ve);
+  int ok = 0;
+  for (int side = 0; side < 2; ++side) {
+    const double rh = side ? -r.hi : r.hi, rl = side ? -r.lo : r.lo;
+    const int m = side ? -ni : ni, j = m & 63;
+    const double c = (rh * v) * fma(rh, even, odd);
+    const D2 s = quick_two_sum(rh, vh);
+    const double e2 = s.lo + (c + (w + rl));
+#if defined(__CUDA_ARCH__)
+    const double th = kExp2TabDev[j][0], tl = kExp2TabDev[j][1];
+#else
+    const double th = kExp2TabHost[j][0], tl = kExp2TabHost[j][1];
+#endif
+    const D2 q = two_prod(th, s.hi);
+    const D2 h = quick_two_sum(th, q.hi);
+    const D2 f = quick_two_sum(h.hi, h.lo + (q.lo + fma(th, e2, fma(tl, s.hi, tl))));
+    double &out = side ? down : up;
+    if (rounds_to(f, f.hi * 8.470329472543003e-22, out)) ok |= 1 << side;  // 2^-70
+    out = scale_normal(out, (m - j) / 64);
+  }
+  return ok;
+}
 A2C_HD bool quick_cr_log(double u, double &out) {
   double err;
   const D2 v = quick_log(u, err);
@@ -685,6 +721,19 @@ A2C_HD double cr_exp(double x) {
   if (quick_cr_exp(x, q)) return q;
 #endif
   return series_exp(x);
+}
+// cr_exp(x) and cr_exp(-x)
+A2C_HD void cr_exp_both(double x, double &up, double &down) {
+#if defined(__CUDA_ARCH__)
+  if (x > -700.0 && x < 700.0) {
+    const int ok = quick_cr_exp_both(x, up, down);
+    if (!(ok & 1)) up = series_exp(x);
+    if (!(ok & 2)) down = series_exp(-x);
+    return;
+  }
+#endif
+  up = cr_exp(x);
+  down = cr_exp(-x);
 }
 A2C_HD double cr_log(double u) {
   if (!(u > 0.0) || !(u < 1.0e300) || u < 1.0e-300) return log(u);

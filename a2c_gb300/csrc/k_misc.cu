@@ -118,8 +118,9 @@ __global__ void k_flags(const int *sites, int n, int nH, int *flags) {
 // lanes, which evaluate that many neighbors side by side and add their
 // terms in list order, so the sum is the serial one.  One thread per site
 // left a 55,296-site slab 2.8 warps per scheduler.  With the quick exp and
-// log of ddmath.cuh the step takes 12 + 199 us at 55,296 H sites, where it
-// took 4,083 us.
+// log of ddmath.cuh the step takes 10 + 160 us at 55,296 H sites (k_diffuse 199
+// with the two exponentials apart: they share the argument's reduction),
+// where it took 4,083 us.
 __global__ void k_hop_potential(const double *x0, const double *gamma, int nH, double *phi) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nH) return;
@@ -143,7 +144,9 @@ __global__ void k_diffuse(const double *x0, const int64_t *hh1_off, const int *h
     if (t0 + lane < e) {
       const int j = hh1[t0 + lane];
       const double xj = x0[j], fj = phi[j];
-      term = xj * (1.0 - xi) * dd::cr_exp(-(fi - fj) / 2.0) - xi * (1.0 - xj) * dd::cr_exp((fi - fj) / 2.0);
+      double up, down;
+      dd::cr_exp_both((fi - fj) / 2.0, up, down);
+      term = xj * (1.0 - xi) * down - xi * (1.0 - xj) * up;
     }
     __syncwarp(group);
 #pragma unroll

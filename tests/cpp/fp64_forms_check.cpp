@@ -33,6 +33,10 @@ int main(int argc, char **argv) {
       const double x = i % 3 == 0 ? (U(g) - 0.5) * 1398 : i % 3 == 1 ? (U(g) - 0.5) * 40 : (U(g) - 0.5) * std::ldexp(1.0, -(int)(g() % 60));
       const bool ok = dd::quick_cr_exp(x, q);
       tally(ok, q, dd::series_exp(x));
+      double up = 0.0, down = 0.0;
+      const int both = dd::quick_cr_exp_both(x, up, down);
+      tally(both & 1, up, dd::series_exp(x));
+      tally(both & 2, down, dd::series_exp(-x));
     } else if (form == "log") {
       const double t = U(g);
       const double x = i % 4 == 0 ? std::exp((t - 0.5) * 1300) : i % 4 == 1 ? t / (1.0 - t) : i % 4 == 2 ? 1.0 + (t - 0.5) * std::ldexp(1.0, -(int)(g() % 50)) : 60 * t;
