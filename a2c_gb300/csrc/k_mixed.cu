@@ -1079,31 +1079,32 @@ __global__ void __launch_bounds__(kBlock) k_grad_recv(MixArgs a, unsigned obj) {
 // and  sum_{j in HH} x_j sum_k W [F'_H(rho_j) f_H(s) + phi_H(s)]  in FP32 with
 // compensated sums over neighbors (F' and F from pass 1 of the same state),
 // then F_H(rho_i), the correction terms (FP64; zero unless coe_* are set)
-// and log(x/(1-x)) + chi/(kB T) in FP64.  One thread per H site; send as in
-// k_chem64.
+// and log(x/(1-x)) + chi/(kB T) in FP64.  kChemLanes lanes per H site take a
+// neighbor each and add their terms in list order: a thread per site left the
+// SMs 11 warps each at 55,296 H sites, waiting for their gathers (115 us,
+// two lanes 80, four 78; with both species in one loop, the constants picked
+// per neighbor, 111).  send as in k_chem64.
+constexpr int kChemLanes = 4;
 __global__ void __launch_bounds__(kBlock) k_chem_mixed(MixArgs a, int nH, double coePd0, double coePd2, double coePd3,
                                                        double coeH0, double coeH1, double coeH2, double coeH3,
                                                        const double *occ64, const int *full, double *send) {
-  const int64_t h = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= nH) return;
-  send[h] = 0.0;
+  const int64_t h = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kChemLanes;
+  const int lane = (int)(threadIdx.x % kChemLanes);
+  if (h >= nH) return;  // a site's lanes together, here and below
+  if (lane == 0) send[h] = 0.0;
   if (full[h] == 1) return;
   const int64_t s = (int64_t)a.nPd + h;
   const int4 pi = a.P[s];
-  const float ui = kSqrt6 * __int_as_float(pi.w), ui2 = ui * ui;
+  const float ui = kSqrt6 * __int_as_float(pi.w);
+  const unsigned group = site_lanes<kChemLanes>();
   const float3 sc = make_float3(a.sc[0], a.sc[1], a.sc[2]);
   const int64_t b = a.off[s], m = b + a.npd[s], e = a.off[s + 1];
   float acc = 0.0f, cmp = 0.0f;
-  for (int64_t t = b; t < e; ++t) {
-    const int64_t j = __ldg(&a.nbr[t]) & kIdMask;
-    const int4 pj = __ldg(&a.P[j]);
+  auto add = [&](const MorseExp &mo, int64_t first, int64_t end, int4 pj, float xj, float Fj) {
     const float3 D = pair_vec(sc, pi, pj);
     const float uj = kSqrt6 * __int_as_float(pj.w);
     const float D2 = fmaf(D.x, D.x, fmaf(D.y, D.y, D.z * D.z));
-    const float Ai = D2 + ui2, Aj = fmaf(uj, uj, D2);
-    const float Fj = __ldg(&a.FF[j].x);
-    const bool jPd = t < m;
-    const MorseExp &mo = jPd ? a.ex.pdh : a.ex.hh;
+    const float Ai = fmaf(ui, ui, D2), Aj = fmaf(uj, uj, D2);
     float part = 0.0f;
     const float Dv[3] = {D.x, D.y, D.z};
 #pragma unroll
@@ -1117,8 +1118,22 @@ __global__ void __launch_bounds__(kBlock) k_chem_mixed(MixArgs a, int nH, double
         part += fmaf(Fj, fH(a.ex, r), phi);
       }
     }
-    kahan(acc, cmp, part * (jPd ? a.W : a.W * __ldg(&a.occ[j])));
-  }
+    const float w = a.W * xj;  // W of a Pd neighbor
+#pragma unroll
+    for (int q = 0; q < kChemLanes; ++q) {
+      const float v = __shfl_sync(group, part, q, kChemLanes), wq = __shfl_sync(group, w, q, kChemLanes);
+      if (first + q < end) kahan_product(acc, cmp, v, wq);
+    }
+  };
+  walk_together<kChemLanes, false, true>(a, b, m, lane,
+                                         [&](bool, int64_t, int64_t first, int4 pj, float xj, float Fj) {
+    add(a.ex.pdh, first, m, pj, xj, Fj);
+  });
+  walk_together<kChemLanes, true, true>(a, m, e, lane,
+                                        [&](bool, int64_t, int64_t first, int4 pj, float xj, float Fj) {
+    add(a.ex.hh, first, e, pj, xj, Fj);
+  });
+  if (lane) return;
   const double T = a.T;
   double sum = (double)a.FF[s].y + (double)(acc - cmp);
   if (coeH0 != 0.0 || coeH1 != 0.0 || coeH2 != 0.0 || coeH3 != 0.0 || coePd0 != 0.0) {
@@ -1809,7 +1824,7 @@ a2c_status mixed_chem(a2c_gpp_ctx *c, const double *dX, double *d_send, const in
   const Tile t = effective_tile(one, N, device_sms(c->device));
   launch_pass1<1, false>(a, c->stream, t);
   const double *cp = c->p.coe_Pd, *ch = c->p.coe_H;
-  k_chem_mixed<<<grid_for(nH, kBlock), kBlock, 0, c->stream>>>(a, nH, cp[0], cp[2], cp[3], ch[0], ch[1], ch[2], ch[3],
+  k_chem_mixed<<<grid_for((int64_t)nH * kChemLanes, kBlock), kBlock, 0, c->stream>>>(a, nH, cp[0], cp[2], cp[3], ch[0], ch[1], ch[2], ch[3],
                                                                c->d_occ, d_full, d_send);
   A2C_CUDA(cudaGetLastError());
   return A2C_OK;
