@@ -547,7 +547,7 @@ __global__ void k_report(const int64_t *total, const int64_t *total1, const int 
 // Skin refilter, one exact pass over the extended lists, a warp per site:
 // site i's neighbors at rc go to tmp[ext_off[i] ...] in the extended list's
 // order -- its Pd part, then its H part, each sorted by id, the order
-// k_nbr_fill gives -- with the counts of k_nbr_count.
+// a full build gives -- with its counts.
 __global__ void __launch_bounds__(32 * kListWarps) k_refilter(GridArgs g, const int64_t *ext_off,
                                                               const uint32_t *ext_nbr, uint32_t *tmp, int64_t *count,
                                                               int *npd, int64_t *hh1count, int *shell, int *most) {

@@ -875,7 +875,7 @@ def run_ours(args):
                 "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 8 * 4 * Ns,
                         "d2h_bytes_per_step": 8 * 4 * Ns + 8},
                 "roofline": roofline, "cpu_baseline": cpu, "clocks": clocks,
-                "gpu_launches": (5 if once else 4) * args.steps,  # k_prep, k_rho_mixed, pass 2 (1 or 2), k_objective
+                "gpu_launches": 4 * args.steps,  # k_prep, k_rho_mixed, k_grad_once + k_grad_recv (or k_grad_mixed + k_objective)
                 "fp64_plain": {"value": value_64, "unit": UNIT, "steps": args.fp64_steps,
                                "ms_per_step": dev_time_64 * 1e3 / args.fp64_steps},
                 "mixed_over_fp64": value / value_64,
