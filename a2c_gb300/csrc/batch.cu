@@ -158,8 +158,12 @@ __device__ __forceinline__ double chunk_max(const double *part, int c0, int c1, 
 // totals, which spares a launch of one block per instance after every chunk
 // kernel -- no block waits for another.  The chunks of an instance are all
 // or none of them worked on by a kernel, so the count ends at `chunks`; it
-// is reset here.
+// is reset here.  What every thread of the block read of the instance's
+// record before the call stays true of it: the barrier comes before the
+// count, and the block that finishes the instance changes the record only
+// after it has seen all counts.
 __device__ __forceinline__ bool chunk_done(Inst &I, int chunks, int *sh_last) {
+  __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     const unsigned n = atomicAdd(&I.arrived, 1u) + 1u;
@@ -583,12 +587,14 @@ __global__ void __launch_bounds__(kBlk) k_objective(Dev D, Cfg cf, double *f) {
   if (threadIdx.x == 0) f[b] = v;
 }
 
-// The line-search decision (lbfgs.cu) of instance b, by a whole block.
-__device__ __forceinline__ void decide(const Dev &D, const Cfg &cf, int b, double *sh) {
+// The line-search decision (lbfgs.cu) of instance b, by a whole block;
+// `first`: this was a phase's first evaluation (I.state == kNeedEval, read
+// before chunk_done: thread 0 changes the state below with no barrier after
+// objective's).
+__device__ __forceinline__ void decide(const Dev &D, const Cfg &cf, int b, bool first, double *sh) {
   Inst &I = D.st[b];
   const double fn = objective(D, cf, b, sh);
   const int e0 = D.ecb[b], e1 = D.ecb[b + 1];
-  const bool first = I.state == kNeedEval;
   double dec = 0.0, dn = 0.0, sy = 0.0, yy = 0.0;
   if (!first) {
     dec = chunk_total(D.part + 4 * cf.nec, e0, e1, sh);
@@ -684,10 +690,11 @@ __global__ void __launch_bounds__(kBlk) k_post(Dev D, Cfg cf, int eblocks) {
     const Chunk ch = elements ? D.ech[c] : D.sch[c];
     const int b = ch.inst;
     Inst &I = D.st[b];
-    if (I.state != kLineSearch && I.state != kNeedEval) continue;
+    const int state = I.state;
+    if (state != kLineSearch && state != kNeedEval) continue;
     if (!elements) {
       objective_chunk(D, cf, c, ch, sh);
-    } else if (I.state == kLineSearch) {
+    } else if (state == kLineSearch) {
       double s[kPer], y[kPer], x[kPer], g[kPer];
       load_chunk(D.xn, ch, s);
       load_chunk(D.x, ch, x);
@@ -713,7 +720,8 @@ __global__ void __launch_bounds__(kBlk) k_post(Dev D, Cfg cf, int eblocks) {
         D.part[7 * cf.nec + c] = yy;
       }
     }
-    if (chunk_done(I, D.ecb[b + 1] - D.ecb[b] + D.scb[b + 1] - D.scb[b], &last)) decide(D, cf, b, sh);
+    if (chunk_done(I, D.ecb[b + 1] - D.ecb[b] + D.scb[b + 1] - D.scb[b], &last))
+      decide(D, cf, b, state == kNeedEval, sh);
   }
 }
 
