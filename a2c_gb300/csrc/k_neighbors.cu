@@ -974,6 +974,7 @@ a2c_status update_neighbors_device(a2c_gpp_ctx *c, const PosScan *scan, int *reb
   }
   const bool need = !c->has_ext || (scan->flags & kPosMoved);
   if (need) {
+    c->has_ext = false;  // until the new ones stand: a failed build leaves offsets without their lists
     A2C_TRY(lists_from_cells(c, *scan, c->p.rc + c->skin, true));
     if (N > 0)
       A2C_CUDA(cudaMemcpyAsync(c->d_xref, c->d_X, sizeof(double) * 4 * N, cudaMemcpyDeviceToDevice, c->stream));
