@@ -493,6 +493,11 @@ __device__ __forceinline__ void write_sorted(uint32_t *src, int n, Out out) {
   }
 }
 
+// Room for a list of n entries, and the dynamic shared memory of a block of
+// k_cell_lists at that room (at most 64 KB, at kMaxPerSite).
+constexpr int list_room(int n) { return (n + 31) & ~31; }
+constexpr size_t list_smem(int room) { return sizeof(uint32_t) * 2 * (size_t)room * kListWarps; }
+
 // The list of every site, sorted by id -- Pd neighbors, then H neighbors --
 // at tmp[i * stride], with its counts; a list longer than `stride` is only
 // counted (the host then calls again with the longest list's length).  Warp
@@ -870,16 +875,19 @@ a2c_status lists_from_cells(a2c_gpp_ctx *c, const PosScan &scan, double cut, boo
     A2C_TRY(clear_counts(c, w));
     if (N > 0) {
       A2C_TRY(grow(&w->tmp, &w->tmp_cap, N * stride));
-      const size_t smem = sizeof(uint32_t) * 2 * (size_t)stride * kListWarps;  // at most 64 KB (kMaxPerSite)
+      const size_t smem = list_smem(stride);
+      // always the largest size: the attribute is the kernel's, and another
+      // thread may be about to launch it for its own context
       if (smem + sizeof(ScanShared) * kListWarps > 48 * 1024)
-        A2C_CUDA(cudaFuncSetAttribute(k_cell_lists, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        A2C_CUDA(cudaFuncSetAttribute(k_cell_lists, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)list_smem(list_room(kMaxPerSite))));
       k_cell_lists<<<blocks, 32 * kListWarps, smem, st>>>(g, w->cstart, w->cpos, w->tmp, stride, w->count, npd,
                                                           ext ? nullptr : w->hh1c, ext ? nullptr : c->d_shell, w->most);
       A2C_CUDA(cudaGetLastError());
     }
     A2C_TRY(place_lists(c, w, ext));
     if (w->report->most <= stride) break;
-    stride = (w->report->most + 31) & ~31;  // place_lists has refused more than kMaxPerSite
+    stride = list_room(w->report->most);  // place_lists has refused more than kMaxPerSite
   }
   if (N > 0) {
     k_pack<<<blocks, 32 * kListWarps, 0, st>>>(g, nullptr, stride, w->tmp, ext ? c->d_ext_off : c->d_off,
