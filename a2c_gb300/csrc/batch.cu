@@ -978,11 +978,14 @@ a2c_status init_tables(a2c_gpp_batch *b, const a2c_gpp_params *params, int n, bo
     G.nH = p.nH;
     for (int64_t i = 0; i < nk; ++i) inst[(size_t)(s0 + i)] = (uint16_t)k;
     for (int64_t i = 0; i < p.nPd; ++i) occ[(size_t)(s0 + i)] = 1.0;
+    // An instance without sites (a context may have none) gets one empty
+    // chunk of either kind: its steps are taken where a chunk is done.
     b->ecb[k] = (int)ech.size();
-    for (int64_t c0 = 0; c0 < 4 * nk; c0 += kChunk)
+    for (int64_t c0 = 0; c0 == 0 || c0 < 4 * nk; c0 += kChunk)
       ech.push_back({4 * s0 + c0, (int)std::min<int64_t>(kChunk, 4 * nk - c0), k});
     b->scb[k] = (int)sch.size();
-    for (int64_t c0 = 0; c0 < nk; c0 += kChunk) sch.push_back({s0 + c0, (int)std::min<int64_t>(kChunk, nk - c0), k});
+    for (int64_t c0 = 0; c0 == 0 || c0 < nk; c0 += kChunk)
+      sch.push_back({s0 + c0, (int)std::min<int64_t>(kChunk, nk - c0), k});
   }
   b->ecb[n] = (int)ech.size();
   b->scb[n] = (int)sch.size();
