@@ -175,6 +175,14 @@ a2c_status copy_in(a2c_gpp_ctx *c, double *dst, const double *src, int64_t n) {
 
 a2c_status finish(a2c_gpp_ctx *c) { return check_status_word(c); }
 
+// Waits for a list build or re-filter and reads its own check: the lists
+// count (has_neighbors) only after it.  An entry that did not find its place
+// is the library's fault, not an argument's.
+a2c_status lists_checked(a2c_gpp_ctx *c) {
+  const a2c_status s = check_status_word(c);
+  return s == A2C_ERR_INVALID ? A2C_ERR_STATE : s;
+}
+
 template <class T>
 a2c_status dalloc(T **p, int64_t n) {
   if (cudaMalloc((void **)p, sizeof(T) * (size_t)std::max<int64_t>(n, 1)) != cudaSuccess) return A2C_ERR_NOMEM;
@@ -535,10 +543,12 @@ a2c_status a2c_gpp_build_neighbors(a2c_gpp_ctx *c, const double *X, int *max_nei
   c->has_neighbors = false;
   c->has_density = false;
   A2C_TRY(build_neighbors_device(c, &scan));
+  const a2c_status mixed = mixed_lists_changed(c);
+  A2C_TRY(lists_checked(c));
   c->has_neighbors = true;
-  A2C_TRY(mixed_lists_changed(c));
+  A2C_TRY(mixed);
   if (max_neighbors) *max_neighbors = c->max_neighbors;
-  return finish(c);
+  return A2C_OK;
 }
 
 // Skin lists (findLocalNeighbors' refilter of the extended lists,
@@ -627,10 +637,12 @@ a2c_status a2c_gpp_update_neighbors(a2c_gpp_ctx *c, const double *X, int *max_ne
   c->has_neighbors = false;
   c->has_density = false;
   A2C_TRY(update_neighbors_device(c, &scan, rebuilt));
+  const a2c_status mixed = mixed_lists_changed(c);
+  A2C_TRY(lists_checked(c));
   c->has_neighbors = true;
-  A2C_TRY(mixed_lists_changed(c));
+  A2C_TRY(mixed);
   if (max_neighbors) *max_neighbors = c->max_neighbors;
-  return finish(c);
+  return A2C_OK;
 }
 
 namespace {
@@ -1104,8 +1116,11 @@ a2c_status a2c_gpp_dmd_run(a2c_gpp_ctx *c, double *X, double *xH, double *gamma,
     double f = 0.0, gn = 0.0;
     int it = 0, fev = 0, why = 0;
     if (k > 0 && dp->neighbor_update) {  // findNeighbors + findLocalNeighbors at the current positions
+      c->has_neighbors = false;
       s = c->skin > 0.0 ? update_neighbors_device(c, nullptr, nullptr) : build_neighbors_device(c, nullptr);
+      if (!s) s = lists_checked(c);
       if (s) break;
+      c->has_neighbors = true;
     }
     s = lbfgs_minimize(c, c->d_X, &dp->lbfgs, &f, &it, &fev, &gn, &why);  // minimizer.cpp:548
     // minimizer.cpp:607-789: densities and chemical potential at the
