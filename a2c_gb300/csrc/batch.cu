@@ -905,9 +905,13 @@ a2c_status ensure_lbfgs(a2c_gpp_batch *b, int m, int W) {
     b->exec = nullptr;
   }
   const int64_t n = 4 * b->c->N;
-  for (double **p : {&b->x, &b->g, &b->pg, &b->d, &b->xn, &b->gn}) A2C_TRY(dmalloc(p, n));
-  A2C_TRY(dmalloc(&b->S, n * (m + 1)));
-  A2C_TRY(dmalloc(&b->Y, n * (m + 1)));
+  auto vectors = [&](double **p, int64_t count) -> a2c_status {
+    const size_t bytes = sizeof(double) * (size_t)std::max<int64_t>(count, 1);
+    return context_malloc(b->c, (void **)p, bytes) == cudaSuccess ? A2C_OK : A2C_ERR_NOMEM;
+  };
+  for (double **p : {&b->x, &b->g, &b->pg, &b->d, &b->xn, &b->gn}) A2C_TRY(vectors(p, n));
+  A2C_TRY(vectors(&b->S, n * (m + 1)));
+  A2C_TRY(vectors(&b->Y, n * (m + 1)));
   A2C_TRY(dmalloc(&b->rho, (int64_t)b->B * (m + 1)));
   A2C_TRY(dmalloc(&b->alph, (int64_t)b->B * (m + 1)));
   A2C_TRY(dmalloc(&b->fh, (int64_t)b->B * (W + 1)));

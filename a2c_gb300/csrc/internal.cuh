@@ -225,6 +225,9 @@ a2c_status update_neighbors_device(a2c_gpp_ctx *c, const PosScan *scan, int *reb
 // since the extended lists were built.
 a2c_status stage_positions(a2c_gpp_ctx *c, const double *X, const double *mX, PosScan *scan);
 void lists_free(a2c_gpp_ctx *c);
+// cudaMalloc for the arrays of a context; where memory is short, the list
+// scratch that the next build allocates again is given back first.
+cudaError_t context_malloc(a2c_gpp_ctx *c, void **p, size_t bytes);
 
 // The span guard of the mixed form: per direction, how far a site may move
 // from the position the lists were built at before a listed pair could

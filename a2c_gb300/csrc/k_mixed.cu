@@ -1529,8 +1529,8 @@ a2c_status ensure_sym(a2c_gpp_ctx *c) {
     M->rev = nullptr;
     M->recv = nullptr;
     M->sym_entries = 0;
-    if (cudaMalloc(&M->rev, sizeof(uint32_t) * E) != cudaSuccess ||
-        cudaMalloc(&M->recv, sizeof(float4) * E) != cudaSuccess) {
+    if (context_malloc(c, (void **)&M->rev, sizeof(uint32_t) * E) != cudaSuccess ||
+        context_malloc(c, (void **)&M->recv, sizeof(float4) * E) != cudaSuccess) {
       (void)cudaGetLastError();  // out of memory: keep the both-sides pass
       M->sym_version = c->nbr_version;
       return A2C_OK;
@@ -1543,8 +1543,8 @@ a2c_status ensure_sym(a2c_gpp_ctx *c) {
     M->npre = nullptr;
     M->Gown = nullptr;
     M->sym_sites = 0;
-    if (cudaMalloc(&M->npre, sizeof(int) * (N + 1)) != cudaSuccess ||
-        cudaMalloc(&M->Gown, sizeof(double) * 4 * (N + 1)) != cudaSuccess) {
+    if (context_malloc(c, (void **)&M->npre, sizeof(int) * (N + 1)) != cudaSuccess ||
+        context_malloc(c, (void **)&M->Gown, sizeof(double) * 4 * (N + 1)) != cudaSuccess) {
       (void)cudaGetLastError();
       M->sym_version = c->nbr_version;
       return A2C_OK;

@@ -499,22 +499,23 @@ constexpr int list_room(int n) { return (n + 31) & ~31; }
 constexpr size_t list_smem(int room) { return sizeof(uint32_t) * 2 * (size_t)room * kListWarps; }
 
 // The list of every site, sorted by id -- Pd neighbors, then H neighbors --
-// at tmp[i * stride], with its counts; a list longer than `stride` is only
-// counted (the host then calls again with the longest list's length).  Warp
-// k takes the k-th site of cpos, so that a block's sites share cells and
-// find their candidates in the L1.  The neighbors gather in the warp's
-// shared memory (two areas of `stride` entries, Pd and H), where each finds
-// its rank.
+// at out[i * room] or, with off, at out[off[i]], with its counts; a list
+// longer than `room` is only counted (the host then calls again with the
+// lists' offsets and the longest one's length).  Warp k takes the k-th site
+// of cpos, so that a block's sites share cells and find their candidates in
+// the L1.  The neighbors gather in the warp's shared memory (two areas of
+// `room` entries, Pd and H), where each finds its rank.
 __global__ void __launch_bounds__(32 * kListWarps) k_cell_lists(GridArgs g, const int *cstart, const float4 *cpos,
-                                                                uint32_t *tmp, int stride, int64_t *count, int *npd,
-                                                                int64_t *hh1count, int *shell, int *most) {
+                                                                uint32_t *out, const int64_t *off, int room,
+                                                                int64_t *count, int *npd, int64_t *hh1count,
+                                                                int *shell, int *most) {
   extern __shared__ uint4 lists[];
   __shared__ ScanShared scan[kListWarps];
   const int64_t k = (int64_t)blockIdx.x * kListWarps + threadIdx.x / 32;
   if (k >= g.N) return;
   const int lane = threadIdx.x & 31;
-  uint32_t *const pd = reinterpret_cast<uint32_t *>(lists) + (size_t)(threadIdx.x / 32) * 2 * stride,
-                  *const h = pd + stride;
+  uint32_t *const pd = reinterpret_cast<uint32_t *>(lists) + (size_t)(threadIdx.x / 32) * 2 * room,
+                  *const h = pd + room;
   const float4 p = __ldg(&cpos[k]);
   const int i = __float_as_int(p.w);
   const bool iPd = i < g.nPd;
@@ -525,17 +526,17 @@ __global__ void __launch_bounds__(32 * kListWarps) k_cell_lists(GridArgs g, cons
     const unsigned mine = __ballot_sync(kAll, hit && jPd);
     if (hit) {
       const int at = jPd ? c.nP + __popc(mine & below) : c.n - c.nP + __popc(mask & ~mine & below);
-      if (at < stride) (jPd ? pd : h)[at] = by_id(e);
+      if (at < room) (jPd ? pd : h)[at] = by_id(e);
     }
     c.add(iPd, jPd, cls, hit, mask, mine);
   });
   if (lane == 0) c.store(g, i, iPd, count, npd, hh1count, shell, most);
-  if (c.n > stride) return;
+  if (c.n > room) return;
   __syncwarp();
-  uint32_t *const out = tmp + (int64_t)i * stride;
+  uint32_t *const list = out + (off ? off[i] : (int64_t)i * room);
   const int nP = c.nP;
-  write_sorted(pd, nP, [&](int r, uint32_t v) { out[r] = from_by_id(v); });
-  write_sorted(h, c.n - nP, [&](int r, uint32_t v) { out[nP + r] = from_by_id(v); });
+  write_sorted(pd, nP, [&](int r, uint32_t v) { list[r] = from_by_id(v); });
+  write_sorted(h, c.n - nP, [&](int r, uint32_t v) { list[nP + r] = from_by_id(v); });
 }
 
 // What the host needs to go on after the counts, into its pinned memory.
@@ -582,7 +583,7 @@ __global__ void __launch_bounds__(32 * kListWarps) k_refilter(GridArgs g, const 
 
 // The lists of k_cell_lists (at i * stride) or k_refilter (at src_off[i])
 // packed at their offsets, and each H site's first H shell (hh1; null for
-// extended lists).
+// extended lists).  tmp may be nbr, with src_off = off: lists in place.
 __global__ void __launch_bounds__(32 * kListWarps) k_pack(GridArgs g, const int64_t *src_off, int stride,
                                                           const uint32_t *tmp, const int64_t *off, uint32_t *nbr,
                                                           const int64_t *hh1_off, int *hh1, int *status) {
@@ -615,64 +616,56 @@ __global__ void __launch_bounds__(32 * kListWarps) k_pack(GridArgs g, const int6
   if (w1 != n1 && lane == 0) atomicOr(status, kStatusBadIndex);
 }
 
-// The scratch of a list build or re-filter, kept with the context: one
-// allocation, laid out by begin(), grown when a part asks for more.
+// The scratch of a list build or re-filter, kept with the context.
 // (Stream-ordered allocations per call went back to the system at every
-// synchronization of the call and cost it more than its kernels.)
+// synchronization of the call and cost it more than its kernels.)  About 90
+// bytes a site in `base`, at most 40 in `cells`; `tmp` holds 4 bytes for
+// each of a site's `stride` entries, at most 512 bytes a site or twice the
+// lists themselves, whichever is more, and is given back when the context
+// needs the memory for something else (context_malloc).
 struct ListWork {
-  void *base = nullptr;
-  size_t cap = 0;
+  void *base = nullptr;     // one allocation for the views below
   uint32_t *tmp = nullptr;  // lists before they are packed
   int64_t tmp_cap = 0;
   int stride = 96, ext_stride = 128;  // entries per site there (a multiple of 4)
+  int *cells = nullptr;  // the cell grid: counts, offsets, and the scratch of their scan
+  int64_t cells_cap = 0;
   // views of base
   double *stage = nullptr;  // 4N
   float4 *Xf = nullptr, *cpos = nullptr;
   int2 *cell = nullptr;
   int64_t *count = nullptr, *hh1c = nullptr;
-  int *npd = nullptr, *ccount = nullptr, *cstart = nullptr, *most = nullptr;
+  int *npd = nullptr, *most = nullptr;
   PosScan *scan = nullptr;
   void *cub = nullptr;
   size_t cub_bytes = 0;
   ListReport *report = nullptr;  // in the context's pinned memory, as is
   PosScan *scanned = nullptr;    // the last scan
-  int64_t ncell = 0;             // cells the layout has room for
-  int moves = 0;                 // times base was replaced (its contents lost)
 };
 
-a2c_status work_for(a2c_gpp_ctx *c, int64_t ncell, ListWork **out) {
+a2c_status work_for(a2c_gpp_ctx *c, ListWork **out) {
   if (!c->list_work) {
     c->list_work = new (std::nothrow) ListWork();
     if (!c->list_work) return A2C_ERR_NOMEM;
   }
   ListWork *w = (ListWork *)c->list_work;
   *out = w;
+  if (w->base) return A2C_OK;
   w->report = (ListReport *)(c->h_small + kHostReport);
   w->scanned = (PosScan *)(w->report + 1);
   static_assert(sizeof(ListReport) + sizeof(PosScan) <= sizeof(double) * (kHostSmall - kHostReport), "pinned area");
-  ncell = w->ncell = std::max(ncell, w->ncell);
   const int64_t N = std::max<int64_t>(c->N, 1), nH = c->p.nH;
-  size_t b0 = 0, b1 = 0, b2 = 0;
+  size_t b0 = 0, b1 = 0;
   A2C_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b0, (const int64_t *)nullptr, (int64_t *)nullptr, N + 1, c->stream));
   A2C_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b1, (const int64_t *)nullptr, (int64_t *)nullptr, nH + 1, c->stream));
-  A2C_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, b2, (const int *)nullptr, (int *)nullptr, ncell + 1, c->stream));
-  const size_t bytes[] = {sizeof(double) * 4 * N, sizeof(float4) * N, sizeof(float4) * N, sizeof(int2) * N,
-                          sizeof(int64_t) * (N + 1), sizeof(int64_t) * (nH + 1), sizeof(int) * N,
-                          sizeof(int) * (ncell + 1), sizeof(int) * (ncell + 1), sizeof(int), sizeof(PosScan),
-                          std::max(b0, std::max(b1, b2))};
-  size_t at[13] = {0};
-  for (int k = 0; k < 12; ++k) at[k + 1] = (at[k] + bytes[k] + 255) & ~(size_t)255;
-  if (at[12] > w->cap) {
-    if (w->base) {
-      A2C_CUDA(cudaStreamSynchronize(c->stream));
-      cudaFree(w->base);
-    }
-    w->base = nullptr;
-    w->cap = 0;
-    ++w->moves;
-    if (cudaMalloc(&w->base, at[12]) != cudaSuccess) return A2C_ERR_NOMEM;
-    w->cap = at[12];
-  }
+  constexpr int kParts = 10;
+  const size_t bytes[kParts] = {sizeof(double) * 4 * N, sizeof(float4) * N,       sizeof(float4) * N,
+                                sizeof(int2) * N,       sizeof(int64_t) * (N + 1), sizeof(int64_t) * (nH + 1),
+                                sizeof(int) * N,        sizeof(int),               sizeof(PosScan),
+                                std::max(b0, b1)};
+  size_t at[kParts + 1] = {0};
+  for (int k = 0; k < kParts; ++k) at[k + 1] = (at[k] + bytes[k] + 255) & ~(size_t)255;
+  if (context_malloc(c, &w->base, at[kParts]) != cudaSuccess) return A2C_ERR_NOMEM;
   char *p = (char *)w->base;
   w->stage = (double *)(p + at[0]);
   w->Xf = (float4 *)(p + at[1]);
@@ -681,21 +674,21 @@ a2c_status work_for(a2c_gpp_ctx *c, int64_t ncell, ListWork **out) {
   w->count = (int64_t *)(p + at[4]);
   w->hh1c = (int64_t *)(p + at[5]);
   w->npd = (int *)(p + at[6]);
-  w->ccount = (int *)(p + at[7]);
-  w->cstart = (int *)(p + at[8]);
-  w->most = (int *)(p + at[9]);
-  w->scan = (PosScan *)(p + at[10]);
-  w->cub = p + at[11];
-  w->cub_bytes = bytes[11];
+  w->most = (int *)(p + at[7]);
+  w->scan = (PosScan *)(p + at[8]);
+  w->cub = p + at[9];
+  w->cub_bytes = bytes[9];
   return A2C_OK;
 }
 
-template <class T, class U>
-a2c_status scan_exclusive(ListWork *w, const T *in, U *out, int64_t n, cudaStream_t st) {
-  size_t bytes = w->cub_bytes;
-  A2C_CUDA(cub::DeviceScan::ExclusiveSum(w->cub, bytes, in, out, n, st));
+a2c_status scan_exclusive(ListWork *w, const int64_t *in, int64_t *out, int64_t n, cudaStream_t st) {
+  A2C_CUDA(cub::DeviceScan::ExclusiveSum(w->cub, w->cub_bytes, in, out, n, st));
   return A2C_OK;
 }
+
+// Cells of a grid whose tables stay with the context; a larger one (a
+// sparse system in free directions) gives them back after the build.
+constexpr int64_t cells_kept(int64_t n_sites) { return 4 * n_sites + 4096; }
 
 // Cell grid for cutoff `cut` (cells at least `cut` wide), from the extents
 // of the free directions; with scan null (a list re-filter, which uses no
@@ -753,18 +746,18 @@ int64_t make_grid(const a2c_gpp_ctx *c, const PosScan *scan, double cut, GridArg
       g.scan_all[d] = n < 2 * g.reach + 1 ? 1 : 0;
       ncell *= n;
     }
-    if (g.reach == 1 || ncell <= 4 * N + 4096) break;
+    if (g.reach == 1 || ncell <= cells_kept(N)) break;
   }
   return ncell;
 }
 
 template <class T>
-a2c_status grow(T **p, int64_t *cap, int64_t need) {
+a2c_status grow(a2c_gpp_ctx *c, T **p, int64_t *cap, int64_t need) {
   if (need <= *cap) return A2C_OK;
   if (*p) cudaFree(*p);
   *p = nullptr;
   *cap = 0;
-  if (cudaMalloc(p, sizeof(T) * std::max<int64_t>(need, 1)) != cudaSuccess) return A2C_ERR_NOMEM;
+  if (context_malloc(c, (void **)p, sizeof(T) * std::max<int64_t>(need, 1)) != cudaSuccess) return A2C_ERR_NOMEM;
   *cap = need;
   return A2C_OK;
 }
@@ -792,7 +785,8 @@ a2c_status scan_positions(a2c_gpp_ctx *c, ListWork *w, const double *X, double *
   return A2C_OK;
 }
 
-// After the counts: offsets, the totals on the host, room for the lists.
+// After the counts: offsets, the totals on the host, room for the lists
+// (for which tmp, and what it holds, may have to go: null then).
 a2c_status place_lists(a2c_gpp_ctx *c, ListWork *w, bool ext) {
   const int64_t N = c->N;
   const int nH = c->p.nH;
@@ -806,11 +800,11 @@ a2c_status place_lists(a2c_gpp_ctx *c, ListWork *w, bool ext) {
   const ListReport r = *w->report;
   if (r.most > kMaxPerSite) return A2C_ERR_NEIGHBOR_OVERFLOW;
   if (ext) {
-    A2C_TRY(grow(&c->d_ext_nbr, &c->ext_cap, r.total));
+    A2C_TRY(grow(c, &c->d_ext_nbr, &c->ext_cap, r.total));
     c->ext_total = r.total;
   } else {
-    A2C_TRY(grow(&c->d_nbr, &c->nbr_cap, r.total));
-    A2C_TRY(grow(&c->d_hh1, &c->hh1_cap, r.total1));
+    A2C_TRY(grow(c, &c->d_nbr, &c->nbr_cap, r.total));
+    A2C_TRY(grow(c, &c->d_hh1, &c->hh1_cap, r.total1));
     c->nbr_total = r.total;
     c->hh1_total = r.total1;
     c->max_neighbors = r.most;
@@ -836,64 +830,85 @@ a2c_status lists_done(a2c_gpp_ctx *c, double cut) {
   return A2C_OK;
 }
 
+// Every site into its cell: the cells' offsets (cstart) and, in their order,
+// the sites (w->cpos).
+a2c_status fill_cells(a2c_gpp_ctx *c, ListWork *w, const GridArgs &g, int64_t ncell, const int **cstart) {
+  cudaStream_t st = c->stream;
+  size_t cub_bytes = 0;
+  A2C_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, cub_bytes, (const int *)nullptr, (int *)nullptr, ncell + 1, st));
+  const int64_t room = (ncell + 1 + 63) & ~(int64_t)63;  // 256-byte parts
+  A2C_TRY(grow(c, &w->cells, &w->cells_cap, 2 * room + (int64_t)(cub_bytes + sizeof(int) - 1) / (int64_t)sizeof(int)));
+  int *const ccount = w->cells, *const start = ccount + room;
+  A2C_CUDA(cudaMemsetAsync(ccount, 0, sizeof(int) * (ncell + 1), st));
+  k_cell_count<<<grid_for(c->N, 256), 256, 0, st>>>(g, w->cell, ccount);
+  A2C_CUDA(cudaGetLastError());
+  A2C_CUDA(cub::DeviceScan::ExclusiveSum(start + room, cub_bytes, (const int *)ccount, start, ncell + 1, st));
+  k_cell_fill<<<grid_for(c->N, 256), 256, 0, st>>>(g, w->cell, start, w->cpos);
+  A2C_CUDA(cudaGetLastError());
+  *cstart = start;
+  return A2C_OK;
+}
+
 // Lists (rc, or rc + skin for the extended lists, which have no shells or
 // first H shells) from a cell list over the scanned positions.  One pass
-// makes the sorted lists at a fixed stride, as long as the longest list of
-// an earlier build (at first 96, 128 for extended lists; a list that does
-// not fit makes it run again), and a copy packs them.  Bound by instruction
-// issue and the latency of the candidate loads (about 1,300 instructions a
-// site).  At 262,144 sites the pass takes 568 us and the copy 137; one
-// thread per site that walked its 27 cells twice, to count and to fill, and
-// sorted in global memory took 930 + 1,500 us; a warp per site over those
-// 27 cells in two passes took 576 + 862 us.
+// makes the sorted lists at a fixed stride (at first 96, 128 for extended
+// lists) and a copy packs them.  Lists that do not fit it, or for whose
+// stride there is no memory, are counted by that pass and written at their
+// offsets by a second; the stride then grows to the longest list unless a
+// few long ones would make it more than twice what the lists take.  Bound by
+// instruction issue and the latency of the candidate loads (about 1,300
+// instructions a site).  At 262,144 sites the pass takes 568 us and the copy
+// 137; one thread per site that walked its 27 cells twice, to count and to
+// fill, and sorted in global memory took 930 + 1,500 us; a warp per site over
+// those 27 cells in two passes took 576 + 862 us.
 a2c_status lists_from_cells(a2c_gpp_ctx *c, const PosScan &scan, double cut, bool ext) {
   const int64_t N = c->N;
   cudaStream_t st = c->stream;
   GridArgs g;
   const int64_t ncell = make_grid(c, &scan, cut, g);
   ListWork *w;
-  const int moves = c->list_work ? ((ListWork *)c->list_work)->moves : -1;
-  A2C_TRY(work_for(c, ncell, &w));
-  if (N > 0 && w->moves != moves) {  // the scratch moved: the scan again, into the new place
-    PosScan again;
-    A2C_TRY(scan_positions(c, w, nullptr, nullptr, nullptr, &again));
-  }
+  A2C_TRY(work_for(c, &w));
   g.Xf = w->Xf;
   g.qmax_bits = &w->scan->qmax_bits;
   const unsigned blocks = grid_for(N, kListWarps);
-  int *npd = ext ? w->npd : c->d_npd;
+  const int *cstart = nullptr;
+  if (N > 0) A2C_TRY(fill_cells(c, w, g, ncell, &cstart));
+  auto pass = [&](uint32_t *out, const int64_t *off, int room) -> a2c_status {
+    const size_t smem = list_smem(room);
+    // always the largest size: the attribute is the kernel's, and another
+    // thread may be about to launch it for its own context
+    if (smem + sizeof(ScanShared) * kListWarps > 48 * 1024)
+      A2C_CUDA(cudaFuncSetAttribute(k_cell_lists, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)list_smem(list_room(kMaxPerSite))));
+    k_cell_lists<<<blocks, 32 * kListWarps, smem, st>>>(g, cstart, w->cpos, out, off, room, w->count,
+                                                        ext ? w->npd : c->d_npd, ext ? nullptr : w->hh1c,
+                                                        ext ? nullptr : c->d_shell, w->most);
+    A2C_CUDA(cudaGetLastError());
+    return A2C_OK;
+  };
   int &stride = ext ? w->ext_stride : w->stride;
+  int room = stride;
+  if (grow(c, &w->tmp, &w->tmp_cap, N * stride) != A2C_OK) room = 0;
+  A2C_TRY(clear_counts(c, w));
+  if (N > 0) A2C_TRY(pass(w->tmp, nullptr, room));
+  A2C_TRY(place_lists(c, w, ext));
   if (N > 0) {
-    A2C_CUDA(cudaMemsetAsync(w->ccount, 0, sizeof(int) * (ncell + 1), st));
-    k_cell_count<<<grid_for(N, 256), 256, 0, st>>>(g, w->cell, w->ccount);
-    A2C_CUDA(cudaGetLastError());
-    A2C_TRY(scan_exclusive(w, (const int *)w->ccount, w->cstart, ncell + 1, st));
-    k_cell_fill<<<grid_for(N, 256), 256, 0, st>>>(g, w->cell, w->cstart, w->cpos);
-    A2C_CUDA(cudaGetLastError());
-  }
-  for (;;) {
-    A2C_TRY(clear_counts(c, w));
-    if (N > 0) {
-      A2C_TRY(grow(&w->tmp, &w->tmp_cap, N * stride));
-      const size_t smem = list_smem(stride);
-      // always the largest size: the attribute is the kernel's, and another
-      // thread may be about to launch it for its own context
-      if (smem + sizeof(ScanShared) * kListWarps > 48 * 1024)
-        A2C_CUDA(cudaFuncSetAttribute(k_cell_lists, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)list_smem(list_room(kMaxPerSite))));
-      k_cell_lists<<<blocks, 32 * kListWarps, smem, st>>>(g, w->cstart, w->cpos, w->tmp, stride, w->count, npd,
-                                                          ext ? nullptr : w->hh1c, ext ? nullptr : c->d_shell, w->most);
+    const int most = w->report->most;  // place_lists has refused more than kMaxPerSite
+    const int64_t *off = ext ? c->d_ext_off : c->d_off;
+    uint32_t *nbr = ext ? c->d_ext_nbr : c->d_nbr;
+    const bool in_place = most > room || !w->tmp;
+    if (in_place) A2C_TRY(pass(nbr, off, list_room(most)));
+    if (!in_place || !ext) {
+      k_pack<<<blocks, 32 * kListWarps, 0, st>>>(g, in_place ? off : nullptr, stride, in_place ? nbr : w->tmp, off, nbr,
+                                                 c->d_hh1_off, ext ? nullptr : c->d_hh1, c->d_status);
       A2C_CUDA(cudaGetLastError());
     }
-    A2C_TRY(place_lists(c, w, ext));
-    if (w->report->most <= stride) break;
-    stride = list_room(w->report->most);  // place_lists has refused more than kMaxPerSite
-  }
-  if (N > 0) {
-    k_pack<<<blocks, 32 * kListWarps, 0, st>>>(g, nullptr, stride, w->tmp, ext ? c->d_ext_off : c->d_off,
-                                               ext ? c->d_ext_nbr : c->d_nbr, c->d_hh1_off, ext ? nullptr : c->d_hh1,
-                                               c->d_status);
-    A2C_CUDA(cudaGetLastError());
+    if (most > stride && N * list_room(most) <= 2 * (int64_t)w->report->total) stride = list_room(most);
+    if (ncell > cells_kept(N)) {
+      cudaFree(w->cells);  // waits for the kernels that use it
+      w->cells = nullptr;
+      w->cells_cap = 0;
+    }
   }
   return ext ? A2C_OK : lists_done(c, cut);
 }
@@ -909,7 +924,7 @@ a2c_status refilter_lists(a2c_gpp_ctx *c) {
   GridArgs g;
   make_grid(c, nullptr, c->p.rc, g);  // only the cutoff and box are read on this path
   ListWork *w = (ListWork *)c->list_work;
-  A2C_TRY(grow(&w->tmp, &w->tmp_cap, c->ext_total));
+  A2C_TRY(grow(c, &w->tmp, &w->tmp_cap, c->ext_total));
   g.Xf = w->Xf;
   g.qmax_bits = &w->scan->qmax_bits;
   A2C_TRY(clear_counts(c, w));
@@ -920,6 +935,7 @@ a2c_status refilter_lists(a2c_gpp_ctx *c) {
     A2C_CUDA(cudaGetLastError());
   }
   A2C_TRY(place_lists(c, w, false));
+  if (!w->tmp && c->ext_total > 0) return A2C_ERR_NOMEM;
   if (N > 0) {
     k_pack<<<blocks, 32 * kListWarps, 0, st>>>(g, c->d_ext_off, 0, w->tmp, c->d_off, c->d_nbr, c->d_hh1_off, c->d_hh1,
                                                c->d_status);
@@ -930,11 +946,25 @@ a2c_status refilter_lists(a2c_gpp_ctx *c) {
 
 }  // namespace
 
+cudaError_t context_malloc(a2c_gpp_ctx *c, void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  ListWork *w = (ListWork *)c->list_work;
+  if (e == cudaErrorMemoryAllocation && w && w->tmp) {
+    cudaFree(w->tmp);  // waits for the kernels that use it
+    w->tmp = nullptr;
+    w->tmp_cap = 0;
+    (void)cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) (void)cudaGetLastError();  // reported here, not by the next launch's check
+  return e;
+}
+
 void lists_free(a2c_gpp_ctx *c) {
   ListWork *w = (ListWork *)c->list_work;
   if (!w) return;
-  if (w->base) cudaFree(w->base);
-  if (w->tmp) cudaFree(w->tmp);
+  for (void *p : {w->base, (void *)w->tmp, (void *)w->cells})
+    if (p) cudaFree(p);
   delete w;
   c->list_work = nullptr;
 }
@@ -943,7 +973,7 @@ a2c_status stage_positions(a2c_gpp_ctx *c, const double *X, const double *mX, Po
   const int64_t N = c->N;
   cudaStream_t st = c->stream;
   ListWork *w;
-  A2C_TRY(work_for(c, 0, &w));
+  A2C_TRY(work_for(c, &w));
   if (N > 0 && !mX) A2C_CUDA(cudaMemcpyAsync(w->stage, X, sizeof(double) * 4 * N, cudaMemcpyHostToDevice, st));
   A2C_TRY(scan_positions(c, w, mX ? mX : w->stage, mX ? w->stage : nullptr, c->has_ext ? c->d_xref : nullptr, scan));
   if (scan->flags & kPosNonfinite) return A2C_ERR_NONFINITE;
@@ -955,7 +985,7 @@ a2c_status stage_positions(a2c_gpp_ctx *c, const double *X, const double *mX, Po
 // The positions already in c->d_X, scanned for a build or update.
 static a2c_status scan_device(a2c_gpp_ctx *c, PosScan *scan) {
   ListWork *w;
-  A2C_TRY(work_for(c, 0, &w));
+  A2C_TRY(work_for(c, &w));
   return scan_positions(c, w, nullptr, nullptr, c->has_ext ? c->d_xref : nullptr, scan);
 }
 

@@ -254,8 +254,9 @@ static a2c_status lbfgs_alloc(a2c_gpp_ctx *c, int m) {
   L->m = m;
   const size_t b = sizeof(double) * (size_t)std::max<int64_t>(n, 1);
   for (double **p : {&L->x, &L->g, &L->pg, &L->d, &L->xn, &L->gn})
-    if (cudaMalloc(p, b) != cudaSuccess) return A2C_ERR_NOMEM;
-  if (cudaMalloc(&L->S, b * (m + 1)) != cudaSuccess || cudaMalloc(&L->Y, b * (m + 1)) != cudaSuccess)
+    if (context_malloc(c, (void **)p, b) != cudaSuccess) return A2C_ERR_NOMEM;
+  if (context_malloc(c, (void **)&L->S, b * (m + 1)) != cudaSuccess ||
+      context_malloc(c, (void **)&L->Y, b * (m + 1)) != cudaSuccess)
     return A2C_ERR_NOMEM;
   if (cudaMalloc(&L->red, sizeof(double) * (2 * kGrid + 64)) != cudaSuccess) return A2C_ERR_NOMEM;
   L->f = L->red + 2 * kGrid;
