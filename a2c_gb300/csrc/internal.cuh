@@ -7,6 +7,7 @@
 #include <functional>
 
 #include "a2c_gpp.h"
+#include "tile.h"
 
 namespace a2c {
 
@@ -154,31 +155,12 @@ inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 
 constexpr int kMaxDevices = 64;
 int device_sms(int dev);
 int current_device_sms();
-// Tile shape of the mixed pair kernels: threads per site (1, 2, 4, 8) and
-// threads per block of pass 1 (256, 512, 768) and pass 2 (128, 256, 512);
-// 0 = the library's choice.
-struct Tile {
-  int tps = 0, rho_block = 0, grad_block = 0;
-  bool wide = false, twin = false;  // a warp, or two lanes, for a site's tps lanes (effective_tile)
-  bool copies = false;              // pass 2 with eight copies of its tables (effective_tile)
-  bool operator==(const Tile &o) const { return tps == o.tps && rho_block == o.rho_block && grad_block == o.grad_block; }
-};
-inline bool valid_tile(int tps, int rho_block, int grad_block) {
-  return (tps == 0 || tps == 1 || tps == 2 || tps == 4 || tps == 8) &&
-         (rho_block == 0 || rho_block == 256 || rho_block == 512 || rho_block == 768) &&
-         (grad_block == 0 || grad_block == 128 || grad_block == 256 || grad_block == 512);
-}
 // The tile tuner (api.cu): threads per site at the default block sizes,
 // then the pass-1 block size, then the pass-2 block size, each stage keeping
 // the fastest; time_tile(tile, &ms) measures one candidate.  ms[10]
 // receives the candidates' times in that order (may be null).
 constexpr int kTileCandidates = 10;
 a2c_status tune_tile(const std::function<a2c_status(const Tile &, float *)> &time_tile, Tile *best, float *ms);
-// Threads per site of the mixed pair kernels when none was chosen: a
-// system with fewer than 2048 sites per SM spreads each site over 4 lanes
-// so that every SM gets work; a larger one runs one lane per site.
-inline int default_threads_per_site(int64_t n_sites, int sms) { return n_sites < (int64_t)sms * 2048 ? 4 : 1; }
-
 // k_fp64.cu
 a2c_status launch_density64(a2c_gpp_ctx *c, const double *dX);
 a2c_status launch_gradient64(a2c_gpp_ctx *c, const double *dX, double *dG);
@@ -252,7 +234,6 @@ int mixed_threads_per_site(a2c_gpp_ctx *c);
 // the context's tile as chosen (zeros: the library's choice) and as used
 a2c_status mixed_set_tile(a2c_gpp_ctx *c, const Tile &t);
 Tile mixed_tile(a2c_gpp_ctx *c);
-Tile effective_tile(const Tile &t, int64_t n_sites, int sms);
 // batched: prep + both passes over the listed sites (G, Vs, Ss; no objective)
 a2c_status mixed_eval_list(a2c_gpp_ctx *c, const double *dX, double *dG, const BatchView &bv, const Tile &tile);
 a2c_status mixed_prepare(a2c_gpp_ctx *c);  // tables and buffers, before any graph capture

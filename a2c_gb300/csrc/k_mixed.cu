@@ -37,7 +37,7 @@
 // (few sites) or serve it badly (one lane per site), TPS > V lanes evaluate
 // the site's neighbors TPS at a time and hand the terms round, each lane
 // adding those its V-th part would have met, in the same order: the same
-// bits (walk_together, add_pairs; effective_tile says when).
+// bits (walk_together, add_pairs; tile.h says when).
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -1613,38 +1613,6 @@ void mixed_free(a2c_gpp_ctx *c) {
 
 int mixed_threads_per_site(a2c_gpp_ctx *c) { return (c->mixed && c->mixed->tps) ? c->mixed->tps : 0; }
 
-Tile effective_tile(const Tile &t, int64_t n_sites, int sms) {
-  Tile e;
-  e.tps = t.tps ? t.tps : default_threads_per_site(n_sites, sms);
-  // Block sizes when none was chosen (they change no result).  Pass 1: two
-  // blocks fit an SM whatever their size, so 512 threads double its warps
-  // (262,144 sites at 4 threads per site: 178 -> 141 us; 33,592: 31 -> 27;
-  // 512: 15.4 either way), except with one thread per site (373,248 sites:
-  // 233 us at 256, 266 at 512).  Pass 2: 128 threads while there are few
-  // blocks to spread (512 sites: 27 against 29 us, 33,592: 54 against 56;
-  // 92,160: 115 against 113).
-  // More lanes per site than its sums' order asks for, where no block size
-  // was chosen: a warp for a site while there are few (passes 1 and 2 with
-  // 4 / 32 lanes, 512 sites: 16.4 + 26.8 / 8.1 + 18.9 us, 4,096: 16.4 + 26.8
-  // / 14.3 + 25.2, 8,000: 16.4 + 29.3 / 19.8 + 37.1), two lanes in place of
-  // one (512,000 sites: 315 + 614 / 303 + 580 us, 2,097,152: 1215 + 2559 /
-  // 1131 + 2399).
-  if (!t.rho_block && !t.grad_block) {
-    e.wide = n_sites <= 27 * (int64_t)sms;
-    e.twin = !e.wide && e.tps == 1;
-  }
-  e.rho_block = t.rho_block ? t.rho_block : e.tps > 1 ? 512 : kBlock;
-  e.grad_block = t.grad_block ? t.grad_block : n_sites < 256 * (int64_t)sms ? 128 : kBlock;
-  // Pass 2's shape of 256 threads (kBlock, or nothing chosen) has eight
-  // copies of f_Pd' under one block of 1024 threads per SM where its warps
-  // come near 32 per SM (pass 2 without / with them, 2 threads per site:
-  // 33,592 sites 59 / 83 us, 92,160: 125 / 109, 262,144: 293 / 266; 4 threads:
-  // 21,952: 45 / 51, 33,592: 58 / 53, 2,097,152: 2,076 / 1,891; two lanes for
-  // one: 33,592: 76 / 96, 92,160: 156 / 123).
-  e.copies = !e.wide && (!t.grad_block || t.grad_block == kBlock) && n_sites * (e.twin ? 2 : e.tps) >= 25 * 32 * (int64_t)sms;
-  return e;
-}
-
 Tile mixed_tile(a2c_gpp_ctx *c) {
   Tile t;
   if (c->mixed) {
@@ -1819,8 +1787,9 @@ a2c_status mixed_chem(a2c_gpp_ctx *c, const double *dX, double *d_send, const in
   a.T = c->p.T;
   // the state's fixed-point form and pass 1 (F and F' of every site)
   k_prep<<<grid_for(N, 256), 256, 0, c->stream>>>(dX, c->d_occ, N, k[0], k[1], k[2], M->P, M->occ, nullptr, span_args(c));
-  Tile one = mixed_tile(c);
-  one.tps = 1;
+  // one lane's order, on the blocks chosen for an evaluation (if any were)
+  const Tile chosen = effective_tile(mixed_tile(c), N, device_sms(c->device));
+  const Tile one = chosen.own ? Tile{1, 0, 0} : Tile{1, chosen.rho_block, chosen.grad_block};
   const Tile t = effective_tile(one, N, device_sms(c->device));
   launch_pass1<1, false>(a, c->stream, t);
   const double *cp = c->p.coe_Pd, *ch = c->p.coe_H;

@@ -1,0 +1,21 @@
+"""The rule that turns a chosen tile into the one that runs (tile.h, plain
+C++) on the host: it may be applied again, and to the three numbers a caller
+reads back, without changing what runs."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+
+
+@pytest.mark.parametrize("sms", [1, 132, 152])
+def test_the_rule_gives_the_same_tile_again(tmp_path, sms):
+    exe = tmp_path / "tile_check"
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(ROOT / "a2c_gb300" / "csrc"),
+                        str(ROOT / "tests" / "cpp" / "tile_check.cpp"), "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe), str(sms)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.returncode
+    n, wide, twin, copies = map(int, r.stdout.split())
+    assert n == 27 * 80 and wide > 0 and twin > 0 and copies > 0
