@@ -867,7 +867,7 @@ a2c_status plan(a2c_gpp_batch *b, const Dev &D) {
   return A2C_OK;
 }
 
-Tile batch_tile(a2c_gpp_batch *b) { return effective_tile(b->tile, b->c->N, device_sms(b->c->device)); }
+Tile batch_tile(a2c_gpp_batch *b) { return effective_tile(b->tile, b->c->N, device_sms(b->c->device), true); }
 
 // Evaluation of every listed site at X into G.  Both forms where a mixed
 // minimization ends in the FP64 polish (a form with an empty list costs an

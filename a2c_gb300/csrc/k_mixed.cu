@@ -1750,7 +1750,7 @@ a2c_status mixed_eval_list(a2c_gpp_ctx *c, const double *dX, double *dG, const B
   const int prep_cap = 8 * device_sms(c->device);
   k_prep_list<<<(unsigned)std::min<int64_t>(grid_for(N, 256), prep_cap), 256, 0, c->stream>>>(
       dX, c->d_occ, bv, M->P, M->occ, c->d_xlist, c->d_status);
-  launch_tile(a, c->stream, nullptr, once, effective_tile(tile, N, device_sms(c->device)), true);
+  launch_tile(a, c->stream, nullptr, once, effective_tile(tile, N, device_sms(c->device), true), true);
   A2C_CUDA(cudaGetLastError());
   return A2C_OK;
 }

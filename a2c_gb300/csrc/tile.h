@@ -30,10 +30,11 @@ inline bool valid_tile(int tps, int rho_block, int grad_block) {
 // so that every SM gets work; a larger one runs one lane per site.
 inline int default_threads_per_site(int64_t n_sites, int sms) { return n_sites < (int64_t)sms * 2048 ? 4 : 1; }
 
-// The tile that runs for a chosen one (zeros: the library's choice).  A tile
+// The tile that runs for a chosen one (zeros: the library's choice) on a
+// whole system or (list) on a batch's or minimization's site lists.  A tile
 // that this function gave, or its three numbers, gives the same tile again:
 // block sizes named explicitly count as the library's choice where they are.
-inline Tile effective_tile(const Tile &t, int64_t n_sites, int sms) {
+inline Tile effective_tile(const Tile &t, int64_t n_sites, int sms, bool list = false) {
   constexpr int kPlain = 256;
   Tile e;
   e.tps = t.tps ? t.tps : default_threads_per_site(n_sites, sms);
@@ -61,9 +62,11 @@ inline Tile effective_tile(const Tile &t, int64_t n_sites, int sms) {
   // 32 per SM (pass 2 without / with them, 2 threads per site: 33,592 sites
   // 59 / 83 us, 92,160: 125 / 109, 262,144: 293 / 266; 4 threads: 21,952:
   // 45 / 51, 33,592: 58 / 53, 2,097,152: 2,076 / 1,891; two lanes for one:
-  // 33,592: 76 / 96, 92,160: 156 / 123).
+  // 33,592: 76 / 96, 92,160: 156 / 123).  On lists a little later (30
+  // iterations of a minimization without / with them: 30,720 sites 6.06 /
+  // 6.14 ms, 32,768: 6.44 / 6.53, 34,816: 6.45 / 6.45, 38,880: 6.65 / 6.38).
   e.copies = !e.wide && (e.grad_block == kPlain || e.grad_block == grad) &&
-             n_sites * (e.twin ? 2 : e.tps) >= 25 * 32 * (int64_t)sms;
+             n_sites * (e.twin ? 2 : e.tps) >= (list ? 27 : 25) * 32 * (int64_t)sms;
   return e;
 }
 

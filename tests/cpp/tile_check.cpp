@@ -16,26 +16,31 @@ int main(int argc, char **argv) {
   if (argc < 2) return 2;
   const int sms = std::atoi(argv[1]);
   std::vector<int64_t> sizes;
-  for (int64_t at : {1, 27, 100, 200, 256, 400, 800, 2048, 13797})  // sites per SM: the thresholds
+  for (int64_t at : {1, 27, 100, 108, 200, 216, 256, 400, 432, 800, 864, 2048, 13797})  // sites per SM: the thresholds
     for (int64_t d : {-1, 0, 1}) sizes.push_back(at * sms + d);
   long n = 0, wide = 0, twin = 0, copies = 0;
-  for (int64_t N : sizes)
+  auto check = [&](int64_t N, bool list) {
     for (int tps : {0, 1, 2, 4, 8})
       for (int rho : {0, 256, 512, 768})
         for (int grad : {0, 128, 256, 512}) {
-          const Tile r = effective_tile(Tile{tps, rho, grad}, N, sms);
+          const Tile r = effective_tile(Tile{tps, rho, grad}, N, sms, list);
           ++n;
           wide += r.wide;
           twin += r.twin;
           copies += r.copies;
           if (!valid_tile(r.tps, r.rho_block, r.grad_block) || !r.tps || !r.rho_block || !r.grad_block) return 3;
-          if (!(effective_tile(r, N, sms) == r)) return 4;
-          if (!(effective_tile(Tile{r.tps, r.rho_block, r.grad_block}, N, sms) == r)) return 5;
-          const Tile lib = effective_tile(Tile{r.tps, 0, 0}, N, sms);
+          if (!(effective_tile(r, N, sms, list) == r)) return 4;
+          if (!(effective_tile(Tile{r.tps, r.rho_block, r.grad_block}, N, sms, list) == r)) return 5;
+          const Tile lib = effective_tile(Tile{r.tps, 0, 0}, N, sms, list);
           const bool own = r.rho_block == lib.rho_block && r.grad_block == lib.grad_block;
           if (own ? !(r == lib) : (r.wide || r.twin)) return 6;
           if (lib.wide != (N <= 27 * (int64_t)sms) || lib.twin != (!lib.wide && lib.tps == 1)) return 7;
         }
+    return 0;
+  };
+  for (int64_t N : sizes)
+    for (bool list : {false, true})
+      if (const int bad = check(N, list)) return bad;
   std::printf("%ld %ld %ld %ld\n", n, wide, twin, copies);
   return 0;
 }

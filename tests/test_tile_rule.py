@@ -18,4 +18,4 @@ def test_the_rule_gives_the_same_tile_again(tmp_path, sms):
     r = subprocess.run([str(exe), str(sms)], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.returncode
     n, wide, twin, copies = map(int, r.stdout.split())
-    assert n == 27 * 80 and wide > 0 and twin > 0 and copies > 0
+    assert n == 39 * 2 * 80 and wide > 0 and twin > 0 and copies > 0
