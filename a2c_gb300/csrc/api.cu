@@ -107,33 +107,6 @@ a2c_status time_context_tile(a2c_gpp_ctx *c, int reps, const Tile &t, float *ms)
   return s;
 }
 
-a2c_status tune_tile(const std::function<a2c_status(const Tile &, float *)> &time_tile, Tile *best, float *ms) {
-  static const int tps_c[4] = {1, 2, 4, 8}, rho_c[3] = {256, 512, 768}, grad_c[3] = {128, 256, 512};
-  Tile b;
-  b.rho_block = 256;
-  b.grad_block = 256;
-  float best_ms = 0.0f;
-  int k = 0;
-  auto trial = [&](const Tile &t) -> a2c_status {
-    float v = 0.0f;
-    A2C_TRY(time_tile(t, &v));
-    if (ms) ms[k] = v;
-    ++k;
-    if (b.tps == 0 || v < best_ms) {
-      best_ms = v;
-      b = t;
-    }
-    return A2C_OK;
-  };
-  for (int q : tps_c) A2C_TRY(trial(Tile{q, 256, 256}));
-  const Tile after_tps = b;
-  for (int q : rho_c) A2C_TRY(trial(Tile{after_tps.tps, q, after_tps.grad_block}));
-  const Tile after_rho = b;
-  for (int q : grad_c) A2C_TRY(trial(Tile{after_rho.tps, after_rho.rho_block, q}));
-  *best = b;
-  return A2C_OK;
-}
-
 }  // namespace a2c
 
 using namespace a2c;
@@ -451,7 +424,8 @@ a2c_status a2c_gpp_autotune_tile(a2c_gpp_ctx *c, int reps, int *tile, float *ms)
   const int saved = c->p.precision;
   c->p.precision = A2C_MIXED;
   Tile best;
-  a2c_status s = tune_tile([&](const Tile &t, float *v) { return time_context_tile(c, reps, t, v); }, &best, ms);
+  a2c_status s = tune_tile([&](const Tile &t, float *v) { return time_context_tile(c, reps, t, v); }, c->N,
+                           device_sms(c->device), false, &best, ms);
   c->p.precision = saved;
   c->has_density = false;
   if (!s) s = mixed_set_tile(c, best);

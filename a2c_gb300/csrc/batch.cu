@@ -1473,7 +1473,8 @@ a2c_status a2c_gpp_batch_autotune_tile(a2c_gpp_batch *b, const double *X, int re
   DeviceGuard dg(b->device);
   A2C_TRY(tune_setup(b, X));
   Tile best;
-  A2C_TRY(tune_tile([&](const Tile &t, float *v) { return time_batch_tile(b, reps, t, v); }, &best, ms));
+  A2C_TRY(tune_tile([&](const Tile &t, float *v) { return time_batch_tile(b, reps, t, v); }, b->c->N,
+                    device_sms(b->c->device), true, &best, ms));
   b->tile = best;
   if (tile) {
     tile[0] = best.tps;

@@ -155,12 +155,6 @@ inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 
 constexpr int kMaxDevices = 64;
 int device_sms(int dev);
 int current_device_sms();
-// The tile tuner (api.cu): threads per site at the default block sizes,
-// then the pass-1 block size, then the pass-2 block size, each stage keeping
-// the fastest; time_tile(tile, &ms) measures one candidate.  ms[10]
-// receives the candidates' times in that order (may be null).
-constexpr int kTileCandidates = 10;
-a2c_status tune_tile(const std::function<a2c_status(const Tile &, float *)> &time_tile, Tile *best, float *ms);
 // k_fp64.cu
 a2c_status launch_density64(a2c_gpp_ctx *c, const double *dX);
 a2c_status launch_gradient64(a2c_gpp_ctx *c, const double *dX, double *dG);

@@ -3,6 +3,9 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
+
+#include "a2c_gpp.h"
 
 namespace a2c {
 
@@ -68,6 +71,47 @@ inline Tile effective_tile(const Tile &t, int64_t n_sites, int sms, bool list = 
   e.copies = !e.wide && (e.grad_block == kPlain || e.grad_block == grad) &&
              n_sites * (e.twin ? 2 : e.tps) >= (list ? 27 : 25) * 32 * (int64_t)sms;
   return e;
+}
+
+// The tile tuner: threads per site at 256-thread blocks, then the pass-1
+// block size, then the pass-2 block size, each stage keeping the fastest;
+// time_tile(tile, &ms) measures one candidate.  ms[10] receives these
+// candidates' times in that order (may be null).  Then the library's own
+// blocks, at its and at the fastest's threads per site, which the stages may
+// have passed by: a tuned system is never slower than an untuned one.  The
+// result is resolved (effective_tile).
+constexpr int kTileCandidates = 10;
+inline a2c_status tune_tile(const std::function<a2c_status(const Tile &, float *)> &time_tile, int64_t n_sites, int sms,
+                            bool list, Tile *best, float *ms) {
+  Tile b{0, 256, 256};
+  float best_ms = 0.0f;
+  int k = 0;
+  auto trial = [&](const Tile &t) -> a2c_status {
+    float v = 0.0f;
+    const a2c_status s = time_tile(t, &v);
+    if (s != A2C_OK) return s;
+    if (ms && k < kTileCandidates) ms[k] = v;
+    ++k;
+    if (b.tps == 0 || v < best_ms) {
+      best_ms = v;
+      b = t;
+    }
+    return A2C_OK;
+  };
+  a2c_status s = A2C_OK;
+  for (int q : {1, 2, 4, 8})
+    if (!s) s = trial(Tile{q, 256, 256});
+  const Tile after_tps = b;
+  for (int q : {256, 512, 768})
+    if (!s) s = trial(Tile{after_tps.tps, q, after_tps.grad_block});
+  const Tile after_rho = b;
+  for (int q : {128, 256, 512})
+    if (!s) s = trial(Tile{after_rho.tps, after_rho.rho_block, q});
+  const Tile own = effective_tile(Tile{}, n_sites, sms, list), same = effective_tile(Tile{b.tps, 0, 0}, n_sites, sms, list);
+  if (!s) s = trial(own);
+  if (!s && !(same == own)) s = trial(same);
+  if (!s) *best = effective_tile(b, n_sites, sms, list);
+  return s;
 }
 
 }  // namespace a2c

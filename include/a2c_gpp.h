@@ -241,9 +241,10 @@ a2c_status a2c_gpp_autotune(a2c_gpp_ctx *ctx, int reps, int *tps, float *ms);
  * pass-2 block}.  a2c_gpp_autotune_tile measures candidates by coordinate
  * descent -- threads per site at 256-thread blocks, then the pass-1 block,
  * then the pass-2 block, each stage keeping the fastest -- on the context's
- * current state, sets the fastest and returns it; ms[10] (may be NULL)
- * receives the mean milliseconds per evaluation of the ten candidates in
- * that order. */
+ * current state, then the library's own block sizes, sets the fastest and
+ * returns it; ms[10] (may be NULL) receives the mean milliseconds per
+ * evaluation of the descent's ten candidates in that order.  Explicit block
+ * sizes that equal the library's choice are that choice. */
 a2c_status a2c_gpp_set_tile(a2c_gpp_ctx *ctx, int tps, int rho_block, int grad_block);
 a2c_status a2c_gpp_get_tile(a2c_gpp_ctx *ctx, int *tile);
 a2c_status a2c_gpp_autotune_tile(a2c_gpp_ctx *ctx, int reps, int *tile, float *ms);
