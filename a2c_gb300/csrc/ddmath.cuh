@@ -65,8 +65,18 @@ A2C_HD D2 quick_two_sum(double a, double b) {
   const double s = a + b;
   return {s, b - (s - a)};
 }
+// a * b rounded, where its rounding error is also carried: never contracted
+// with a sum that it enters (k_mixed.cu is compiled with contraction; a
+// product fused into the sum would count its error twice).
+A2C_HD double rounded_product(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  return __dmul_rn(a, b);
+#else
+  return a * b;  // host builds: -ffp-contract=off
+#endif
+}
 A2C_HD D2 two_prod(double a, double b) {
-  const double p = a * b;
+  const double p = rounded_product(a, b);
   return {p, fma(a, b, -p)};
 }
 A2C_HD D2 add(D2 a, D2 b) {
@@ -432,10 +442,10 @@ A2C_HD D2 quick_exp(D2 a, int &k) {
   const int ni = lo_word(t), j = ni & 63;
   k = (ni - j) / 64;
   const double r1 = fma(-n, 0.010830424696223417, a.hi);  // exact
-  const double p = n * 2.572804622327669e-14, pe = fma(n, 2.572804622327669e-14, -p);
+  const double p = rounded_product(n, 2.572804622327669e-14), pe = fma(n, 2.572804622327669e-14, -p);
   D2 r = two_sum(r1, -p);
   r = two_sum(r.hi, r.lo - pe + a.lo);
-  const double v = r.hi * r.hi, ve = fma(r.hi, r.hi, -v);
+  const double v = rounded_product(r.hi, r.hi), ve = fma(r.hi, r.hi, -v);
   double c = fma(r.hi, 1.984126984126984e-04, 1.388888888888889e-03);
   c = fma(r.hi, c, 8.333333333333333e-03);
   c = fma(r.hi, c, 4.1666666666666664e-02);
@@ -608,7 +618,7 @@ A2C_HD D2 quick_log(double u, double &err) {
 #endif
   const D2 p = two_prod(m, c);
   const double z = p.hi - 1.0, zl = p.lo;
-  const double v = z * z, ve = fma(z, z, -v);
+  const double v = rounded_product(z, z), ve = fma(z, z, -v);
   double q = fma(z, 9.090909090909091e-02, -0.1);
   q = fma(z, q, 1.1111111111111111e-01);
   q = fma(z, q, -0.125);
@@ -653,10 +663,10 @@ A2C_HD int quick_cr_exp_both(double x, double &up, double &down) {
   const double n = t - kRoundShift;
   const int ni = lo_word(t);
   const double r1 = fma(-n, 0.010830424696223417, x);
-  const double p = n * 2.572804622327669e-14, pe = fma(n, 2.572804622327669e-14, -p);
+  const double p = rounded_product(n, 2.572804622327669e-14), pe = fma(n, 2.572804622327669e-14, -p);
   D2 r = two_sum(r1, -p);
   r = quick_two_sum(r.hi, r.lo - pe);
-  const double v = r.hi * r.hi, ve = fma(r.hi, r.hi, -v), vh = 0.5 * v;
+  const double v = rounded_product(r.hi, r.hi), ve = fma(r.hi, r.hi, -v), vh = 0.5 * v;
   const double odd = fma(v, fma(v, 1.984126984126984e-04, 8.333333333333333e-03), 1.6666666666666666e-01);
   const double even = fma(v, 1.388888888888889e-03, 4.1666666666666664e-02);
   const double w = fma(r.hi, r.lo, 0.5 * ve);
