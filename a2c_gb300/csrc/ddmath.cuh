@@ -280,9 +280,9 @@ A2C_HD double mul_int(double a, double b) {
   return from_words((int)(r >> 32), (int)(unsigned)r);
 #endif
 }
-// |x| in [2^-511, 2^513): the product of two such values is normal
+// |x| in [2^-511, 2^512): the product of two such values is normal
 A2C_HD bool mul_int_ok(double x) {
-  return (unsigned)((hi_word(x) & 0x7ff00000) - 0x20000000) < 0x40000000u;
+  return (unsigned)((hi_word(x) & 0x7ff00000) - 0x20000000) < 0x3ff00000u;
 }
 
 // Adding 1.5 2^52 rounds |v| < 2^31 to an integer (ties to even), held in
