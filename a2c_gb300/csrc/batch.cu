@@ -880,7 +880,7 @@ a2c_status eval_lists(a2c_gpp_batch *b, const double *X, double *G, const Cfg &c
 
 // One tick (see the file comment); the same launches whether captured or
 // not.  262,144 sites, one instance, 5 pairs: about 600 us,
-// 415 of them the evaluation (20 iterations 25.3 -> 20.1 ms).
+// 415 of them the evaluation (20 iterations 24.8 -> 20.5 ms).
 a2c_status tick(a2c_gpp_batch *b, const Dev &D, const Cfg &cf, const Tile &tps) {
   cudaStream_t s = b->c->stream;
   const int ge = chunk_grid(cf.nec), gs = chunk_grid(cf.nsc);

@@ -1,5 +1,5 @@
 // The pair functions of eam64.cuh as the FP64 pair kernels evaluate them:
-// the same bits (tests/test_fp64_pair_forms.py compares them on the host)
+// the same bits (tests/test_fp64_forms.py compares them on the host)
 // in fewer FP64 operations.  GB300's FP64 pipe takes two lanes per SM and
 // clock, so a warp's FP64 instruction occupies its scheduler's share of the
 // pipe for 64 clocks and the count of such instructions is the time of

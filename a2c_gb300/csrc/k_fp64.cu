@@ -18,7 +18,7 @@
 // functions' fewer operations (eam64_pair.cuh) an evaluation takes, one
 // thread per site -> now: 15.3 -> 0.70 ms at 512 sites, 23.0 -> 5.5 ms at
 // 10,296, 210.6 -> 108.5 ms at 262,144.  Five blocks of pass 2 per SM: 10,296
-// sites then fit at once (5.6 -> 4.6 ms).
+// sites then fit at once (the evaluation 5.57 -> 5.29 ms).
 //
 // Geometry: for quadrature point k = 2m (+sqrt(3)) or 2m+1 (-sqrt(3)) only
 // coordinate m of R^6 is non-zero, so r_k differs from the pair's base

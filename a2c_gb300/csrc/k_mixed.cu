@@ -62,7 +62,7 @@ struct Mixed {
   int grid_cap[9] = {};       // persistent grid size per threads-per-site
   float4 *tabEmb = nullptr;   // per rho interval: F_Pd cubics, then F_H cubics
   int tps = 0;                // threads per site (0 = choose)
-  int rho_block = 0, grad_block = 0;  // threads per block of pass 1 and pass 2 (0 = 256)
+  int rho_block = 0, grad_block = 0;  // threads per block of pass 1 and pass 2 (0: tile.h chooses)
   // Pass 2 with every pair evaluated once (sorted, symmetric lists): per
   // list entry of a pair the site owns (neighbor id below its own) the slot
   // of the reverse entry; per site the count of such entries, with the
@@ -1381,7 +1381,7 @@ void launch_grad(const MixArgs &a, cudaStream_t st, bool once) {
 }
 
 // Pass 1 at V lanes per site in its sums' order, on the lanes the size asks
-// for (see spread).
+// for (tile.h).
 template <int V, bool LIST>
 void launch_pass1(const MixArgs &a, cudaStream_t st, const Tile &t) {
   if (t.wide) {

@@ -690,7 +690,7 @@ a2c_status scan_exclusive(ListWork *w, const int64_t *in, int64_t *out, int64_t 
 // sparse system in free directions) gives them back after the build.
 constexpr int64_t cells_kept(int64_t n_sites) { return 4 * n_sites + 4096; }
 
-// Cell grid for cutoff `cut` (cells at least `cut` wide), from the extents
+// Cell grid for cutoff `cut` (`reach` cells to either side span it), from the extents
 // of the free directions; with scan null (a list re-filter, which uses no
 // cells) they are left nominal.
 int64_t make_grid(const a2c_gpp_ctx *c, const PosScan *scan, double cut, GridArgs &g) {
