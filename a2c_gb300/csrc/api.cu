@@ -963,12 +963,12 @@ a2c_status a2c_gpp_apply_dirichlet(a2c_gpp_ctx *c, const int *sites, int n, doub
   A2C_CUDA(cudaMemcpyAsync(h->sites, sites, sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
   A2C_TRY(launch_dirichlet(c, h->sites, n, gamma_bd, xUb, nullptr, nullptr));
   c->has_density = false;
-  A2C_TRY(finish(c));
+  const a2c_status s = finish(c);  // may report an earlier evaluation: the condition is applied all the same
   for (int t = 0; t < n; ++t) {
     gamma[sites[t]] = gamma_bd;
     full_H[sites[t]] = 1;
   }
-  return A2C_OK;
+  return s;
 }
 
 a2c_status a2c_gpp_diffuse(a2c_gpp_ctx *c, double dt, double nu, double Qm, double xLb, double xUb,
