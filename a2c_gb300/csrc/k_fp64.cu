@@ -17,8 +17,8 @@
 // two ends (rho_sites_per_warp, grad_sites_per_warp).  With the pair
 // functions' fewer operations (eam64_pair.cuh) an evaluation takes, one
 // thread per site -> now: 15.3 -> 0.70 ms at 512 sites, 23.0 -> 5.5 ms at
-// 10,296, 210.6 -> 108.5 ms at 262,144.  Five blocks of pass 2 per SM: 10,296
-// sites then fit at once (the evaluation 5.57 -> 5.29 ms).
+// 10,296, 210.6 -> 108.5 ms at 262,144.  Five blocks of pass 2 per SM in place of
+// four: an evaluation of 10,296 sites 5.67 -> 5.38 ms, of 262,144 110.5 -> 108.5.
 //
 // Geometry: for quadrature point k = 2m (+sqrt(3)) or 2m+1 (-sqrt(3)) only
 // coordinate m of R^6 is non-zero, so r_k differs from the pair's base
