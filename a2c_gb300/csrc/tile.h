@@ -65,11 +65,12 @@ inline Tile effective_tile(const Tile &t, int64_t n_sites, int sms, bool list = 
   // 32 per SM (pass 2 without / with them, 2 threads per site: 33,592 sites
   // 59 / 83 us, 92,160: 125 / 109, 262,144: 293 / 266; 4 threads: 21,952:
   // 45 / 51, 33,592: 58 / 53, 2,097,152: 2,076 / 1,891; two lanes for one:
-  // 33,592: 76 / 96, 92,160: 156 / 123).  On lists a little later (30
-  // iterations of a minimization without / with them: 30,720 sites 6.06 /
-  // 6.14 ms, 32,768: 6.44 / 6.53, 34,816: 6.45 / 6.45, 38,880: 6.65 / 6.38).
-  e.copies = !e.wide && (e.grad_block == kPlain || e.grad_block == grad) &&
-             n_sites * (e.twin ? 2 : e.tps) >= (list ? 27 : 25) * 32 * (int64_t)sms;
+  // 33,592: 76 / 96, 92,160: 156 / 123).  Lists keep the library's 128-thread
+  // blocks where it chooses those: a batch of five lattices with 33,144 sites
+  // takes 2,658 us without, 2,740 with them; 30 iterations of one
+  // minimization 6.06 / 6.14 ms at 30,720 sites, 6.65 / 6.38 at 38,880.
+  e.copies = !e.wide && (e.grad_block == kPlain || (e.grad_block == grad && !list)) &&
+             n_sites * (e.twin ? 2 : e.tps) >= 25 * 32 * (int64_t)sms;
   return e;
 }
 
