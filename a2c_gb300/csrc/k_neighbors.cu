@@ -856,8 +856,8 @@ a2c_status fill_cells(a2c_gpp_ctx *c, ListWork *w, const GridArgs &g, int64_t nc
 // stride there is no memory, are counted by that pass and written at their
 // offsets by a second; the stride then grows to the longest list unless a
 // few long ones would make it more than twice what the lists take.  Bound by
-// instruction issue and the latency of the candidate loads (about 1,300
-// instructions a site).  At 262,144 sites the pass takes 568 us and the copy
+// instruction issue and the latency of the candidate loads (about 2,100
+// instructions a site by a warp).  At 262,144 sites the pass takes 568 us and the copy
 // 137; one thread per site that walked its 27 cells twice, to count and to
 // fill, and sorted in global memory took 930 + 1,500 us; a warp per site over
 // those 27 cells in two passes took 576 + 862 us.
